@@ -1,7 +1,7 @@
 // Single-warp fused 1D run: a line of up to 512 cells held by ONE warp, CPT
 // consecutive cells per lane in registers, the whole time loop in one launch.
 //
-// The step keeps the reference's serial order (E -> source -> DFT -> ABC -> H,
+// The step keeps the reference's serial order (E -> source -> ABC -> H,
 // fd1d/program/fd1d_2_2.py:138-142) and calls the same per-cell formulas as
 // the per-function kernels, so the fields are bitwise equal to them.  What
 // makes it short is that nothing per step depends on where the line ends:
@@ -18,13 +18,10 @@
 //     nx-1 are the last two cells of their lane, also compile-time positions;
 //     otherwise the mask selects find them;
 //   * the left neighbour's last hy and the right neighbour's first ex travel
-//     by one warp shuffle each; no barrier and no shared memory in the step
-//     (the probe DFT publishes its cells through a shared slot per step
-//     parity);
+//     by one warp shuffle each; no barrier and no shared memory in the step;
 //   * the source values of 32 steps are read by one coalesced load, one per
 //     lane, a chunk ahead, and broadcast by shuffle in the step.
-// Probe DFT accumulators sit in registers of lane f when nf <= 32, else they
-// are accumulated in place in global memory (lanes stride over f).
+// Runs with the running DFT take the chunked kernel (fd1d_halo.cuh) instead.
 #pragma once
 
 #include "fdtd_common.cuh"
@@ -43,15 +40,13 @@ __device__ __forceinline__ float bsel(unsigned m, float a, float b) {
 }
 
 // SOFT: the source adds to the field (else it replaces it, or is absent)
-template <int FORM, int CPT, bool HI_END, bool DFT, bool SOFT>
+template <int FORM, int CPT, bool HI_END, bool SOFT>
 __global__ void __launch_bounds__(32) k_fd1d_warp(const Warp1DArgs a) {
   constexpr bool DF = (FORM == FDTD1D_FORM_DFORM || FORM == FDTD1D_FORM_DEBYE);
   constexpr bool DB = (FORM == FDTD1D_FORM_DEBYE);
   constexpr unsigned kAll = 0xffffffffu;
   const fdtd1d_params& p = a.p;
   const fdtd1d_state& s = a.s;
-  __shared__ float x_probe[2][FDTD1D_MAX_PROBES];
-
   const int lane = threadIdx.x;
   const int nx = p.nx;
   const int g0 = lane * CPT;
@@ -113,23 +108,8 @@ __global__ void __launch_bounds__(32) k_fd1d_warp(const Warp1DArgs a) {
     bc3 = s.bc[3];
   }
 
-  // probe DFT (lane f holds frequency f when nf <= 32)
-  const int nf = DFT ? p.nf : 0;
-  const int npr = DFT ? p.nprobe : 0;
-  const bool pr_reg = nf <= 32;
-  float pr_r[FDTD1D_MAX_PROBES], pr_i[FDTD1D_MAX_PROBES];
-#pragma unroll
-  for (int q = 0; q < FDTD1D_MAX_PROBES; ++q) {
-    pr_r[q] = 0.f;
-    pr_i[q] = 0.f;
-    if (DFT && q < npr && pr_reg && lane < nf) {
-      pr_r[q] = s.r_pr[(size_t)q * nf + lane];
-      pr_i[q] = s.i_pr[(size_t)q * nf + lane];
-    }
-  }
-
-  // one time step t with source value v; branch-free except the DFT
-  auto step = [&](const int t, const float v) {
+  // one time step t with source value v; branch-free
+  auto step = [&](const float v) {
     // ---------------- E stage (+ source)
     // lane 0 receives its own value: cell 0 is never E-updated
     const float hy_left = __shfl_up_sync(kAll, hy[CPT - 1], 1);
@@ -166,60 +146,6 @@ __global__ void __launch_bounds__(32) k_fd1d_warp(const Warp1DArgs a) {
           ex[c] = e;
           ixa[c] = ixn;
           if (DB) sxa[c] = sxn;
-        }
-      }
-    }
-
-    // ---------------- running DFT (before the ABC, as fourier() precedes hfield())
-    if (DFT) {
-      const int buf = t & 1;
-      for (int q = 0; q < npr; ++q) {
-        const int k = p.probe_k[q];
-        if (k / CPT == lane) {
-          float e = 0.f;
-#pragma unroll
-          for (int c = 0; c < CPT; ++c)
-            if (g0 + c == k) e = ex[c];
-          x_probe[buf][q] = e;
-        }
-      }
-      const float* cs = p.dft_cos + (size_t)(t - 1) * nf;
-      const float* sn = p.dft_sin + (size_t)(t - 1) * nf;
-      if (p.full_dft) {
-        for (int f = 0; f < nf; ++f) {
-          const float cf = __ldg(cs + f), sf = __ldg(sn + f);
-#pragma unroll
-          for (int c = 0; c < CPT; ++c) {
-            const int g = g0 + c;
-            if (g < nx) {
-              const size_t m = (size_t)f * nx + g;
-              s.r_pt[m] = __fmaf_rn(cf, ex[c], s.r_pt[m]);
-              s.i_pt[m] = __fmaf_rn(-sf, ex[c], s.i_pt[m]);
-            }
-          }
-        }
-      }
-      __syncwarp();
-      if (pr_reg) {
-        if (lane < nf) {
-          const float cf = __ldg(cs + lane), sf = __ldg(sn + lane);
-#pragma unroll
-          for (int q = 0; q < FDTD1D_MAX_PROBES; ++q)
-            if (q < npr) {
-              const float e = x_probe[buf][q];
-              pr_r[q] = __fmaf_rn(cf, e, pr_r[q]);
-              pr_i[q] = __fmaf_rn(-sf, e, pr_i[q]);
-            }
-        }
-      } else {
-        for (int f = lane; f < nf; f += 32) {
-          const float cf = __ldg(cs + f), sf = __ldg(sn + f);
-          for (int q = 0; q < npr; ++q) {
-            const float e = x_probe[buf][q];
-            const size_t m = (size_t)q * nf + f;
-            s.r_pr[m] = __fmaf_rn(cf, e, s.r_pr[m]);
-            s.i_pr[m] = __fmaf_rn(-sf, e, s.i_pr[m]);
-          }
         }
       }
     }
@@ -267,15 +193,13 @@ __global__ void __launch_bounds__(32) k_fd1d_warp(const Warp1DArgs a) {
     const int tn = tc + 32 + lane;
     const float vn = (have_src && tn < t_end) ? __ldg(p.src_table + tn) : 0.f;
     int j = 0;
-    if (!DFT) {
-      // 16 steps unrolled: the scheduler interleaves neighbouring steps
-      // (47 us per config-1 run against 51 us for 4 and 55 us for none)
-      for (; j + 16 <= nchunk; j += 16) {
+    // 16 steps unrolled: the scheduler interleaves neighbouring steps
+    // (47 us per config-1 run against 51 us for 4 and 55 us for none)
+    for (; j + 16 <= nchunk; j += 16) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) step(tc + j + i + 1, __shfl_sync(kAll, vc, j + i));
-      }
+      for (int i = 0; i < 16; ++i) step(__shfl_sync(kAll, vc, j + i));
     }
-    for (; j < nchunk; ++j) step(tc + j + 1, __shfl_sync(kAll, vc, j));
+    for (; j < nchunk; ++j) step(__shfl_sync(kAll, vc, j));
     vc = vn;
   }
 
@@ -303,43 +227,9 @@ __global__ void __launch_bounds__(32) k_fd1d_warp(const Warp1DArgs a) {
     s.bc[2] = bc2;
     s.bc[3] = bc3;
   }
-  if (DFT && pr_reg && lane < nf) {
-#pragma unroll
-    for (int q = 0; q < FDTD1D_MAX_PROBES; ++q)
-      if (q < npr) {
-        s.r_pr[(size_t)q * nf + lane] = pr_r[q];
-        s.i_pr[(size_t)q * nf + lane] = pr_i[q];
-      }
-  }
 }
 
 // Launches the single-warp run; FDTD_ERR_SIZE when nx > 32 * 16.
 int launch_fd1d_warp(const fdtd1d_params& p, const fdtd1d_state& s, int t0, int nsteps, cudaStream_t st);
-// the two halves of the dispatch (one per translation unit)
-int launch_fd1d_warp_plain(const Warp1DArgs& a, int cpt, bool hi_end, cudaStream_t st);
-int launch_fd1d_warp_dft(const Warp1DArgs& a, int cpt, bool hi_end, cudaStream_t st);
-
-template <bool DFT>
-int launch_fd1d_warp_half(const Warp1DArgs& a, int cpt, bool hi_end, cudaStream_t st) {
-  auto go = [&](auto kern) -> int {
-    kern<<<1, 32, 0, st>>>(a);
-    return fdtd_host::check_launch();
-  };
-  const bool soft = a.p.src_kind == FDTD_SRC_SOFT;
-#define FDTD_WARP_CASE(F, C)                                                          \
-  if (a.p.form == F && cpt == C) {                                                    \
-    if (soft) return hi_end ? go(k_fd1d_warp<F, C, true, DFT, true>) : go(k_fd1d_warp<F, C, false, DFT, true>); \
-    return hi_end ? go(k_fd1d_warp<F, C, true, DFT, false>) : go(k_fd1d_warp<F, C, false, DFT, false>);       \
-  }
-#define FDTD_WARP_FORM(F) \
-  FDTD_WARP_CASE(F, 2) FDTD_WARP_CASE(F, 4) FDTD_WARP_CASE(F, 8) FDTD_WARP_CASE(F, 16)
-  FDTD_WARP_FORM(FDTD1D_FORM_CB)
-  FDTD_WARP_FORM(FDTD1D_FORM_CACB)
-  FDTD_WARP_FORM(FDTD1D_FORM_DFORM)
-  FDTD_WARP_FORM(FDTD1D_FORM_DEBYE)
-#undef FDTD_WARP_FORM
-#undef FDTD_WARP_CASE
-  return FDTD_ERR_ARG;
-}
 
 }  // namespace fdtd
