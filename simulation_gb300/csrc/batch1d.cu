@@ -8,24 +8,39 @@
 // no batched form; this is the library's extension for spectra sweeps.
 //
 // Execution model:
-//   * a run is executed by a TEAM of warps inside a thread block: each thread
-//     holds CPT consecutive cells (ex, hy) in registers; warp shuffles carry
-//     the neighbour values inside a warp and a few shared-memory slots carry
-//     them across warps; two team barriers per time step (a named barrier
-//     `bar.sync id, n` for multi-warp teams, __syncwarp for one-warp teams);
-//   * the per-cell (ca, cb) pairs are expanded from the run's layer table into
-//     shared memory once per run;
+//   * a run is executed by a TEAM of warps inside a thread block: each lane
+//     holds CPT consecutive cells (ex, hy) in registers and warp shuffles carry
+//     the neighbour values inside a warp;
+//   * neighbouring warps overlap by one lane: lane 31 of a warp and lane 0 of
+//     the next hold the same CPT cells, the first half owned by the former, the
+//     second by the latter, and each advances the other's half redundantly.
+//     Wrong values creep in by one cell a step, so the warps exchange their
+//     halves once in H = CPT/2 steps, with ONE team barrier (a named barrier
+//     `bar.sync id, n`), instead of two barriers in every step;
+//   * the cells' updates are packed two to an instruction (f32x2: the same
+//     rounding), 3.5 instructions per cell-step.  A warp whose lanes each lie
+//     in one material reads its (ca, cb) from two registers; only warps that
+//     hold a material boundary read per-cell pairs from shared memory, where
+//     they are expanded from the layer table once per run;
+//   * the probe cells are sampled into shared memory and the team adds the
+//     samples to its DFT accumulators once per exchange, spread over its warps;
 //   * the host planner (fdtd1d_batch_plan, C++ below) sizes each team as
-//     ceil(ke / CPT) rounded up to whole warps, so every run costs about the
-//     same per step, and packs teams into "bundles" that fill a block
-//     (first-fit decreasing, <= 15 multi-warp teams per block);
+//     ceil(ke / cells_per_thread) rounded up to whole warps, so every run costs
+//     about the same per step, and packs teams into "bundles" that fill a block
+//     (first-fit decreasing, <= 15 multi-warp teams per block).  A lane holds
+//     two cells more than the plan's cells_per_thread, which more than pays for
+//     the overlaps, so every run that the plan admits fits its team;
 //   * persistent blocks take bundles from a device counter (atomicAdd); there
 //     is no spin-wait anywhere.  An optional clock budget stops a block from
 //     taking new bundles and raises FDTD_STATUS_TIMEOUT; per-run `done` flags
 //     say which runs finished.
+// What bounds it: the FP32 pipe and issue slots (5 FP32 operations and 3.5
+// instructions per cell-step, four warps per scheduler).
 #include <algorithm>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "fdtd_common.cuh"
@@ -56,146 +71,294 @@ __device__ __forceinline__ void team_sync(int bar_id, int nthreads) {
   }
 }
 
-// a[c] for a runtime c: a switch (an indexed branch taken by the calling
-// lane), not a compare-and-select per cell; callers keep it to one thread
-#define FDTD_CELL_CASE(k)        \
-  case k:                        \
-    if constexpr (k < CPT) body(a[k < CPT ? k : 0]); \
-    break;
-template <int CPT, class A, class F>
-__device__ __forceinline__ void cell_at(A& a, int c, F&& body) {
-  static_assert(CPT <= 64, "cells per thread");
-  switch (c) { FDTD_CELL_CASE(0) FDTD_CELL_CASE(1) FDTD_CELL_CASE(2) FDTD_CELL_CASE(3) FDTD_CELL_CASE(4) FDTD_CELL_CASE(5) FDTD_CELL_CASE(6) FDTD_CELL_CASE(7) FDTD_CELL_CASE(8) FDTD_CELL_CASE(9) FDTD_CELL_CASE(10) FDTD_CELL_CASE(11) FDTD_CELL_CASE(12) FDTD_CELL_CASE(13) FDTD_CELL_CASE(14) FDTD_CELL_CASE(15) FDTD_CELL_CASE(16) FDTD_CELL_CASE(17) FDTD_CELL_CASE(18) FDTD_CELL_CASE(19) FDTD_CELL_CASE(20) FDTD_CELL_CASE(21) FDTD_CELL_CASE(22) FDTD_CELL_CASE(23) FDTD_CELL_CASE(24) FDTD_CELL_CASE(25) FDTD_CELL_CASE(26) FDTD_CELL_CASE(27) FDTD_CELL_CASE(28) FDTD_CELL_CASE(29) FDTD_CELL_CASE(30) FDTD_CELL_CASE(31) FDTD_CELL_CASE(32) FDTD_CELL_CASE(33) FDTD_CELL_CASE(34) FDTD_CELL_CASE(35) FDTD_CELL_CASE(36) FDTD_CELL_CASE(37) FDTD_CELL_CASE(38) FDTD_CELL_CASE(39) FDTD_CELL_CASE(40) FDTD_CELL_CASE(41) FDTD_CELL_CASE(42) FDTD_CELL_CASE(43) FDTD_CELL_CASE(44) FDTD_CELL_CASE(45) FDTD_CELL_CASE(46) FDTD_CELL_CASE(47) FDTD_CELL_CASE(48) FDTD_CELL_CASE(49) FDTD_CELL_CASE(50) FDTD_CELL_CASE(51) FDTD_CELL_CASE(52) FDTD_CELL_CASE(53) FDTD_CELL_CASE(54) FDTD_CELL_CASE(55) FDTD_CELL_CASE(56) FDTD_CELL_CASE(57) FDTD_CELL_CASE(58) FDTD_CELL_CASE(59) FDTD_CELL_CASE(60) FDTD_CELL_CASE(61) FDTD_CELL_CASE(62) FDTD_CELL_CASE(63) }
+// body(K) for each of the up to 7 cells K around the runtime cell c, which is
+// the same in the whole warp: a tree of uniform branches to a short run of
+// straight-line code, in which the body selects its lane and cell by
+// predicates.  (An indexed branch to one of 42 cases took more than the whole
+// step: 44 ms against 20 without any special cell, for 4096 runs of 2000
+// steps.)
+template <int LO, class F, int... K>
+__device__ __forceinline__ void cell_each(F& body, std::integer_sequence<int, K...>) {
+  (body(std::integral_constant<int, LO + K>{}), ...);
 }
-#undef FDTD_CELL_CASE
-template <int CPT>
-__device__ __forceinline__ float cell_get(const float (&a)[CPT], int c) {
-  float r = 0.f;
-  cell_at<CPT>(a, c, [&](const float& x) { r = x; });
-  return r;
+template <int LO, int HI, class F>
+__device__ __forceinline__ void cell_at(int c, F&& body) {
+  if constexpr (HI - LO <= 7) {
+    cell_each<LO>(body, std::make_integer_sequence<int, HI - LO>{});
+  } else {
+    constexpr int MID = (LO + HI) / 2;
+    if (c < MID) cell_at<LO, MID>(c, body);
+    else cell_at<MID, HI>(c, body);
+  }
 }
-template <int CPT>
-__device__ __forceinline__ void cell_set(float (&a)[CPT], int c, float v) {
-  cell_at<CPT>(a, c, [&](float& x) { x = v; });
+// cell K of a packed register array
+template <int K, int N>
+__device__ __forceinline__ float& cell(float2 (&a)[N]) {
+  if constexpr (K % 2 == 0) return a[K / 2].x;
+  else return a[K / 2].y;
+}
+// cells [LO, LO+N) to or from consecutive floats, in pairs where they are aligned (p: pairs start at even offsets)
+template <int LO, int N, int M>
+__device__ __forceinline__ void cells_put(float2 (&a)[M], float* p) {
+  if constexpr (LO % 2) *p = cell<LO>(a);
+#pragma unroll
+  for (int k = (LO + 1) / 2; k < (LO + N) / 2; ++k) *reinterpret_cast<float2*>(p + 2 * k - LO / 2 * 2) = a[k];
+  if constexpr ((LO + N) % 2) p[LO + N - 1 - LO / 2 * 2] = cell<LO + N - 1>(a);
+}
+template <int LO, int N, int M>
+__device__ __forceinline__ void cells_get(float2 (&a)[M], const float* p) {
+  if constexpr (LO % 2) cell<LO>(a) = *p;
+#pragma unroll
+  for (int k = (LO + 1) / 2; k < (LO + N) / 2; ++k) a[k] = *reinterpret_cast<const float2*>(p + 2 * k - LO / 2 * 2);
+  if constexpr ((LO + N) % 2) cell<LO + N - 1>(a) = p[LO + N - 1 - LO / 2 * 2];
 }
 
+// a 16-byte shared-memory read that stays where it is written (the compiler
+// would sink it to its use, which then waits for it)
+__device__ __forceinline__ float4 lds4(const float4* p) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+  return v;
+}
+
+// floats of one warp's edge buffer (ex and hy of half a lane, padded to pairs) and of one team's probe samples
+__host__ __device__ constexpr int edge_floats(int cpt) { return 2 * ((cpt / 2 + 2) / 2 * 2); }
+__host__ __device__ constexpr int sample_floats(int cpt) { return 2 * (cpt / 2 + 1); }
+
 template <int CPT>
-__device__ void run_team(const BatchArgs& A, int run, int T, int tt, int bar_id, int warp_base, float2* coef,
-                         float* x_last_hy, float* x_first_ex, float* x_last_ex, float* x_probe, float* acc) {
+__device__ void run_team(const BatchArgs& A, int run, int T, int tt, int bar_id, int wb, float4* coef, float* edges,
+                         float* samples, float* acc) {
+  static_assert(CPT / 2 <= 32, "one lane per source value of an epoch");
+  constexpr int H = CPT / 2, NP = CPT / 2, EF = edge_floats(CPT), HF = EF / 2, SF = sample_floats(CPT);
   const fdtd1d_batch_params& p = A.p;
   const int lane = threadIdx.x & 31;
-  const int w = tt >> 5;              // warp index inside the team
-  const int nw = T >> 5;
+  const int w = tt >> 5;  // warp index inside the team
   const int nx = p.ke[run];
+  // warps that hold cells: cell 31*CPT*w is the first of warp w
+  const int nw = nx <= 32 * CPT ? 1 : ((nx + CPT - 1) / CPT - 1 + 30) / 31;
+  const int g0 = (31 * w + lane) * CPT;  // first cell of this lane
+  const bool active = w < nw;
 
-  // expand the layer table: background ca=1, cb=0.5 (free space of fd1d_1_5);
-  // cells past the run's end get ca=cb=0, which keeps them exactly 0, so the
-  // cell loops below need no range test (their H update adds 0.5*(0-0)).
-  // Cell c of thread (warp w, lane l) is stored at coef[(w*CPT + c)*32 + l]:
-  // the warp's read of its c-th cells touches 32 consecutive float2 (a
-  // thread-major layout puts lanes CPT*8 bytes apart: 8-way bank conflicts),
-  // and each thread reads at constant offsets c*256 bytes from its own base.
+  // expand the layer table: background ca=1, cb=0.5 (free space of fd1d_1_5).
+  // Cells past the run's end are free space too, so the cell loops need no
+  // range test: nothing flows back from them, since ex[nx-1] is set by the ABC
+  // after every E update (nor from hy[nx-1], which only that update reads; it
+  // is kept at 0, as the reference never updates it, where a probe sees the
+  // updated ex[nx-1] before the ABC).
   const int l0 = p.layer_off[run], l1 = p.layer_off[run + 1];
-  for (int i = tt; i < T * CPT; i += T) {
-    float ca = i < nx ? 1.f : 0.f, cb = i < nx ? 0.5f : 0.f;
-    for (int l = l0; l < l1; ++l)
-      if (i >= p.layer_start[l] && i < p.layer_end[l]) {
-        ca = p.layer_ca[l];
-        cb = p.layer_cb[l];
+  float2 ca = make_float2(1.f, 1.f), cb = make_float2(0.5f, 0.5f);  // of a lane in one material
+  bool one = true;
+  if (active) {
+    float4* const mine = coef + (size_t)w * NP * 32 + lane;  // [pair][lane]: 16-byte reads without bank conflicts
+#pragma unroll 1
+    for (int k = 0; k < NP; ++k) {
+      float a2[2], b2[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = g0 + 2 * k + h;
+        a2[h] = 1.f;
+        b2[h] = 0.5f;
+        if (i < nx)
+          for (int l = l0; l < l1; ++l)
+            if (i >= p.layer_start[l] && i < p.layer_end[l]) {
+              a2[h] = p.layer_ca[l];
+              b2[h] = p.layer_cb[l];
+            }
+        if (k == 0 && h == 0) {
+          ca = make_float2(a2[0], a2[0]);
+          cb = make_float2(b2[0], b2[0]);
+        }
+        one &= a2[h] == ca.x && b2[h] == cb.x;
       }
-    const int th = i / CPT, c = i - th * CPT;
-    coef[((th >> 5) * CPT + c) * 32 + (th & 31)] = make_float2(ca, cb);
+      mine[k * 32] = make_float4(a2[0], a2[1], b2[0], b2[1]);
+    }
   }
-  const float2* my_coef = coef + (size_t)w * CPT * 32 + lane;
+  const bool uniform = __all_sync(FULL, one);
+  const float4* const my_coef = coef + (size_t)w * NP * 32 + lane;  // read by the lane that wrote it
   const int pin = p.probe_in[run], pout = p.probe_out[run];
   const int nf = p.nf;
   // DFT accumulators of the team in shared memory: acc[4][nf] (re/im at the
-  // entry probe, re/im at the exit probe); thread tt owns frequencies tt, tt+T
+  // entry probe, re/im at the exit probe)
   for (int f = tt; f < 4 * nf; f += T) acc[f] = 0.f;
 
-  float ex[CPT], hy[CPT];
+  float2 ex[NP], hy[NP];
 #pragma unroll
-  for (int c = 0; c < CPT; ++c) ex[c] = hy[c] = 0.f;
-  const bool own_lo = (tt == 0);
-  const int hi_thr = (nx - 1) / CPT;
-  const int hi_c = (nx - 1) - hi_thr * CPT;
-  const bool own_hi = (tt == hi_thr);
-  // the threads (and their cells) holding the source and the two probes
-  const bool own_src = tt == p.src_k / CPT, own_pin = tt == pin / CPT, own_pout = tt == pout / CPT;
-  const int src_c = p.src_k % CPT, pin_c = pin % CPT, pout_c = pout % CPT;
+  for (int k = 0; k < NP; ++k) ex[k] = hy[k] = make_float2(0.f, 0.f);
+  // the lanes (and their cells) that differ: cell 0 and 1, nx-1, the source
+  // (in both copies of an overlap), the probes (in their owner)
+  const bool owned = active && !(lane == 0 && w > 0) && !(lane == 31 && w < nw - 1);
+  auto holds = [&](int k) { return active && k / CPT == g0 / CPT; };
+  // the owner of a cell in an overlap holds it in its half of the lane
+  auto owns = [&](int k) {
+    return holds(k) && (owned || (lane == 31 ? k - g0 < H : k - g0 >= H));
+  };
+  // the cell (in its lane) of a special cell that this warp holds, in the whole
+  // warp, or -1; and the same in the one lane that holds it, -1 in the others
+  auto in_warp = [&](bool mine, int k) { return __any_sync(FULL, mine) ? k % CPT : -1; };
+  const bool src_l = holds(p.src_k), pin_l = owns(pin), pout_l = owns(pout), hi_l = w == nw - 1 && holds(nx - 1);
+  const int src_c = in_warp(src_l, p.src_k), pin_c = in_warp(pin_l, pin), pout_c = in_warp(pout_l, pout),
+            hi_c = in_warp(hi_l, nx - 1);
+  const bool end_probe = pin == nx - 1 || pout == nx - 1;
+  const bool lo_warp = w == 0;
+  const bool special = lo_warp || src_c >= 0 || pin_c >= 0 || pout_c >= 0 || hi_c >= 0;
   float bc0 = 0.f, bc1 = 0.f, bc2 = 0.f, bc3 = 0.f;
-  if (lane == 31) x_last_hy[warp_base + w] = 0.f;
-  team_sync(bar_id, T);
+  const float2 half = make_float2(0.5f, 0.5f);
 
-  for (int t = 1; t <= p.nsteps; ++t) {
-    // DFT factors of this step, loaded early (consumed after barrier A)
-    float cf[2], sf[2];
+  // steps i0 .. i1-1 of an epoch, samples into smp, the epoch's source values vs in lane order;
+  // UNI: every lane in one material; SPEC: the warp holds cells that differ
+  auto steps = [&](auto uni_tag, auto spec_tag, const int i0, const int i1, float* smp, const float vs) {
+    constexpr int PFD = 4;
+    constexpr bool UNI = decltype(uni_tag)::value, SPEC = decltype(spec_tag)::value;
+#pragma unroll 1
+    for (int i = i0; i < i1; ++i) {
+      // ---------------- E stage: ex = ca*ex + cb*(hy[i-1]-hy[i])
+      float4 kc[UNI ? 1 : PFD];  // coefficients of the next PFD pairs, on their way from shared memory
+      if constexpr (!UNI) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int f = tt + k * T;
-      cf[k] = (f < nf) ? __ldg(p.dft_cos + (size_t)(t - 1) * nf + f) : 0.f;
-      sf[k] = (f < nf) ? __ldg(p.dft_sin + (size_t)(t - 1) * nf + f) : 0.f;
-    }
-    const float v = __ldg(p.src_table + t - 1);
-    // ---------------- E stage: ex = ca*ex + cb*(hy[i-1]-hy[i])
-    float hy_left = __shfl_up_sync(FULL, hy[CPT - 1], 1);
-    if (lane == 0) hy_left = (w > 0) ? x_last_hy[warp_base + w - 1] : 0.f;
-    const float ex0 = ex[0];
+        for (int k = 0; k < PFD; ++k) kc[k] = lds4(my_coef + k * 32);
+      }
+      const float hy_left = __shfl_up_sync(FULL, hy[NP - 1].y, 1);
+      const float ex0 = ex[0].x;
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-      const float hym = (c == 0) ? hy_left : hy[c - 1];
-      const float2 k = my_coef[c * 32];
-      ex[c] = ex_update_cacb(ex[c], hym, hy[c], k.x, k.y);
-    }
-    if (own_lo) ex[0] = ex0;  // cell 0 is not E-updated
-    // soft source, fd1d/program/fd1d_1_5.py:67, then the probes read their cells
-    if (own_src) cell_set<CPT>(ex, src_c, __fadd_rn(cell_get<CPT>(ex, src_c), v));
-    if (own_pin) x_probe[0] = cell_get<CPT>(ex, pin_c);
-    if (own_pout) x_probe[1] = cell_get<CPT>(ex, pout_c);
-    // ABC (fd1d/program/fd1d_1_2.py:47-48): low side here, high side's
-    // ex[nx-1] here and its state shift after barrier A
-    if (own_lo) {
-      const float e1 = ex[1];
-      ex[0] = bc0;
-      bc0 = bc1;
-      bc1 = e1;
-    }
-    if (own_hi) cell_set<CPT>(ex, hi_c, bc3);
-    const float prev_last_ex = __shfl_up_sync(FULL, ex[CPT - 1], 1);
-    if (lane == 0) x_first_ex[warp_base + w] = ex[0];
-    if (lane == 31) x_last_ex[warp_base + w] = ex[CPT - 1];
-    team_sync(bar_id, T);  // barrier A
-
-    // ---------------- DFT probes, ABC high-side state, H stage
-    {
-      const float ein = x_probe[0], eout = x_probe[1];
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int f = tt + k * T;
-        if (f < nf) {
-          acc[0 * nf + f] = __fmaf_rn(cf[k], ein, acc[0 * nf + f]);
-          acc[1 * nf + f] = __fmaf_rn(-sf[k], ein, acc[1 * nf + f]);
-          acc[2 * nf + f] = __fmaf_rn(cf[k], eout, acc[2 * nf + f]);
-          acc[3 * nf + f] = __fmaf_rn(-sf[k], eout, acc[3 * nf + f]);
+      for (int k = 0; k < NP; ++k) {
+        const float hym = (k == 0) ? hy_left : hy[k - 1].y;
+        const float2 d = make_float2(__fsub_rn(hym, hy[k].x), __fsub_rn(hy[k].x, hy[k].y));
+        if constexpr (UNI) {
+          ex[k] = __ffma2_rn(ca, ex[k], __fmul2_rn(cb, d));
+        } else {
+          const float4 c = kc[k % PFD];
+          if (k + PFD < NP) kc[k % PFD] = lds4(my_coef + (k + PFD) * 32);
+          ex[k] = __ffma2_rn(make_float2(c.x, c.y), ex[k], __fmul2_rn(make_float2(c.z, c.w), d));
         }
       }
-    }
-    float hy_hi = 0.f;  // hy[nx-1] is never updated: kept across the unmasked H loop
-    if (own_hi) {
-      const float e_nm2 = hi_c >= 1 ? cell_get<CPT>(ex, hi_c - 1)
-                                    : ((lane > 0) ? prev_last_ex : x_last_ex[warp_base + w - 1]);
-      bc3 = bc2;
-      bc2 = e_nm2;
-      hy_hi = cell_get<CPT>(hy, hi_c);
-    }
-    float ex_right = __shfl_down_sync(FULL, ex[0], 1);
-    if (lane == 31) ex_right = (w + 1 < nw) ? x_first_ex[warp_base + w + 1] : 0.f;
+      if constexpr (SPEC) {
+        if (lo_warp) ex[0].x = lane == 0 ? ex0 : ex[0].x;  // cell 0 is not E-updated
+        // soft source, fd1d/program/fd1d_1_5.py:67 (a pulse that has passed adds
+        // exact zeros: skipped), then the probes read their cells
+        const float v = __shfl_sync(FULL, vs, i);
+        if (src_c >= 0 && v != 0.f)
+          cell_at<0, CPT>(src_c, [&](auto K) {
+            float& e = cell<decltype(K)::value>(ex);
+            if (src_l && src_c == K) e = __fadd_rn(e, v);
+          });
+        if (pin_c >= 0) {
+          float e = 0.f;
+          cell_at<0, CPT>(pin_c, [&](auto K) { e = pin_c == K ? cell<decltype(K)::value>(ex) : e; });
+          if (pin_l) smp[i] = e;
+        }
+        if (pout_c >= 0) {
+          float e = 0.f;
+          cell_at<0, CPT>(pout_c, [&](auto K) { e = pout_c == K ? cell<decltype(K)::value>(ex) : e; });
+          if (pout_l) smp[H + i] = e;
+        }
+        // two-step-back ABC (fd1d/program/fd1d_1_2.py:47-48); the state moves
+        // in every lane, only lane 0 and the lane of nx-1 use theirs
+        if (lo_warp) {
+          const float e1 = ex[0].y;
+          ex[0].x = lane == 0 ? bc0 : ex[0].x;
+          bc0 = bc1;
+          bc1 = e1;
+        }
+        if (hi_c >= 0) {
+          float e2 = __shfl_up_sync(FULL, ex[NP - 1].y, 1);  // nx-2 when nx-1 is its lane's first cell
+          cell_at<0, CPT>(hi_c, [&](auto K) {
+            constexpr int k = decltype(K)::value;
+            float& e = cell<k>(ex);
+            if constexpr (k > 0) e2 = hi_c == k ? cell<(k > 0 ? k - 1 : 0)>(ex) : e2;
+            e = hi_l && hi_c == k ? bc3 : e;
+          });
+          bc3 = bc2;
+          bc2 = e2;
+        }
+      }
+      // ---------------- H stage
+      float ex_right = __shfl_down_sync(FULL, ex[0].x, 1);
+      if (SPEC && lane == 31) ex_right = 0.f;  // behind the run's end: keeps the cells there bounded
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) hy[c] = hy_update(hy[c], ex[c], (c == CPT - 1) ? ex_right : ex[c + 1]);
-    if (own_hi) cell_set<CPT>(hy, hi_c, hy_hi);
-    if (lane == 31) x_last_hy[warp_base + w] = hy[CPT - 1];
-    team_sync(bar_id, T);  // barrier B
+      for (int k = 0; k < NP; ++k) {
+        const float er = (k == NP - 1) ? ex_right : ex[k + 1].x;
+        hy[k] = __ffma2_rn(half, make_float2(__fsub_rn(ex[k].x, ex[k].y), __fsub_rn(ex[k].y, er)), hy[k]);
+      }
+      if (SPEC && end_probe && hi_c >= 0)
+        cell_at<0, CPT>(hi_c, [&](auto K) {
+          float& h = cell<decltype(K)::value>(hy);
+          if (hi_l && hi_c == K) h = 0.f;
+        });
+    }
+  };
+
+  // running DFT of an epoch's m samples (steps t+1 ..), in step order: item q =
+  // (frequency, probe), spread evenly over the team's warps
+  auto dft = [&](const float* smp, const int t, const int m) {
+    const int tw = T >> 5;
+    for (int q = lane * tw + w; q < 2 * nf; q += T) {
+      const int f = q >> 1, pr = q & 1;
+      const float* const e = smp + pr * H;
+      const float* const dc = p.dft_cos + (size_t)t * nf + f;
+      const float* const ds = p.dft_sin + (size_t)t * nf + f;
+      float* const a = acc + 2 * pr * nf + f;
+      float re = a[0], im = a[nf];
+#pragma unroll 7
+      for (int i = 0; i < m; ++i) {
+        re = __fmaf_rn(__ldg(dc + (size_t)i * nf), e[i], re);
+        im = __fmaf_rn(-__ldg(ds + (size_t)i * nf), e[i], im);
+      }
+      a[0] = re;
+      a[nf] = im;
+    }
+  };
+
+  team_sync(bar_id, T);  // the accumulators are cleared
+  float vnext = lane < p.nsteps ? __ldg(p.src_table + lane) : 0.f;
+  for (int t = 0, b = 0; t < p.nsteps; t += H, b ^= 1) {
+    const int m = min(H, p.nsteps - t);
+    float* const smp = samples + b * SF;
+    const float vs = vnext;  // the next epoch's source values are on their way while this one runs
+    if (special) vnext = t + H + lane < p.nsteps ? __ldg(p.src_table + t + H + lane) : 0.f;
+    // the DFT of the epoch before is added part-way through this one, at another
+    // step in each of a scheduler's warps: its table reads (L2) are then waited
+    // for while the other warps compute (100 ns of a step's 1150 when all did it
+    // behind the barrier)
+    const int mid = min(m, (wb + w) / 4 * (H / 4));
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+      const int i0 = part ? mid : 0, i1 = part ? m : mid;
+      if (active) {
+        if (special) steps(std::false_type{}, std::true_type{}, i0, i1, smp, vs);
+        else if (uniform) steps(std::true_type{}, std::false_type{}, i0, i1, smp, 0.f);
+        else steps(std::false_type{}, std::false_type{}, i0, i1, smp, 0.f);
+      }
+      if (part == 0 && t > 0) dft(samples + (b ^ 1) * SF, t - H, H);
+    }
+    // exchange of the overlaps' halves; the two buffers alternate, so one
+    // barrier orders both this exchange's reads and the next but one's writes
+    float* const mine = edges + ((size_t)b * MAX_WARPS + wb + w) * 2 * EF;  // [left edge][right edge]
+    if (active) {
+      if (lane == 31 && w < nw - 1) {
+        cells_put<0, H>(ex, mine + EF);
+        cells_put<0, H>(hy, mine + EF + HF);
+      }
+      if (lane == 0 && w > 0) {
+        cells_put<H, H>(ex, mine);
+        cells_put<H, H>(hy, mine + HF);
+      }
+    }
+    team_sync(bar_id, T);
+    if (active) {
+      if (lane == 0 && w > 0) {
+        cells_get<0, H>(ex, mine - EF);  // warp w-1's right edge
+        cells_get<0, H>(hy, mine - EF + HF);
+      }
+      if (lane == 31 && w < nw - 1) {
+        cells_get<H, H>(ex, mine + 2 * EF);  // warp w+1's left edge
+        cells_get<H, H>(hy, mine + 2 * EF + HF);
+      }
+    }
+    if (t + H >= p.nsteps) dft(smp, t, m);  // the last epoch's
   }
+  team_sync(bar_id, T);
   bool fin = true;
   float* sp = A.o.spec + (size_t)run * 4 * nf;
   for (int f = tt; f < 4 * nf; f += T) {
@@ -209,13 +372,11 @@ __device__ void run_team(const BatchArgs& A, int run, int T, int tt, int bar_id,
 template <int CPT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1) k_batch(const BatchArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* coef = reinterpret_cast<float2*>(smem_raw);  // [blockDim * CPT]
-  float* x = reinterpret_cast<float*>(coef + (size_t)blockDim.x * CPT);
-  float* x_last_hy = x;                    // [MAX_WARPS]
-  float* x_first_ex = x + MAX_WARPS;       // [MAX_WARPS]
-  float* x_last_ex = x + 2 * MAX_WARPS;    // [MAX_WARPS]
-  float* x_probe = x + 3 * MAX_WARPS;      // [MAX_WARPS][2] (per team, indexed by its first warp)
-  float* x_acc = x + 5 * MAX_WARPS;        // [MAX_WARPS][4*64] DFT accumulators (per team)
+  float4* coef = reinterpret_cast<float4*>(smem_raw);  // [blockDim * CPT / 2]
+  const int nwarps = blockDim.x >> 5;
+  float* edges = reinterpret_cast<float*>(coef + (size_t)blockDim.x * (CPT / 2));  // [2][MAX_WARPS][2][edge]
+  float* x_smp = edges + (size_t)2 * MAX_WARPS * 2 * edge_floats(CPT);  // [warps][2][samples] (per team, by its first warp)
+  float* x_acc = x_smp + (size_t)nwarps * 2 * sample_floats(CPT);       // [warps][4*64] DFT accumulators (per team)
   __shared__ int s_bundle;
   const long long t_start = clock64();
   for (;;) {
@@ -236,8 +397,8 @@ __global__ void __launch_bounds__(BLOCK, 1) k_batch(const BatchArgs A) {
       const int* en = A.entries + (size_t)e * ENTRY_INTS;
       const int off = en[2], T = en[1];
       if ((int)threadIdx.x >= off && (int)threadIdx.x < off + T) {
-        run_team<CPT>(A, en[0], T, threadIdx.x - off, en[3], off >> 5, coef + (size_t)off * CPT, x_last_hy,
-                      x_first_ex, x_last_ex, x_probe + 2 * (off >> 5), x_acc + (size_t)256 * (off >> 5));
+        run_team<CPT>(A, en[0], T, threadIdx.x - off, en[3], off >> 5, coef + (size_t)(off >> 5) * 32 * (CPT / 2), edges,
+                      x_smp + (size_t)(off >> 5) * 2 * sample_floats(CPT), x_acc + (size_t)256 * (off >> 5));
       }
     }
     __syncthreads();
@@ -248,7 +409,9 @@ __global__ void __launch_bounds__(BLOCK, 1) k_batch(const BatchArgs A) {
 
 // smem bytes of one block
 static size_t batch_smem(int threads, int cpt) {
-  return (size_t)threads * cpt * sizeof(float2) + (size_t)MAX_WARPS * (5 + 256) * sizeof(float);
+  const size_t warps = threads / 32;
+  return (size_t)threads * (cpt / 2) * sizeof(float4) +
+         sizeof(float) * ((size_t)2 * MAX_WARPS * 2 * edge_floats(cpt) + warps * (2 * sample_floats(cpt) + 256));
 }
 
 template <int CPT, int BLOCK>
@@ -379,14 +542,15 @@ int fdtd1d_batch_run(const fdtd1d_batch_params* p, fdtd1d_batch_out* o, const in
   A.bstart = plan_device + 4;
   A.entries = plan_device + 4 + nbundles + 1;
   A.max_cycles = max_cycles;
-  // cells per thread and the largest block each supports (register budget:
-  // 64 per thread for 1024-thread blocks, 128 for 512)
+  // the plan's cells per thread, two more in the kernel's lanes, and the
+  // largest block each supports (register budget: 64 per thread for
+  // 1024-thread blocks, 128 for 512)
   switch (cells_per_thread) {
-    case 8: return fdtd::launch_batch_t<8, 1024>(A, block_threads, ctas_per_sm, st);
-    case 16: return fdtd::launch_batch_t<16, 1024>(A, block_threads, ctas_per_sm, st);
-    case 24: return fdtd::launch_batch_t<24, 512>(A, block_threads, ctas_per_sm, st);
-    case 32: return fdtd::launch_batch_t<32, 512>(A, block_threads, ctas_per_sm, st);
-    case 40: return fdtd::launch_batch_t<40, 512>(A, block_threads, ctas_per_sm, st);
+    case 8: return fdtd::launch_batch_t<10, 1024>(A, block_threads, ctas_per_sm, st);
+    case 16: return fdtd::launch_batch_t<18, 1024>(A, block_threads, ctas_per_sm, st);
+    case 24: return fdtd::launch_batch_t<26, 512>(A, block_threads, ctas_per_sm, st);
+    case 32: return fdtd::launch_batch_t<34, 512>(A, block_threads, ctas_per_sm, st);
+    case 40: return fdtd::launch_batch_t<42, 512>(A, block_threads, ctas_per_sm, st);
     default: return FDTD_ERR_ARG;
   }
 }
