@@ -156,6 +156,11 @@ int fdtd2d_fourier(int t, const fdtd2d_params* p, fdtd2d_state* s, fdtd_stream_t
  * the ping-pong field copies, plus 64 incident-line rows of ny floats with
  * TF/SF on. */
 size_t fdtd2d_workspace_size(const fdtd2d_params* p, int steps_per_pass);
+/* Bytes of device workspace with which fdtd2d_step_n takes its fastest path on
+ * the current device (at least fdtd2d_workspace_size): with them, grids that
+ * fit on the chip run a whole call in one launch.  A smaller workspace, down to
+ * fdtd2d_workspace_size, gives the same results. */
+size_t fdtd2d_fast_workspace_size(const fdtd2d_params* p, int steps_per_pass);
 
 /* fdtd2d_step_n: the program's time loop for t = t0+1 .. t0+nsteps, in the
  * reference's step order (fd2d/python/fd2d_3_4.py:268-277).  The core

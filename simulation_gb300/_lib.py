@@ -126,6 +126,7 @@ _SIGS = {
     "fdtd2d_incth": ([C.POINTER(Params2D), C.POINTER(State2D), P], C.c_int),
     "fdtd2d_fourier": ([C.c_int, C.POINTER(Params2D), C.POINTER(State2D), P], C.c_int),
     "fdtd2d_workspace_size": ([C.POINTER(Params2D), C.c_int], C.c_size_t),
+    "fdtd2d_fast_workspace_size": ([C.POINTER(Params2D), C.c_int], C.c_size_t),
     "fdtd2d_step_n": ([C.POINTER(Params2D), C.POINTER(State2D), C.c_int, C.c_int, C.c_int, P, C.c_size_t, P],
                       C.c_int),
     "fdtd2d_set_march_config": ([C.c_int, C.c_int, C.c_int], C.c_int),

@@ -2,6 +2,7 @@
 #include <vector>
 
 #include "fd2d_internal.cuh"
+#include "fd2d_tile.cuh"
 
 namespace {
 
@@ -87,6 +88,39 @@ size_t line_bytes(const fdtd2d_params* p) {
 }
 size_t fused_workspace_bytes(const fdtd2d_params* p) { return slot_bytes(p) * nslots(p) + line_bytes(p); }
 
+// The on-chip loop (fd2d_tile.cuh): point-source programs whose tiles fit the
+// SMs, with the library's choice of steps per pass.  Its workspace: one
+// exchange set of the evolving fields (as the march's ping-pong set) and the
+// blocks' flags.
+bool tile_ok(const fdtd2d_params* p, int steps_per_pass, TilePlan& pl) {
+  if (ext_on(p) || steps_per_pass != 0) return false;
+  int dev = 0, nsm = 0, coop = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return tile_plan(p->nx, p->ny, p->nbz != nullptr, has_pml(*p), std::min(nsm, kTileMaxBlocks), pl);
+}
+size_t tile_workspace_bytes(const fdtd2d_params* p) { return slot_bytes(p) * nslots(p) + kTileFlagBytes; }
+
+FieldSet workspace_set(const fdtd2d_params* p, void* workspace) {
+  FieldSet ws{};
+  char* base = (char*)workspace;
+  const size_t sb = slot_bytes(p);
+  int k = 0;
+  ws.dz = (float*)(base + sb * k++);
+  ws.hx = (float*)(base + sb * k++);
+  ws.hy = (float*)(base + sb * k++);
+  if (p->nbz) ws.iz = (float*)(base + sb * k++);
+  if (has_pml(*p)) {
+    ws.ihx = (float*)(base + sb * k++);
+    ws.ihy = (float*)(base + sb * k++);
+  }
+  return ws;
+}
+
 // one time step in the reference's order (fd2d/python/fd2d_3_4.py:268-277):
 // ezinct, dfield, inctdz, efield, fourier, hxinct, hfield, incthx, incthy in
 // three launches (launch_step3), bitwise equal to the nine functions
@@ -169,6 +203,13 @@ size_t fdtd2d_workspace_size(const fdtd2d_params* p, int steps_per_pass) {
   return fused_workspace_bytes(p);
 }
 
+size_t fdtd2d_fast_workspace_size(const fdtd2d_params* p, int steps_per_pass) {
+  const size_t need = fdtd2d_workspace_size(p, steps_per_pass);
+  if (!p || p->nx < 3 || p->ny < 3) return 0;
+  TilePlan pl;
+  return tile_ok(p, steps_per_pass, pl) ? std::max(need, tile_workspace_bytes(p)) : need;
+}
+
 int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, int steps_per_pass, void* workspace,
                   size_t workspace_bytes, fdtd_stream_t stream) {
   if (t0 < 0 || nsteps < 0) return FDTD_ERR_ARG;
@@ -177,6 +218,16 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
   if (steps_per_pass < 0 || steps_per_pass > march_max_steps_per_pass()) return FDTD_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   if (nsteps == 0) return FDTD_OK;
+
+  TilePlan tile;
+  // (a call's load and store of the tiles, 15 us at 1024^2, is two march passes: not worth it below 4 steps)
+  if (nsteps >= 4 && workspace && ((uintptr_t)workspace & 255u) == 0 && workspace_bytes >= tile_workspace_bytes(p) &&
+      tile_ok(p, steps_per_pass, tile)) {
+    const FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
+    unsigned* flags = (unsigned*)((char*)workspace + slot_bytes(p) * nslots(p));
+    return launch_tile(*p, user, user, workspace_set(p, workspace), user, s->ez, t0, nsteps, s->status, s->probe_ez,
+                       flags, tile, st);
+  }
 
   if (!fused_ok(p, s) || nsteps == 1) {
     for (int t = t0 + 1; t <= t0 + nsteps; ++t)
@@ -216,20 +267,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
   }
 
   FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
-  FieldSet ws{};
-  {
-    char* base = (char*)workspace;
-    const size_t sb = slot_bytes(p);
-    int k = 0;
-    ws.dz = (float*)(base + sb * k++);
-    ws.hx = (float*)(base + sb * k++);
-    ws.hy = (float*)(base + sb * k++);
-    if (p->nbz) ws.iz = (float*)(base + sb * k++);
-    if (has_pml(*p)) {
-      ws.ihx = (float*)(base + sb * k++);
-      ws.ihy = (float*)(base + sb * k++);
-    }
-  }
+  const FieldSet ws = workspace_set(p, workspace);
   MarchExt ext{};
   float* inc_e = nullptr;
   float* inc_h = nullptr;

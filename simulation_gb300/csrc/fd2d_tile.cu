@@ -1,0 +1,132 @@
+// Launch and layout choice of the on-chip 2D time loop (fd2d_tile.cuh).
+#include "fd2d_tile.cuh"
+
+#include <type_traits>
+
+namespace fdtd {
+
+// The layout with the shortest modelled step among those whose tiles fit the
+// SMs, one block each; false when none does (the caller marches).  The model,
+// in us, fitted to measured layouts with an absorbing layer (the general
+// steps, on which all tiles wait): a step takes 0.35 + 0.27 V (V = 1: 0.58,
+// 2: 0.75, 5: 1.7), loss adds 0.1 V; an exchange 2.1 + 0.52 V (fence, flag and
+// read latencies, and the halo's traffic), once in T steps.  100^2 runs 1.2 a
+// step with V = 1, T = 4 (6.2 marching), 1024^2 3.3 with V = 5, T = 4 (10.5).
+bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& best) {
+  double best_cost = 1e30;
+  for (int V = 1; V <= 5; ++V)
+    for (int T = 2; T <= 8; ++T) {
+      TilePlan pl;
+      pl.V = V;
+      pl.T = T;
+      pl.hc = ny <= kTileCols ? 0 : (T + 3) / 4 * 4;  // whole lanes
+      pl.own_r = kTileWarps * V - 2 * T;
+      pl.own_c = kTileCols - 2 * pl.hc;
+      if (pl.own_r < T) continue;
+      pl.n_ti = (nx + pl.own_r - 1) / pl.own_r;
+      pl.n_tj = (ny + pl.own_c - 1) / pl.own_c;
+      const long blocks = (long)pl.n_ti * pl.n_tj;
+      if (blocks > max_blocks) continue;
+      const double step = 0.35 + V * ((pml ? 0.27 : 0.2) + (lossy ? 0.1 : 0.0));
+      const double cost = step + (blocks > 1 ? (2.1 + 0.52 * V) / T : 0.0);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = pl;
+      }
+    }
+  return best_cost < 1e30;
+}
+
+namespace {
+
+template <int V, bool LOSSY, bool PML>
+int launch_t(const TileArgs& a, cudaStream_t st) {
+  auto kern = k_tile<V, LOSSY, PML>;
+  const size_t smem = tile_smem_bytes(V, LOSSY, PML);
+  cudaError_t e = cudaSuccess;
+  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.n_ti * a.n_tj, 1, 1);
+    cfg.blockDim = dim3(kTileWarps * 32, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;  // all blocks resident: they wait on one another
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, a);
+  }
+  if (e != cudaSuccess) {
+    fdtd_host::note_cuda_error(e);
+    return FDTD_ERR_CUDA;
+  }
+  return fdtd_host::check_launch();
+}
+
+template <int V>
+int launch_v(const TileArgs& a, bool lossy, bool pml, cudaStream_t st) {
+  if (lossy) return pml ? launch_t<V, true, true>(a, st) : launch_t<V, true, false>(a, st);
+  return pml ? launch_t<V, false, true>(a, st) : launch_t<V, false, false>(a, st);
+}
+
+bool al16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+}  // namespace
+
+int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, const FieldSet& x0, const FieldSet& x1,
+                float* ez, int t0, int nsteps, int* status, float* probe_ez, unsigned* flags, const TilePlan& pl,
+                cudaStream_t st) {
+  TileArgs a{};
+  a.nx = p.nx;
+  a.ny = p.ny;
+  a.in = in;
+  a.out = out;
+  a.x[0] = x0;
+  a.x[1] = x1;
+  a.ez = ez;
+  a.naz = p.naz;
+  a.nbz = p.nbz;
+  a.pml = p.pml;
+  a.src_kind = p.src.kind;
+  a.src_i = p.src.i;
+  a.src_j = p.src.j;
+  a.src_table = p.src.table;
+  a.t0 = t0;
+  a.nsteps = nsteps;
+  a.status = status;
+  a.probe_i = p.probe_i;
+  a.probe_j = p.probe_j;
+  a.probe_ez = probe_ez;
+  a.flags = flags;
+  a.T = pl.T;
+  a.hc = pl.hc;
+  a.n_ti = pl.n_ti;
+  a.n_tj = pl.n_tj;
+  a.own_r = pl.own_r;
+  a.own_c = pl.own_c;
+  const bool lossy = p.nbz != nullptr, pml = has_pml(p);
+  bool v = p.ny % 4 == 0 && al16(p.naz) && al16(ez) && (!lossy || al16(p.nbz));
+  for (const FieldSet* f : {&in, &out, &x0, &x1})
+    v = v && al16(f->dz) && al16(f->hx) && al16(f->hy) && (!lossy || al16(f->iz)) &&
+        (!pml || (al16(f->ihx) && al16(f->ihy)));
+  a.vec = v;
+  if (pl.n_ti * pl.n_tj > 1) {
+    const cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)pl.n_ti * pl.n_tj * 128, st);
+    if (e != cudaSuccess) {
+      fdtd_host::note_cuda_error(e);
+      return FDTD_ERR_CUDA;
+    }
+  }
+  switch (pl.V) {
+    case 1: return launch_v<1>(a, lossy, pml, st);
+    case 2: return launch_v<2>(a, lossy, pml, st);
+    case 3: return launch_v<3>(a, lossy, pml, st);
+    case 4: return launch_v<4>(a, lossy, pml, st);
+    case 5: return launch_v<5>(a, lossy, pml, st);
+    default: return FDTD_ERR_ARG;
+  }
+}
+
+}  // namespace fdtd

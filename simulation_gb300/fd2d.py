@@ -188,7 +188,7 @@ class SimTM2D:
             self._tables(max(t_last, 2 * self._ns))
 
     def workspace(self):
-        n = _lib.lib().fdtd2d_workspace_size(self._p, self.steps_per_pass)
+        n = _lib.lib().fdtd2d_fast_workspace_size(self._p, self.steps_per_pass)
         if n and (self._workspace is None or self._workspace.numel() < n):
             self._workspace = torch.empty(n, dtype=torch.uint8, device=self.device)
             self._graphs = {}
