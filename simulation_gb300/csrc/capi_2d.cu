@@ -1,6 +1,7 @@
 // C-ABI entry points of the 2D TM path: argument checks, then launches.
 #include <vector>
 
+#include "fd2d_chain.cuh"
 #include "fd2d_internal.cuh"
 #include "fd2d_tile.cuh"
 
@@ -241,11 +242,13 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
   if (((uintptr_t)workspace & 255u) != 0) return FDTD_ERR_ALIGN;
 
   // pass schedule with an even number of passes, so the last pass writes the
-  // caller's arrays (split one pass if needed)
+  // caller's arrays (split one pass if needed).  Left to the library, large
+  // grids take chained passes of 8 and 4 steps (fd2d_chain.cuh)
+  const bool chain = steps_per_pass == 0 && !ext_on(p) && !s->probe_ez && chain_better(p->nx, p->ny);
   const int K = steps_per_pass == 0 ? march_default_steps(p->nx, p->ny) : steps_per_pass;
   std::vector<int> sched;
   for (int rem = nsteps; rem > 0;) {
-    const int k = rem < K ? rem : K;
+    const int k = chain && rem >= 8 ? 8 : rem < K ? rem : K;
     sched.push_back(k);
     rem -= k;
   }
@@ -297,8 +300,12 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
     // Inf/NaN yields Inf/NaN, and it spreads to the neighbours each step), so
     // that one test sees anything an earlier pass would have
     int* status = (i + 1 == sched.size()) ? s->status : nullptr;
-    if (!ext_on(p)) {
-      rc = launch_march(*p, in, out, s->ez, t, sched[i], status, s->probe_ez, st);
+    // ez is a result of the call, not an input of the passes: only the last stores it
+    float* ez = (i + 1 == sched.size()) ? s->ez : nullptr;
+    if (chain && (sched[i] == 8 || sched[i] == 4)) {
+      rc = launch_chain(*p, in, out, ez, t, sched[i] / 4, status, march_gen_cost(), st);
+    } else if (!ext_on(p)) {
+      rc = launch_march(*p, in, out, ez, t, sched[i], status, s->probe_ez, st);
     } else {
       if (p->tfsf_npml > 0) {
         if (t + sched[i] > line_t0 + line_n) {  // next chunk of whole passes
@@ -311,7 +318,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
         ext.inc_e = inc_e + (size_t)(t - line_t0) * p->ny;
         ext.inc_h = inc_h + (size_t)(t - line_t0) * 2;
       }
-      rc = launch_march_ext(*p, in, out, s->ez, t, sched[i], status, ext, st);
+      rc = launch_march_ext(*p, in, out, ez, t, sched[i], status, ext, st);
     }
     if (rc) return rc;
     t += sched[i];

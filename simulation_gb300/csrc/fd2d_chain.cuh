@@ -1,0 +1,422 @@
+// Fused 2D pass of 4 or 8 time steps for large grids: the streaming march
+// (fd2d_march.cuh) in chains of warps.
+//
+// A pass moves 56 bytes per cell (6 evolving fields in and out, two
+// materials; ez only in a call's last pass) whatever its number of steps K,
+// so large grids are bound by 56/K bytes per cell-update: the K = 4 march ran
+// at 85% of the copy bandwidth and could only gain by more steps.  Four steps
+// of state fill a warp's registers, so K = 8 is two warps in a chain: the
+// first does steps 1-4 of a row and hands it, through a ring in shared memory,
+// to the second, which does steps 5-8 and stores it.
+//
+// A block is one chain: it owns a stripe of 128 columns (4 per lane, K on each
+// side recomputed by the neighbours) and marches down a segment of rows.  At
+// iteration r level s of a warp (s = 0..3) does D and E of row r-s and H of
+// row r-s-1.  A row's values stay in the same registers through all four
+// levels: five rows are in flight, row r in register set r mod 5, and the loop
+// is unrolled by five rows, so no value ever moves (the march's register
+// shifts were a third of its instructions).  Updates are packed two cells to
+// an instruction.  Input rows arrive by cp.async three rows ahead.
+//
+// Blocks of five rows run in one of two forms, as in the march: interior (unit
+// coefficients, nothing that the reference's loops leave out, no source) or
+// general, decided on the coefficient vectors themselves.  Same per-cell
+// formulas and order as the per-function kernels: bitwise equal results.
+#pragma once
+
+#include <type_traits>
+
+#include "fd2d_internal.cuh"
+#include "fd2d_pack.cuh"
+
+namespace fdtd {
+
+constexpr int kChainCols = 128;
+constexpr int kChainAhead = 3;  // rows between a row's cp.async and its use
+constexpr int kChainLag = 9;    // rows by which a warp's level 0 is behind that of the warp before it
+// rows of the material ring: from 3 ahead of the first warp's to the second's
+// level 4, 12 behind, in whole blocks of five
+constexpr int kChainMat = 20;
+
+struct ChainArgs {
+  int nx, ny;
+  FieldSet in, out;
+  float* ez;  // null: not stored by this pass
+  const float* naz;
+  const float* nbz;
+  fdtd2d_pml pml;
+  int src_kind, src_i, src_j;
+  const float* src_table;
+  int t0;
+  int* status;  // null: no Inf/NaN test
+  // blocks 0 .. n_int*n_segs-1: the stripes away from the edges; then the
+  // general stripes at either edge with their shorter segments
+  int n_stripes, n_gen_lo, n_gen_hi, n_segs, seg_first, seg_rows, n_segs_g, seg_rows_g;
+};
+
+// floats of a block's shared memory: field ring [5 rows][fields][128], one
+// hand-over ring of the same size per link of the chain, material ring
+// [20 rows][1 or 2][128], column coefficients [5][128]
+__host__ __device__ constexpr int chain_fields(bool lossy, bool pml) { return 3 + (lossy ? 1 : 0) + (pml ? 2 : 0); }
+__host__ __device__ constexpr size_t chain_smem_bytes(int nc, bool lossy, bool pml) {
+  return sizeof(float) * kChainCols *
+         ((size_t)nc * 5 * chain_fields(lossy, pml) + kChainMat * (lossy ? 2 : 1) + (pml ? 5 : 0));
+}
+
+// block -> stripe and rows; false: no work
+__host__ __device__ inline bool chain_work(const ChainArgs& a, int b, int& stripe, int& i_s, int& i_e) {
+  const int n_int = a.n_stripes - a.n_gen_lo - a.n_gen_hi, n_main = n_int * a.n_segs;
+  if (b < n_main) {
+    stripe = a.n_gen_lo + b % n_int;
+    const int seg = b / n_int;
+    i_s = seg == 0 ? 0 : a.seg_first + (seg - 1) * a.seg_rows;
+    i_e = seg == a.n_segs - 1 ? a.nx : seg == 0 ? a.seg_first : i_s + a.seg_rows;
+  } else {
+    const int n_gen = a.n_gen_lo + a.n_gen_hi;
+    if (n_gen == 0) return false;
+    const int k = b - n_main, g = k % n_gen, seg = k / n_gen;
+    if (seg >= a.n_segs_g) return false;
+    stripe = g < a.n_gen_lo ? g : a.n_stripes - n_gen + g;
+    i_s = seg * a.seg_rows_g;
+    i_e = i_s + a.seg_rows_g;
+  }
+  i_e = i_e < a.nx ? i_e : a.nx;
+  return i_s < i_e;
+}
+
+// One wave of blocks over the grid: the stripes that the absorbing layer (P
+// cells, 0: unknown) or the grid's edge makes general get gen_cost times as
+// many segments, and the other stripes' first and last segments are shortened
+// by the time of their general rows.  Returns the number of blocks.
+inline long chain_layout(ChainArgs& a, int K, long resident, int P, float gen_cost) {
+  const int outw = kChainCols - 2 * K;
+  a.n_stripes = (a.ny + outw - 1) / outw;
+  auto general = [&](int s) {
+    const int lo = s * outw - K, hi = lo + kChainCols - 1;
+    return lo < std::max(P, 1) || hi > a.ny - 2 - P;
+  };
+  int glo = 0, ghi = 0;
+  while (glo < a.n_stripes && general(glo)) ++glo;
+  while (ghi < a.n_stripes - glo && general(a.n_stripes - 1 - ghi)) ++ghi;
+  const int n_int = a.n_stripes - glo - ghi, n_gen = glo + ghi, mn = 4 * K;
+  const double G = gen_cost >= 1.f ? gen_cost : 1.0;
+  const long n_segs = std::max(1L, (long)((double)resident / (n_int + G * n_gen)));
+  const long n_segs_g = std::max(1L, (long)(G * n_segs));
+  a.seg_rows_g = std::max((int)((a.nx + n_segs_g - 1) / n_segs_g), mn);
+  a.n_segs_g = (a.nx + a.seg_rows_g - 1) / a.seg_rows_g;
+  const int T = (int)((G - 1.0) * (P + K + 1));
+  int L = a.nx, f = a.nx, ns = 1;
+  if (n_segs > 1) {
+    L = std::max((int)((a.nx + 2L * T + n_segs - 1) / n_segs), mn);
+    f = std::min(std::max(L - T, mn), a.nx);
+    ns = a.nx <= f ? 1 : 1 + (a.nx - f + L - 1) / L;
+  }
+  a.seg_rows = L;
+  a.seg_first = f;
+  a.n_segs = ns;
+  a.n_gen_lo = glo;
+  a.n_gen_hi = ghi;
+  return (long)n_int * ns + (long)n_gen * a.n_segs_g;
+}
+
+// one pass of 4*nc steps (fd2d_chain.cu); FDTD_ERR_UNSUPPORTED where the march
+// is the faster form
+int launch_chain(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int nc, int* status,
+                 float gen_cost, cudaStream_t st);
+
+namespace {
+
+__device__ __forceinline__ void chain_cp16(float* dst, const float* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(ok ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ F4 chain_lds(const float* p) { return f4(*reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ void chain_sts(float* p, const F4& v) { *reinterpret_cast<float4*>(p) = to4(v); }
+__device__ __forceinline__ bool chain_finite(const F4& v) {
+  return isfinite(v.a.x) && isfinite(v.a.y) && isfinite(v.b.x) && isfinite(v.b.y);
+}
+
+struct ChainRow {
+  F4 dz, iz, hx, hy, ihx, ihy, ez;
+};
+
+template <int NC, bool LOSSY, bool PML>
+__global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ ChainArgs a) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int W = kChainCols, K = 4 * NC, HB = K;  // halo columns on each side (whole lanes)
+  constexpr int NF = chain_fields(LOSSY, PML), NM = LOSSY ? 2 : 1;
+  constexpr int F_IZ = 3, F_IHX = 3 + (LOSSY ? 1 : 0), F_IHY = F_IHX + 1;
+  constexpr int MT = kChainMat;
+  extern __shared__ float4 chain_sm[];
+  int stripe, i_s, i_e;
+  if (!chain_work(a, blockIdx.x, stripe, i_s, i_e)) return;  // the whole block
+
+  const int lane = threadIdx.x & 31, cw = threadIdx.x >> 5;
+  const int nx = a.nx, ny = a.ny;
+  const int j0 = stripe * (W - 2 * HB) - HB + lane * 4;
+  const bool vin = j0 >= 0 && j0 + 4 <= ny;  // ny % 4 == 0: a lane's vector is wholly in or out
+  const bool vout = vin && lane * 4 >= HB && lane * 4 < W - HB;
+  float* const sm = reinterpret_cast<float*>(chain_sm) + lane * 4;
+  float* const fin_ring = sm + cw * 5 * NF * W;                // rows into this warp
+  float* const fout_ring = sm + (cw + 1) * 5 * NF * W;         // rows out of it (not the last warp's)
+  float* const mring = sm + NC * 5 * NF * W;                   // [20][NM][W], row r in slot r mod 20
+  float* const cc = mring + MT * NM * W;                       // [5][W] gy2/2, gy3, fy1, fy2, fy3
+
+  // ---- columns
+  bool col_ok = j0 >= 1 && j0 + 3 <= ny - 2;
+  if (PML) {
+    float v[5][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int j = j0 + c;
+      const bool in = j >= 0 && j < ny;
+      v[0][c] = 0.5f * (in ? __ldg(a.pml.gy2 + j) : 1.f);  // exact
+      v[1][c] = in ? __ldg(a.pml.gy3 + j) : 1.f;
+      v[2][c] = in ? __ldg(a.pml.fy1 + j) : 0.f;
+      v[3][c] = in ? __ldg(a.pml.fy2 + j) : 1.f;
+      v[4][c] = in ? __ldg(a.pml.fy3 + j) : 1.f;
+      col_ok &= v[0][c] == 0.5f && v[1][c] == 1.f && v[2][c] == 0.f && v[3][c] == 1.f && v[4][c] == 1.f;
+    }
+    if (cw == 0)
+#pragma unroll
+      for (int k = 0; k < 5; ++k) chain_sts(cc + k * W, f4(make_float4(v[k][0], v[k][1], v[k][2], v[k][3])));
+  }
+  const bool cint = __all_sync(kAll, col_ok);
+  const bool src_here = a.src_kind != FDTD_SRC_NONE && a.src_j >= j0 - lane * 4 && a.src_j < j0 - lane * 4 + W;
+  const bool col0 = j0 == 0, last_col = j0 + 4 == ny;
+
+  // bit l: row b+l may be touched by an interior iteration
+  auto rows_ok = [&](int b) -> unsigned {
+    const int row = b + lane;
+    bool g = row >= 1 && row <= nx - 2;
+    if (PML && g)
+      g = __ldg(a.pml.gx2 + row) == 1.f && __ldg(a.pml.gx3 + row) == 1.f && __ldg(a.pml.fx1 + row) == 0.f &&
+          __ldg(a.pml.fx2 + row) == 1.f && __ldg(a.pml.fx3 + row) == 1.f;
+    if (src_here && row == a.src_i) g = false;
+    return __ballot_sync(kAll, g);
+  };
+
+  // ---- rows on their way in (first warp): fields into ring slot `slot`,
+  // materials into theirs; zeros outside the grid
+  auto fetch = [&](int row, int slot, int mslot) {
+    const bool ok = vin && row >= 0 && row < nx;
+    const size_t off = ok ? (size_t)row * ny + j0 : 0;
+    float* const f = fin_ring + slot * NF * W;
+    chain_cp16(f + 0 * W, a.in.dz + off, ok);
+    chain_cp16(f + 1 * W, a.in.hx + off, ok);
+    chain_cp16(f + 2 * W, a.in.hy + off, ok);
+    if (LOSSY) chain_cp16(f + F_IZ * W, a.in.iz + off, ok);
+    if (PML) {
+      chain_cp16(f + F_IHX * W, a.in.ihx + off, ok);
+      chain_cp16(f + F_IHY * W, a.in.ihy + off, ok);
+    }
+    float* const m = mring + mslot * NM * W;
+    chain_cp16(m, a.naz + off, ok);
+    if (LOSSY) chain_cp16(m + W, a.nbz + off, ok);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+
+  const F4 zero = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  ChainRow R[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) R[k].dz = R[k].iz = R[k].hx = R[k].hy = R[k].ihx = R[k].ihy = R[k].ez = zero;
+  // rows before the first that is read: no output depends on them
+  if (cw == 0) {
+    for (int k = 0; k < MT * NM; ++k) chain_sts(mring + k * W, zero);
+    for (int k = 5 * NF; k < NC * 5 * NF; ++k) chain_sts(sm + k * W, zero);
+  }
+  __syncthreads();
+  const int first = i_s - K;
+  const int b0 = (first >= 0 ? first / 5 : -((4 - first) / 5)) * 5;  // first row, of a block of five
+  int rb = b0 - kChainLag * cw;                                       // this warp's level-0 row
+  int ms = ((rb - 3) % MT + MT) % MT + 3;                             // material slot of row rb, in 3 .. 22
+  if (cw == 0) {
+#pragma unroll
+    for (int k = 0; k < kChainAhead; ++k) fetch(rb + k, k, (ms + k) % MT);
+  }
+  bool fin = true;
+
+  // ---- iteration I of the block of five that starts at row rb: this warp's
+  // level 0 takes row rb+I
+  auto iterate = [&](auto itag, auto inttag) {
+    constexpr int I = decltype(itag)::value;
+    constexpr bool INT = decltype(inttag)::value;
+    const int r = rb + I;
+    if (cw == 0) {  // row r+3 starts its way in; row r's copies complete
+      const int mf = ms + I + kChainAhead;
+      fetch(r + kChainAhead, (I + kChainAhead) % 5, mf >= MT ? mf - MT : mf);
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kChainAhead) : "memory");
+    }
+    {
+      const float* const f = fin_ring + I * NF * W;
+      ChainRow& q = R[I];
+      q.dz = chain_lds(f + 0 * W);
+      q.hx = chain_lds(f + 1 * W);
+      q.hy = chain_lds(f + 2 * W);
+      if (LOSSY) q.iz = chain_lds(f + F_IZ * W);
+      if (PML) {
+        q.ihx = chain_lds(f + F_IHX * W);
+        q.ihy = chain_lds(f + F_IHY * W);
+      }
+    }
+    // every warp has taken slot I: the warp before may refill it below
+    if (NC > 1) __syncthreads();
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int qi = (I - s + 5) % 5, pi = (I - s + 4) % 5;
+      ChainRow &q = R[qi], &p = R[pi];
+      const int row = r - s;
+      const int t = a.t0 + 4 * cw + s;  // table row of this level's time step
+      // D and E on row r-s
+      const float hl = __shfl_up_sync(kAll, q.hx.b.y, 1);
+      const F4 d = sub4(sub4(q.hy, p.hy), q.hx);
+      const F4 curl = {make_float2(__fadd_rn(d.a.x, hl), __fadd_rn(d.a.y, q.hx.a.x)),
+                       make_float2(__fadd_rn(d.b.x, q.hx.a.y), __fadd_rn(d.b.y, q.hx.b.x))};
+      if (INT) {
+        q.dz = add4(q.dz, mul4(0.5f, curl));
+      } else {
+        F4 nd;
+        const bool in = row >= 1 && row < nx;
+        if (PML) {
+          const float gx2 = in ? __ldg(a.pml.gx2 + row) : 1.f, gx3 = in ? __ldg(a.pml.gx3 + row) : 1.f;
+          // gx2*(gy2/2) is (gx2*gy2)/2 exactly
+          nd = fma4(mul4(gx3, chain_lds(cc + 1 * W)), q.dz, mul4(mul4(gx2, chain_lds(cc + 0 * W)), curl));
+        } else {
+          nd = add4(q.dz, mul4(0.5f, curl));
+        }
+        q.dz.a.x = in && !col0 ? nd.a.x : q.dz.a.x;
+        q.dz.a.y = in ? nd.a.y : q.dz.a.y;
+        q.dz.b.x = in ? nd.b.x : q.dz.b.x;
+        q.dz.b.y = in ? nd.b.y : q.dz.b.y;
+        if (src_here && row == a.src_i) {
+          const float v = __ldg(a.src_table + t);
+          auto put = [&](float& x, int j) {
+            if (j == a.src_j) x = a.src_kind == FDTD_SRC_HARD ? v : __fadd_rn(x, v);
+          };
+          put(q.dz.a.x, j0);
+          put(q.dz.a.y, j0 + 1);
+          put(q.dz.b.x, j0 + 2);
+          put(q.dz.b.y, j0 + 3);
+        }
+      }
+      const int mi = ms + I - s;
+      const float* const m = mring + (mi >= MT ? mi - MT : mi) * NM * W;
+      const F4 na = chain_lds(m);
+      if (LOSSY) {
+        q.ez = mul4(na, sub4(q.dz, q.iz));
+        q.iz = fma4(chain_lds(m + W), q.ez, q.iz);
+      } else {
+        q.ez = mul4(na, q.dz);
+      }
+      // H on row r-s-1
+      const float er = __shfl_down_sync(kAll, p.ez.a.x, 1);
+      const F4 cx = {make_float2(__fsub_rn(p.ez.a.x, p.ez.a.y), __fsub_rn(p.ez.a.y, p.ez.b.x)),
+                     make_float2(__fsub_rn(p.ez.b.x, p.ez.b.y), __fsub_rn(p.ez.b.y, er))};
+      const F4 cy = sub4(p.ez, q.ez);
+      if (INT) {
+        if (PML) {
+          p.ihx = add4(p.ihx, cx);
+          p.ihy = add4(p.ihy, cy);
+          p.hx = add4(p.hx, mul4(0.5f, cx));
+          p.hy = sub4(p.hy, mul4(0.5f, cy));
+        } else {
+          p.hx = fma4(0.5f, cx, p.hx);
+          p.hy = fma4(-0.5f, cy, p.hy);
+        }
+      } else {
+        const int pr = row - 1;
+        const bool in = pr >= 0 && pr <= nx - 2;
+        F4 nhx, nhy, nix, niy;
+        if (PML) {
+          const float fx1 = in ? __ldg(a.pml.fx1 + pr) : 0.f, fx2 = in ? __ldg(a.pml.fx2 + pr) : 1.f,
+                      fx3 = in ? __ldg(a.pml.fx3 + pr) : 1.f;
+          nix = add4(p.ihx, cx);
+          niy = add4(p.ihy, cy);
+          nhx = fma4(chain_lds(cc + 4 * W), p.hx, mul4(chain_lds(cc + 3 * W), fma4(fx1, nix, mul4(0.5f, cx))));
+          // (-fx2)*z is -(fx2*z) exactly
+          nhy = fma4(fx3, p.hy, mul4(-fx2, fma4(chain_lds(cc + 2 * W), niy, mul4(0.5f, cy))));
+        } else {
+          nhx = fma4(0.5f, cx, p.hx);
+          nhy = fma4(-0.5f, cy, p.hy);
+        }
+        // row nx-1 and column ny-1 (the last of its lane) are not updated
+        auto take = [&](F4& x, const F4& nw) {
+          x.a.x = in ? nw.a.x : x.a.x;
+          x.a.y = in ? nw.a.y : x.a.y;
+          x.b.x = in ? nw.b.x : x.b.x;
+          x.b.y = in && !last_col ? nw.b.y : x.b.y;
+        };
+        take(p.hx, nhx);
+        take(p.hy, nhy);
+        if (PML) {
+          take(p.ihx, nix);
+          take(p.ihy, niy);
+        }
+      }
+    }
+    // ---- row r-4 is complete: to the next warp's ring, or out
+    ChainRow& c = R[(I + 1) % 5];
+    if (NC > 1 && cw < NC - 1) {
+      float* const f = fout_ring + I * NF * W;
+      chain_sts(f + 0 * W, c.dz);
+      chain_sts(f + 1 * W, c.hx);
+      chain_sts(f + 2 * W, c.hy);
+      if (LOSSY) chain_sts(f + F_IZ * W, c.iz);
+      if (PML) {
+        chain_sts(f + F_IHX * W, c.ihx);
+        chain_sts(f + F_IHY * W, c.ihy);
+      }
+    } else {
+      const int row = r - 4;
+      if (vout && row >= i_s && row < i_e) {
+        const size_t off = (size_t)row * ny + j0;
+        auto st = [&](float* p, const F4& v) { __stcs(reinterpret_cast<float4*>(p + off), to4(v)); };
+        st(a.out.dz, c.dz);
+        st(a.out.hx, c.hx);
+        st(a.out.hy, c.hy);
+        if (LOSSY) st(a.out.iz, c.iz);
+        if (PML) {
+          st(a.out.ihx, c.ihx);
+          st(a.out.ihy, c.ihy);
+        }
+        if (a.ez) st(a.ez, c.ez);
+        if (a.status) {
+          fin &= chain_finite(c.dz) && chain_finite(c.hx) && chain_finite(c.hy) && chain_finite(c.ez);
+          if (LOSSY) fin &= chain_finite(c.iz);
+          if (PML) fin &= chain_finite(c.ihx) && chain_finite(c.ihy);
+        }
+      }
+    }
+  };
+  auto five = [&](auto inttag) {
+    iterate(std::integral_constant<int, 0>{}, inttag);
+    iterate(std::integral_constant<int, 1>{}, inttag);
+    iterate(std::integral_constant<int, 2>{}, inttag);
+    iterate(std::integral_constant<int, 3>{}, inttag);
+    iterate(std::integral_constant<int, 4>{}, inttag);
+  };
+
+  // ---- down the segment: the last warp's level 4 has to complete row i_e-1
+  const int n_blk = (i_e - 1 + kChainLag * (NC - 1) - b0 + 4) / 5 + 1;
+  int gb = rb - 4;  // rows gb .. gb+63 are in gm
+  unsigned long long gm = cint ? rows_ok(gb) | (unsigned long long)rows_ok(gb + 32) << 32 : 0ull;
+  for (int k = 0; k < n_blk; ++k) {
+    bool interior = false;  // the nine rows rb-4 .. rb+4 that the five iterations touch
+    if (cint) {
+      if (rb + 4 - gb >= 64) {
+        gb += 32;
+        gm = gm >> 32 | (unsigned long long)rows_ok(gb + 32) << 32;
+      }
+      interior = ((gm >> (rb - 4 - gb)) & 0x1ffull) == 0x1ffull;
+    }
+    if (interior) five(std::true_type{});
+    else five(std::false_type{});
+    rb += 5;
+    ms = ms + 5 >= MT + 3 ? ms + 5 - MT : ms + 5;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (a.status && __any_sync(kAll, !fin) && lane == 0) raise_status(a.status, ST_NONFINITE);
+}
+
+}  // namespace
+}  // namespace fdtd

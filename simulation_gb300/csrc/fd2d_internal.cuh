@@ -38,6 +38,11 @@ int launch_march(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out
 int march_max_steps_per_pass();
 // steps per pass the library picks for a grid (steps_per_pass = 0)
 int march_default_steps(int nx, int ny);
+// the caller's balance knob (fdtd2d_set_march_balance; 0: default)
+float march_gen_cost();
+// whether large-grid passes go through the chained kernel (fd2d_chain.cuh):
+// grids that do not fit on the chip, without a caller's own march shape
+bool chain_better(int nx, int ny);
 // A pass that also records the state after each of its steps (the adjoint's
 // recompute): rec[s] receives dz, iz, hx, hy after step t0+s+1, s < k.
 // Point source only, with PML (plain kernels, 64-column stripes).

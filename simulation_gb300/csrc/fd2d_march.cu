@@ -47,6 +47,13 @@ int march_max_steps_per_pass() { return HALO; }
 // GPU); at 2048^2 and above 4 are fastest (18.4 against 29.8 us).
 int march_default_steps(int nx, int ny) { return (long long)nx * ny < (1LL << 21) ? 2 : HALO; }
 
+float march_gen_cost() { return g_cfg.gen_cost; }
+
+bool chain_better(int nx, int ny) {
+  if (g_cfg.cpl || g_cfg.seg_rows) return false;
+  return (long long)nx * ny >= (1LL << 20) && nx >= 64 && ny >= 128;
+}
+
 namespace {
 MarchArgs march_args(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0,
                      int* status, float* probe_ez) {

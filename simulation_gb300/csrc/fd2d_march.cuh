@@ -62,7 +62,7 @@ constexpr int kTraceNone = 0, kTraceProbe = 1, kTraceRecord = 2;  // what a plai
 struct MarchArgs {
   int nx, ny;
   FieldSet in, out;
-  float* ez;
+  float* ez;  // null: not stored by this pass
   const float* naz;
   const float* nbz;
   fdtd2d_pml pml;
@@ -650,7 +650,7 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, const int stripe,
         st_row<CPL>(a.out.dz + off, p_dz[s]);
         st_row<CPL>(a.out.hx + off, ohx);
         st_row<CPL>(a.out.hy + off, ohy);
-        st_row<CPL>(a.ez + off, p_ez[s]);
+        if (a.ez) st_row<CPL>(a.ez + off, p_ez[s]);
         if (LOSSY) st_row<CPL>(a.out.iz + off, p_iz[s]);
         if (PML) {
           st_row<CPL>(a.out.ihx + off, oihx);

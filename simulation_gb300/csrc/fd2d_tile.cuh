@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "fd2d_internal.cuh"
+#include "fd2d_pack.cuh"
 
 namespace fdtd {
 
@@ -92,28 +93,6 @@ constexpr int kTileEdge = 2;   // and row 0, row nx-1 or column ny-1 anywhere: t
 constexpr int kTilePoint = 3;  // and the source or the probe
 
 namespace {
-
-struct F4 {  // four cells of a lane as two packed pairs
-  float2 a, b;
-};
-__device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 sub2(float2 x, float2 y) { return __ffma2_rn(y, bc2(-1.f), x); }  // x - y, rounded once
-__device__ __forceinline__ F4 f4(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
-__device__ __forceinline__ float4 to4(const F4& v) { return make_float4(v.a.x, v.a.y, v.b.x, v.b.y); }
-__device__ __forceinline__ F4 sub4(const F4& x, const F4& y) { return {sub2(x.a, y.a), sub2(x.b, y.b)}; }
-__device__ __forceinline__ F4 add4(const F4& x, const F4& y) { return {__fadd2_rn(x.a, y.a), __fadd2_rn(x.b, y.b)}; }
-__device__ __forceinline__ F4 mul4(const F4& x, const F4& y) { return {__fmul2_rn(x.a, y.a), __fmul2_rn(x.b, y.b)}; }
-__device__ __forceinline__ F4 mul4(float s, const F4& y) { return {__fmul2_rn(bc2(s), y.a), __fmul2_rn(bc2(s), y.b)}; }
-__device__ __forceinline__ F4 fma4(const F4& x, const F4& y, const F4& z) {
-  return {__ffma2_rn(x.a, y.a, z.a), __ffma2_rn(x.b, y.b, z.b)};
-}
-__device__ __forceinline__ F4 mul4(float2 s, const F4& y) { return {__fmul2_rn(s, y.a), __fmul2_rn(s, y.b)}; }
-__device__ __forceinline__ F4 fma4(float2 s, const F4& y, const F4& z) {
-  return {__ffma2_rn(s, y.a, z.a), __ffma2_rn(s, y.b, z.b)};
-}
-__device__ __forceinline__ F4 fma4(float s, const F4& y, const F4& z) {
-  return {__ffma2_rn(bc2(s), y.a, z.a), __ffma2_rn(bc2(s), y.b, z.b)};
-}
 
 // one lane's four columns of row i from or to global memory, past L1 (other
 // blocks write them); columns outside the grid read as 0
