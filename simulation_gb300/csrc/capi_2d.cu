@@ -303,7 +303,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
     // ez is a result of the call, not an input of the passes: only the last stores it
     float* ez = (i + 1 == sched.size()) ? s->ez : nullptr;
     if (chain && (sched[i] == 8 || sched[i] == 4)) {
-      rc = launch_chain(*p, in, out, ez, t, sched[i] / 4, status, march_gen_cost(), st);
+      rc = launch_chain(*p, in, out, ez, t, sched[i] / kChainLv, status, march_gen_cost(), st);
     } else if (!ext_on(p)) {
       rc = launch_march(*p, in, out, ez, t, sched[i], status, s->probe_ez, st);
     } else {

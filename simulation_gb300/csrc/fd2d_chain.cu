@@ -18,7 +18,7 @@ int launch_t(ChainArgs a, int pml_cells, float gen_cost, cudaStream_t st) {
     fdtd_host::note_cuda_error(e);
     return FDTD_ERR_CUDA;
   }
-  const long blocks = chain_layout(a, 4 * NC, (long)nsm * std::max(per_sm, 1), pml_cells, gen_cost > 0.f ? gen_cost : 2.5f);
+  const long blocks = chain_layout(a, kChainLv * NC, (long)nsm * std::max(per_sm, 1), pml_cells, gen_cost > 0.f ? gen_cost : 2.5f);
   kern<<<(unsigned)blocks, 32 * NC, smem, st>>>(a);
   return fdtd_host::check_launch();
 }
@@ -49,8 +49,8 @@ int launch_chain(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out
   a.t0 = t0;
   a.status = status;
   const bool lossy = p.nbz != nullptr, pml = has_pml(p);
-  if (nc == 1) return launch_nc<1>(a, lossy, pml, p.pml_cells, gen_cost, st);
   if (nc == 2) return launch_nc<2>(a, lossy, pml, p.pml_cells, gen_cost, st);
+  if (nc == 4) return launch_nc<4>(a, lossy, pml, p.pml_cells, gen_cost, st);
   return FDTD_ERR_ARG;
 }
 

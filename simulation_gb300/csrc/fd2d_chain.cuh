@@ -4,21 +4,24 @@
 // A pass moves 56 bytes per cell (6 evolving fields in and out, two
 // materials; ez only in a call's last pass) whatever its number of steps K,
 // so large grids are bound by 56/K bytes per cell-update: the K = 4 march ran
-// at 85% of the copy bandwidth and could only gain by more steps.  Four steps
-// of state fill a warp's registers, so K = 8 is two warps in a chain: the
-// first does steps 1-4 of a row and hands it, through a ring in shared memory,
-// to the second, which does steps 5-8 and stores it.
+// at 85% of the copy bandwidth and could only gain by more steps per pass,
+// whose state does not fit one warp's registers.  K = 8 is four warps in a
+// chain, two steps each: a warp hands its rows through a ring in shared memory
+// to the next, the last stores them.
 //
 // A block is one chain: it owns a stripe of 128 columns (4 per lane, K on each
 // side recomputed by the neighbours) and marches down a segment of rows.  At
-// iteration r level s of a warp (s = 0..3) does D and E of row r-s and H of
-// row r-s-1.  A row's values stay in the same registers through all four
-// levels: five rows are in flight, row r in register set r mod 5, and the loop
-// is unrolled by five rows, so no value ever moves (the march's register
-// shifts were a third of its instructions).  Updates are packed two cells to
-// an instruction.  Input rows arrive by cp.async three rows ahead.
+// iteration r level s of a warp (s = 0, 1) does D and E of row r-s and H of
+// row r-s-1.  A row's values stay in the same registers through both levels:
+// three rows are in flight, row r in register set r mod 3, and the loop is
+// unrolled by three rows, so no value ever moves (the march's register shifts
+// were a third of its instructions).  Two steps a warp rather than four: four
+// need five rows and a body of 20 levels, 21 KB of code, whose fetch stalled
+// each issue by 1.5 cycles.  Updates are packed two cells to an instruction.
+// Input rows arrive by cp.async five rows ahead.  One block barrier per row
+// keeps the chain in step.
 //
-// Blocks of five rows run in one of two forms, as in the march: interior (unit
+// Blocks of three rows run in one of two forms, as in the march: interior (unit
 // coefficients, nothing that the reference's loops leave out, no source) or
 // general, decided on the coefficient vectors themselves.  Same per-cell
 // formulas and order as the per-function kernels: bitwise equal results.
@@ -32,11 +35,15 @@
 namespace fdtd {
 
 constexpr int kChainCols = 128;
-constexpr int kChainAhead = 3;  // rows between a row's cp.async and its use
-constexpr int kChainLag = 9;    // rows by which a warp's level 0 is behind that of the warp before it
-// rows of the material ring: from 3 ahead of the first warp's to the second's
-// level 4, 12 behind, in whole blocks of five
-constexpr int kChainMat = 20;
+constexpr int kChainLv = 2;                // time steps (levels) per warp
+constexpr int kChainRf = kChainLv + 1;     // rows in flight in a warp's registers
+constexpr int kChainIn = 2 * kChainRf;     // input ring: a row is fetched 5 rows before its use
+constexpr int kChainLag = kChainLv + kChainRf;  // rows by which a warp's first level is behind the warp before it
+// rows of the material ring: from the row being fetched to the last level of
+// the last warp, and one for the warps' skew within an iteration
+__host__ __device__ constexpr int chain_mat(int nc) {
+  return (kChainIn + kChainLag * (nc - 1) + kChainLv + kChainRf) / kChainRf * kChainRf;
+}
 
 struct ChainArgs {
   int nx, ny;
@@ -54,13 +61,14 @@ struct ChainArgs {
   int n_stripes, n_gen_lo, n_gen_hi, n_segs, seg_first, seg_rows, n_segs_g, seg_rows_g;
 };
 
-// floats of a block's shared memory: field ring [5 rows][fields][128], one
-// hand-over ring of the same size per link of the chain, material ring
-// [20 rows][1 or 2][128], column coefficients [5][128]
+// floats of a block's shared memory: input ring [6 rows][fields][128], a
+// hand-over ring [3 rows][fields][128] per link, the material ring
+// [rows][1 or 2][128], column coefficients [5][128]
 __host__ __device__ constexpr int chain_fields(bool lossy, bool pml) { return 3 + (lossy ? 1 : 0) + (pml ? 2 : 0); }
 __host__ __device__ constexpr size_t chain_smem_bytes(int nc, bool lossy, bool pml) {
   return sizeof(float) * kChainCols *
-         ((size_t)nc * 5 * chain_fields(lossy, pml) + kChainMat * (lossy ? 2 : 1) + (pml ? 5 : 0));
+         ((size_t)(kChainIn + (nc - 1) * kChainRf) * chain_fields(lossy, pml) + chain_mat(nc) * (lossy ? 2 : 1) +
+          (pml ? 5 : 0));
 }
 
 // block -> stripe and rows; false: no work
@@ -89,10 +97,10 @@ __host__ __device__ inline bool chain_work(const ChainArgs& a, int b, int& strip
 // many segments, and the other stripes' first and last segments are shortened
 // by the time of their general rows.  Returns the number of blocks.
 inline long chain_layout(ChainArgs& a, int K, long resident, int P, float gen_cost) {
-  const int outw = kChainCols - 2 * K;
+  const int hb = (K + 3) / 4 * 4, outw = kChainCols - 2 * hb;
   a.n_stripes = (a.ny + outw - 1) / outw;
   auto general = [&](int s) {
-    const int lo = s * outw - K, hi = lo + kChainCols - 1;
+    const int lo = s * outw - hb, hi = lo + kChainCols - 1;
     return lo < std::max(P, 1) || hi > a.ny - 2 - P;
   };
   int glo = 0, ghi = 0;
@@ -119,16 +127,15 @@ inline long chain_layout(ChainArgs& a, int K, long resident, int P, float gen_co
   return (long)n_int * ns + (long)n_gen * a.n_segs_g;
 }
 
-// one pass of 4*nc steps (fd2d_chain.cu); FDTD_ERR_UNSUPPORTED where the march
-// is the faster form
+// one pass of kChainLv*nc steps (fd2d_chain.cu)
 int launch_chain(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int nc, int* status,
                  float gen_cost, cudaStream_t st);
 
 namespace {
 
-__device__ __forceinline__ void chain_cp16(float* dst, const float* src, bool ok) {
+__device__ __forceinline__ void chain_cp16(float* dst, const float* base, unsigned off, bool ok) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(ok ? 16u : 0u) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(base + off), "r"(ok ? 16u : 0u) : "memory");
 }
 __device__ __forceinline__ F4 chain_lds(const float* p) { return f4(*reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ void chain_sts(float* p, const F4& v) { *reinterpret_cast<float4*>(p) = to4(v); }
@@ -143,10 +150,9 @@ struct ChainRow {
 template <int NC, bool LOSSY, bool PML>
 __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ ChainArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
-  constexpr int W = kChainCols, K = 4 * NC, HB = K;  // halo columns on each side (whole lanes)
-  constexpr int NF = chain_fields(LOSSY, PML), NM = LOSSY ? 2 : 1;
+  constexpr int W = kChainCols, LV = kChainLv, RF = kChainRf, K = LV * NC, HB = (K + 3) / 4 * 4;  // halo columns: whole lanes
+  constexpr int NF = chain_fields(LOSSY, PML), NM = LOSSY ? 2 : 1, MT = chain_mat(NC);
   constexpr int F_IZ = 3, F_IHX = 3 + (LOSSY ? 1 : 0), F_IHY = F_IHX + 1;
-  constexpr int MT = kChainMat;
   extern __shared__ float4 chain_sm[];
   int stripe, i_s, i_e;
   if (!chain_work(a, blockIdx.x, stripe, i_s, i_e)) return;  // the whole block
@@ -157,10 +163,11 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
   const bool vin = j0 >= 0 && j0 + 4 <= ny;  // ny % 4 == 0: a lane's vector is wholly in or out
   const bool vout = vin && lane * 4 >= HB && lane * 4 < W - HB;
   float* const sm = reinterpret_cast<float*>(chain_sm) + lane * 4;
-  float* const fin_ring = sm + cw * 5 * NF * W;                // rows into this warp
-  float* const fout_ring = sm + (cw + 1) * 5 * NF * W;         // rows out of it (not the last warp's)
-  float* const mring = sm + NC * 5 * NF * W;                   // [20][NM][W], row r in slot r mod 20
-  float* const cc = mring + MT * NM * W;                       // [5][W] gy2/2, gy3, fy1, fy2, fy3
+  float* const links = sm + kChainIn * NF * W;                      // [NC-1][RF][NF][W]
+  float* const mring = links + (NC - 1) * RF * NF * W;              // [MT][NM][W], row r in slot r mod MT
+  float* const cc = mring + MT * NM * W;                            // [5][W] gy2/2, gy3, fy1, fy2, fy3
+  const float* const from = cw == 0 ? sm : links + (cw - 1) * RF * NF * W;  // rows into this warp
+  float* const to = links + cw * RF * NF * W;                               // rows out of it (not the last warp's)
 
   // ---- columns
   bool col_ok = j0 >= 1 && j0 + 3 <= ny - 2;
@@ -196,59 +203,59 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
     return __ballot_sync(kAll, g);
   };
 
-  // ---- rows on their way in (first warp): fields into ring slot `slot`,
-  // materials into theirs; zeros outside the grid
+  // ---- rows on their way in (first warp): fields into input ring slot `slot`,
+  // materials into theirs; zeros outside the grid.  32-bit offsets (the launch
+  // checks the grid's size): half the address arithmetic
   auto fetch = [&](int row, int slot, int mslot) {
     const bool ok = vin && row >= 0 && row < nx;
-    const size_t off = ok ? (size_t)row * ny + j0 : 0;
-    float* const f = fin_ring + slot * NF * W;
-    chain_cp16(f + 0 * W, a.in.dz + off, ok);
-    chain_cp16(f + 1 * W, a.in.hx + off, ok);
-    chain_cp16(f + 2 * W, a.in.hy + off, ok);
-    if (LOSSY) chain_cp16(f + F_IZ * W, a.in.iz + off, ok);
+    const unsigned off = ok ? (unsigned)row * (unsigned)ny + (unsigned)j0 : 0u;
+    float* const f = sm + slot * NF * W;
+    chain_cp16(f + 0 * W, a.in.dz, off, ok);
+    chain_cp16(f + 1 * W, a.in.hx, off, ok);
+    chain_cp16(f + 2 * W, a.in.hy, off, ok);
+    if (LOSSY) chain_cp16(f + F_IZ * W, a.in.iz, off, ok);
     if (PML) {
-      chain_cp16(f + F_IHX * W, a.in.ihx + off, ok);
-      chain_cp16(f + F_IHY * W, a.in.ihy + off, ok);
+      chain_cp16(f + F_IHX * W, a.in.ihx, off, ok);
+      chain_cp16(f + F_IHY * W, a.in.ihy, off, ok);
     }
     float* const m = mring + mslot * NM * W;
-    chain_cp16(m, a.naz + off, ok);
-    if (LOSSY) chain_cp16(m + W, a.nbz + off, ok);
+    chain_cp16(m, a.naz, off, ok);
+    if (LOSSY) chain_cp16(m + W, a.nbz, off, ok);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
 
   const F4 zero = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-  ChainRow R[5];
+  ChainRow R[RF];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) R[k].dz = R[k].iz = R[k].hx = R[k].hy = R[k].ihx = R[k].ihy = R[k].ez = zero;
+  for (int k = 0; k < RF; ++k) R[k].dz = R[k].iz = R[k].hx = R[k].hy = R[k].ihx = R[k].ihy = R[k].ez = zero;
   // rows before the first that is read: no output depends on them
-  if (cw == 0) {
-    for (int k = 0; k < MT * NM; ++k) chain_sts(mring + k * W, zero);
-    for (int k = 5 * NF; k < NC * 5 * NF; ++k) chain_sts(sm + k * W, zero);
-  }
+  for (int k = cw; k < (NC - 1) * RF * NF + MT * NM; k += NC) chain_sts(links + k * W, zero);
   __syncthreads();
   const int first = i_s - K;
-  const int b0 = (first >= 0 ? first / 5 : -((4 - first) / 5)) * 5;  // first row, of a block of five
-  int rb = b0 - kChainLag * cw;                                       // this warp's level-0 row
-  int ms = ((rb - 3) % MT + MT) % MT + 3;                             // material slot of row rb, in 3 .. 22
+  const int b0 = (first >= 0 ? first / RF : -((RF - 1 - first) / RF)) * RF;  // first row, of a block of RF
+  int rb = b0 - kChainLag * cw;                                              // this warp's first level's row
+  int ms = ((rb - (LV - 1)) % MT + MT) % MT + LV - 1;                        // material slot of row rb, in LV-1 .. MT+LV-2
+  int par = 0;                                                               // half of the input ring that holds the block's rows
   if (cw == 0) {
 #pragma unroll
-    for (int k = 0; k < kChainAhead; ++k) fetch(rb + k, k, (ms + k) % MT);
+    for (int k = 0; k < kChainIn - 1; ++k) fetch(rb + k, k, (ms + k) % MT);
   }
   bool fin = true;
 
-  // ---- iteration I of the block of five that starts at row rb: this warp's
+  // ---- iteration I of the block of RF rows that starts at row rb: this warp's
   // level 0 takes row rb+I
   auto iterate = [&](auto itag, auto inttag) {
     constexpr int I = decltype(itag)::value;
     constexpr bool INT = decltype(inttag)::value;
     const int r = rb + I;
-    if (cw == 0) {  // row r+3 starts its way in; row r's copies complete
-      const int mf = ms + I + kChainAhead;
-      fetch(r + kChainAhead, (I + kChainAhead) % 5, mf >= MT ? mf - MT : mf);
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(kChainAhead) : "memory");
+    const float* f = from + I * NF * W;
+    if (cw == 0) {  // row r+5 starts its way in, into row r-1's slot; row r's copies complete
+      const int mf = ms + I + kChainIn - 1;
+      fetch(r + kChainIn - 1, I > 0 ? par + I - 1 : RF - par + RF - 1, mf >= MT ? mf - MT : mf);
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kChainIn - 1) : "memory");
+      f += par * NF * W;
     }
     {
-      const float* const f = fin_ring + I * NF * W;
       ChainRow& q = R[I];
       q.dz = chain_lds(f + 0 * W);
       q.hx = chain_lds(f + 1 * W);
@@ -259,14 +266,14 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
         q.ihy = chain_lds(f + F_IHY * W);
       }
     }
-    // every warp has taken slot I: the warp before may refill it below
+    // every warp has taken its row: the warp before may refill the slot below
     if (NC > 1) __syncthreads();
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int qi = (I - s + 5) % 5, pi = (I - s + 4) % 5;
+    for (int s = 0; s < LV; ++s) {
+      const int qi = (I - s + RF) % RF, pi = (I - s - 1 + RF) % RF;
       ChainRow &q = R[qi], &p = R[pi];
       const int row = r - s;
-      const int t = a.t0 + 4 * cw + s;  // table row of this level's time step
+      const int t = a.t0 + LV * cw + s;  // table row of this level's time step
       // D and E on row r-s
       const float hl = __shfl_up_sync(kAll, q.hx.b.y, 1);
       const F4 d = sub4(sub4(q.hy, p.hy), q.hx);
@@ -354,10 +361,10 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
         }
       }
     }
-    // ---- row r-4 is complete: to the next warp's ring, or out
-    ChainRow& c = R[(I + 1) % 5];
+    // ---- row r-LV is complete: to the next warp's ring, or out
+    ChainRow& c = R[(I + 1) % RF];
     if (NC > 1 && cw < NC - 1) {
-      float* const f = fout_ring + I * NF * W;
+      float* const f = to + I * NF * W;
       chain_sts(f + 0 * W, c.dz);
       chain_sts(f + 1 * W, c.hx);
       chain_sts(f + 2 * W, c.hy);
@@ -367,9 +374,9 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
         chain_sts(f + F_IHY * W, c.ihy);
       }
     } else {
-      const int row = r - 4;
+      const int row = r - LV;
       if (vout && row >= i_s && row < i_e) {
-        const size_t off = (size_t)row * ny + j0;
+        const unsigned off = (unsigned)row * (unsigned)ny + (unsigned)j0;
         auto st = [&](float* p, const F4& v) { __stcs(reinterpret_cast<float4*>(p + off), to4(v)); };
         st(a.out.dz, c.dz);
         st(a.out.hx, c.hx);
@@ -388,31 +395,32 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
       }
     }
   };
-  auto five = [&](auto inttag) {
+  static_assert(RF == 3, "block() names the iterations of a block");
+  auto block = [&](auto inttag) {
     iterate(std::integral_constant<int, 0>{}, inttag);
     iterate(std::integral_constant<int, 1>{}, inttag);
     iterate(std::integral_constant<int, 2>{}, inttag);
-    iterate(std::integral_constant<int, 3>{}, inttag);
-    iterate(std::integral_constant<int, 4>{}, inttag);
   };
 
-  // ---- down the segment: the last warp's level 4 has to complete row i_e-1
-  const int n_blk = (i_e - 1 + kChainLag * (NC - 1) - b0 + 4) / 5 + 1;
-  int gb = rb - 4;  // rows gb .. gb+63 are in gm
+  // ---- down the segment: the last warp's last level has to complete row i_e-1
+  const int n_blk = (i_e - 1 + LV - (RF - 1) + kChainLag * (NC - 1) - b0 + RF - 1) / RF + 1;
+  int gb = rb - LV;  // rows gb .. gb+63 are in gm
   unsigned long long gm = cint ? rows_ok(gb) | (unsigned long long)rows_ok(gb + 32) << 32 : 0ull;
+  constexpr unsigned long long kTouch = (1ull << (LV + RF)) - 1;  // rows rb-LV .. rb+RF-1 that a block touches
   for (int k = 0; k < n_blk; ++k) {
-    bool interior = false;  // the nine rows rb-4 .. rb+4 that the five iterations touch
+    bool interior = false;
     if (cint) {
-      if (rb + 4 - gb >= 64) {
+      if (rb + RF - 1 - gb >= 64) {
         gb += 32;
         gm = gm >> 32 | (unsigned long long)rows_ok(gb + 32) << 32;
       }
-      interior = ((gm >> (rb - 4 - gb)) & 0x1ffull) == 0x1ffull;
+      interior = ((gm >> (rb - LV - gb)) & kTouch) == kTouch;
     }
-    if (interior) five(std::true_type{});
-    else five(std::false_type{});
-    rb += 5;
-    ms = ms + 5 >= MT + 3 ? ms + 5 - MT : ms + 5;
+    if (interior) block(std::true_type{});
+    else block(std::false_type{});
+    rb += RF;
+    ms = ms + RF >= MT + LV - 1 ? ms + RF - MT : ms + RF;
+    par = RF - par;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (a.status && __any_sync(kAll, !fin) && lane == 0) raise_status(a.status, ST_NONFINITE);

@@ -51,7 +51,8 @@ float march_gen_cost() { return g_cfg.gen_cost; }
 
 bool chain_better(int nx, int ny) {
   if (g_cfg.cpl || g_cfg.seg_rows) return false;
-  return (long long)nx * ny >= (1LL << 20) && nx >= 64 && ny >= 128;
+  // (32-bit element offsets)
+  return (long long)nx * ny >= (1LL << 20) && (long long)nx * ny < (1LL << 31) && nx >= 64 && ny >= 128;
 }
 
 namespace {
