@@ -106,10 +106,23 @@ bool tile_ok(const fdtd2d_params* p, int steps_per_pass, TilePlan& pl) {
 }
 size_t tile_workspace_bytes(const fdtd2d_params* p) { return slot_bytes(p) * nslots(p) + kTileFlagBytes; }
 
-FieldSet workspace_set(const fdtd2d_params* p, void* workspace) {
+// Chained passes over padded copies, for grids whose rows are no multiple of 16
+// bytes (they would otherwise go three launches a step): two ping-pong sets,
+// the materials and ez, all with rows of pad_pitch floats.
+int pad_pitch(const fdtd2d_params* p) { return (p->ny + 3) / 4 * 4; }
+size_t pad_slot_bytes(const fdtd2d_params* p) {
+  return ((size_t)p->nx * pad_pitch(p) * sizeof(float) + 255) & ~(size_t)255;
+}
+size_t pad_workspace_bytes(const fdtd2d_params* p) {
+  return pad_slot_bytes(p) * (2 * nslots(p) + (p->nbz ? 2 : 1) + 1);
+}
+bool pad_ok(const fdtd2d_params* p, int steps_per_pass) {
+  return p->ny % 4 != 0 && !ext_on(p) && steps_per_pass == 0 && chain_better(p->nx, p->ny) && p->nx <= 8 * 65535;
+}
+
+FieldSet workspace_set(const fdtd2d_params* p, void* workspace, size_t sb) {
   FieldSet ws{};
   char* base = (char*)workspace;
-  const size_t sb = slot_bytes(p);
   int k = 0;
   ws.dz = (float*)(base + sb * k++);
   ws.hx = (float*)(base + sb * k++);
@@ -120,6 +133,37 @@ FieldSet workspace_set(const fdtd2d_params* p, void* workspace) {
     ws.ihy = (float*)(base + sb * k++);
   }
   return ws;
+}
+
+int step_three_launches(int t, const fdtd2d_params& p, const fdtd2d_state& s, cudaStream_t st);
+
+// nsteps >= 8 steps of a ragged grid: the remainder modulo 4 by single steps,
+// the rest in chained passes over padded copies
+int step_padded(const fdtd2d_params* p, const fdtd2d_state* s, int t0, int nsteps, void* workspace, cudaStream_t st) {
+  const size_t sb = pad_slot_bytes(p);
+  const int pitch = pad_pitch(p), nf = nslots(p);
+  const FieldSet set[2] = {workspace_set(p, workspace, sb), workspace_set(p, (char*)workspace + sb * nf, sb)};
+  char* rest = (char*)workspace + sb * 2 * nf;
+  float* naz = (float*)rest;
+  float* nbz = p->nbz ? (float*)(rest + sb) : nullptr;
+  float* ez = (float*)(rest + sb * (p->nbz ? 2 : 1));
+  int rc;
+  int t = t0;
+  for (; (t0 + nsteps - t) % 4 != 0; ++t)
+    if ((rc = step_three_launches(t + 1, *p, *s, st))) return rc;
+  const FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
+  if ((rc = launch_pad(user, set[0], p->naz, naz, p->nbz, nbz, p->nx, p->ny, pitch, st))) return rc;
+  int cur = 0;
+  while (t < t0 + nsteps) {
+    const int rem = t0 + nsteps - t, k = rem >= 8 ? 8 : 4;
+    const bool last = k == rem;
+    rc = launch_chain(*p, pitch, naz, nbz, set[cur], set[1 - cur], last ? ez : nullptr, t, k, last ? s->status : nullptr,
+                      march_gen_cost(), st);
+    if (rc) return rc;
+    cur = 1 - cur;
+    t += k;
+  }
+  return launch_unpad(set[cur], user, ez, s->ez, p->nx, p->ny, pitch, st);
 }
 
 // one time step in the reference's order (fd2d/python/fd2d_3_4.py:268-277):
@@ -208,7 +252,8 @@ size_t fdtd2d_fast_workspace_size(const fdtd2d_params* p, int steps_per_pass) {
   const size_t need = fdtd2d_workspace_size(p, steps_per_pass);
   if (!p || p->nx < 3 || p->ny < 3) return 0;
   TilePlan pl;
-  return tile_ok(p, steps_per_pass, pl) ? std::max(need, tile_workspace_bytes(p)) : need;
+  if (tile_ok(p, steps_per_pass, pl)) return std::max(need, tile_workspace_bytes(p));
+  return pad_ok(p, steps_per_pass) ? pad_workspace_bytes(p) : need;
 }
 
 int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, int steps_per_pass, void* workspace,
@@ -226,9 +271,13 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
       tile_ok(p, steps_per_pass, tile)) {
     const FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
     unsigned* flags = (unsigned*)((char*)workspace + slot_bytes(p) * nslots(p));
-    return launch_tile(*p, user, user, workspace_set(p, workspace), user, s->ez, t0, nsteps, s->status, s->probe_ez,
+    return launch_tile(*p, user, user, workspace_set(p, workspace, slot_bytes(p)), user, s->ez, t0, nsteps, s->status, s->probe_ez,
                        flags, tile, st);
   }
+
+  if (nsteps >= 8 && !s->probe_ez && pad_ok(p, steps_per_pass) && workspace && ((uintptr_t)workspace & 255u) == 0 &&
+      workspace_bytes >= pad_workspace_bytes(p))
+    return step_padded(p, s, t0, nsteps, workspace, st);
 
   if (!fused_ok(p, s) || nsteps == 1) {
     for (int t = t0 + 1; t <= t0 + nsteps; ++t)
@@ -270,7 +319,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
   }
 
   FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
-  const FieldSet ws = workspace_set(p, workspace);
+  const FieldSet ws = workspace_set(p, workspace, slot_bytes(p));
   MarchExt ext{};
   float* inc_e = nullptr;
   float* inc_h = nullptr;
@@ -303,7 +352,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
     // ez is a result of the call, not an input of the passes: only the last stores it
     float* ez = (i + 1 == sched.size()) ? s->ez : nullptr;
     if (chain && (sched[i] == 8 || sched[i] == 4)) {
-      rc = launch_chain(*p, in, out, ez, t, sched[i] / kChainLv, status, march_gen_cost(), st);
+      rc = launch_chain(*p, p->ny, p->naz, p->nbz, in, out, ez, t, sched[i], status, march_gen_cost(), st);
     } else if (!ext_on(p)) {
       rc = launch_march(*p, in, out, ez, t, sched[i], status, s->probe_ez, st);
     } else {

@@ -5,23 +5,30 @@
 // materials; ez only in a call's last pass) whatever its number of steps K,
 // so large grids are bound by 56/K bytes per cell-update: the K = 4 march ran
 // at 85% of the copy bandwidth and could only gain by more steps per pass,
-// whose state does not fit one warp's registers.  K = 8 is four warps in a
-// chain, two steps each: a warp hands its rows through a ring in shared memory
-// to the next, the last stores them.
+// whose state does not fit one warp's registers.  K = 8 is a chain of warps,
+// each of which does LV steps and hands its rows through a ring in shared
+// memory to the next; the last stores them.
 //
 // A block is one chain: it owns a stripe of 128 columns (4 per lane, K on each
 // side recomputed by the neighbours) and marches down a segment of rows.  At
-// iteration r level s of a warp (s = 0, 1) does D and E of row r-s and H of
-// row r-s-1.  A row's values stay in the same registers through both levels:
-// three rows are in flight, row r in register set r mod 3, and the loop is
-// unrolled by three rows, so no value ever moves (the march's register shifts
-// were a third of its instructions).  Two steps a warp rather than four: four
-// need five rows and a body of 20 levels, 21 KB of code, whose fetch stalled
-// each issue by 1.5 cycles.  Updates are packed two cells to an instruction.
-// Input rows arrive by cp.async five rows ahead.  One block barrier per row
-// keeps the chain in step.
+// iteration r level s of a warp (s = 0 .. LV-1) does D and E of row r-s and H
+// of row r-s-1.  A row's values stay in the same registers through all levels:
+// RF = LV+1 rows are in flight, row r in register set r mod RF, and the loop is
+// unrolled by RF rows, so no value ever moves (the march's register shifts were
+// a third of its instructions).  Updates are packed two cells to an
+// instruction.  Input rows arrive by cp.async RF-1 rows ahead.  One block
+// barrier per row keeps the chain in step.
 //
-// Blocks of three rows run in one of two forms, as in the march: interior (unit
+// Two shapes, measured in Gcell-updates/s (lossy with absorbing layer /
+// lossless with / lossy without; the march: 373 at 8192^2):
+//   2 warps x 4 steps: 717 / 866 / 1212 at 8192^2, 521 / 651 / 1015 at 4096^2,
+//     291 / 349 at 2048^2: fewer rows pass through shared memory, but a body of
+//     20 levels (fetching its code costs 0.6 cycles an issue) and 2 warps per
+//     scheduler;
+//   4 warps x 2 steps: 643 / 742 / 995, 594 / 689 / 907, 417 / 479.
+// The choice is in fd2d_chain.cu.
+//
+// Blocks of RF rows run in one of two forms, as in the march: interior (unit
 // coefficients, nothing that the reference's loops leave out, no source) or
 // general, decided on the coefficient vectors themselves.  Same per-cell
 // formulas and order as the per-function kernels: bitwise equal results.
@@ -35,18 +42,18 @@
 namespace fdtd {
 
 constexpr int kChainCols = 128;
-constexpr int kChainLv = 2;                // time steps (levels) per warp
-constexpr int kChainRf = kChainLv + 1;     // rows in flight in a warp's registers
-constexpr int kChainIn = 2 * kChainRf;     // input ring: a row is fetched 5 rows before its use
-constexpr int kChainLag = kChainLv + kChainRf;  // rows by which a warp's first level is behind the warp before it
-// rows of the material ring: from the row being fetched to the last level of
-// the last warp, and one for the warps' skew within an iteration
-__host__ __device__ constexpr int chain_mat(int nc) {
-  return (kChainIn + kChainLag * (nc - 1) + kChainLv + kChainRf) / kChainRf * kChainRf;
-}
+// LV: time steps (levels) per warp; NC: warps in the chain
+__host__ __device__ constexpr int chain_rf(int lv) { return lv + 1; }              // rows in flight in a warp's registers
+__host__ __device__ constexpr int chain_lag(int lv) { return lv + chain_rf(lv); }  // rows a warp is behind the one before
+// rows of the material ring: from the row being fetched (RF-1 ahead) to the last
+// level of the last warp, and one for the warps' skew within an iteration
+__host__ __device__ constexpr int chain_mat(int lv, int nc) { return chain_rf(lv) + chain_lag(lv) * (nc - 1) + lv + 1; }
+// halo columns on each side of a stripe: whole lanes
+__host__ __device__ constexpr int chain_halo(int lv, int nc) { return (lv * nc + 3) / 4 * 4; }
 
 struct ChainArgs {
   int nx, ny;
+  int pitch;  // columns from one row of every array to the next, a multiple of 4, >= ny
   FieldSet in, out;
   float* ez;  // null: not stored by this pass
   const float* naz;
@@ -56,48 +63,47 @@ struct ChainArgs {
   const float* src_table;
   int t0;
   int* status;  // null: no Inf/NaN test
-  // blocks 0 .. n_int*n_segs-1: the stripes away from the edges; then the
-  // general stripes at either edge with their shorter segments
+  // blocks 0 .. n_gen*n_segs_g-1: the general stripes at either edge, in shorter
+  // segments; then the other stripes
   int n_stripes, n_gen_lo, n_gen_hi, n_segs, seg_first, seg_rows, n_segs_g, seg_rows_g;
 };
 
-// floats of a block's shared memory: input ring [6 rows][fields][128], a
-// hand-over ring [3 rows][fields][128] per link, the material ring
-// [rows][1 or 2][128], column coefficients [5][128]
+// floats of a block's shared memory: an input ring and a hand-over ring per
+// link [RF rows][fields][128], the material ring [rows][1 or 2][128], column
+// coefficients [5][128]
 __host__ __device__ constexpr int chain_fields(bool lossy, bool pml) { return 3 + (lossy ? 1 : 0) + (pml ? 2 : 0); }
-__host__ __device__ constexpr size_t chain_smem_bytes(int nc, bool lossy, bool pml) {
+__host__ __device__ constexpr size_t chain_smem_bytes(int lv, int nc, bool lossy, bool pml) {
   return sizeof(float) * kChainCols *
-         ((size_t)(kChainIn + (nc - 1) * kChainRf) * chain_fields(lossy, pml) + chain_mat(nc) * (lossy ? 2 : 1) +
-          (pml ? 5 : 0));
+         ((size_t)nc * chain_rf(lv) * chain_fields(lossy, pml) + chain_mat(lv, nc) * (lossy ? 2 : 1) + (pml ? 5 : 0));
 }
 
 // block -> stripe and rows; false: no work
 __host__ __device__ inline bool chain_work(const ChainArgs& a, int b, int& stripe, int& i_s, int& i_e) {
-  const int n_int = a.n_stripes - a.n_gen_lo - a.n_gen_hi, n_main = n_int * a.n_segs;
-  if (b < n_main) {
-    stripe = a.n_gen_lo + b % n_int;
-    const int seg = b / n_int;
-    i_s = seg == 0 ? 0 : a.seg_first + (seg - 1) * a.seg_rows;
-    i_e = seg == a.n_segs - 1 ? a.nx : seg == 0 ? a.seg_first : i_s + a.seg_rows;
-  } else {
-    const int n_gen = a.n_gen_lo + a.n_gen_hi;
-    if (n_gen == 0) return false;
-    const int k = b - n_main, g = k % n_gen, seg = k / n_gen;
-    if (seg >= a.n_segs_g) return false;
+  const int n_gen = a.n_gen_lo + a.n_gen_hi, n_int = a.n_stripes - n_gen, n_first = n_gen * a.n_segs_g;
+  if (b < n_first) {
+    const int g = b % n_gen, seg = b / n_gen;
     stripe = g < a.n_gen_lo ? g : a.n_stripes - n_gen + g;
     i_s = seg * a.seg_rows_g;
     i_e = i_s + a.seg_rows_g;
+  } else {
+    const int k = b - n_first;
+    if (n_int == 0 || k >= n_int * a.n_segs) return false;
+    stripe = a.n_gen_lo + k % n_int;
+    // the first and last segments of a stripe, which hold general rows, before the others
+    const int q = k / n_int, seg = q == 0 ? 0 : q == 1 ? a.n_segs - 1 : q - 1;
+    i_s = seg == 0 ? 0 : a.seg_first + (seg - 1) * a.seg_rows;
+    i_e = seg == a.n_segs - 1 ? a.nx : seg == 0 ? a.seg_first : i_s + a.seg_rows;
   }
   i_e = i_e < a.nx ? i_e : a.nx;
   return i_s < i_e;
 }
 
-// One wave of blocks over the grid: the stripes that the absorbing layer (P
+// About `blocks` blocks over the grid: the stripes that the absorbing layer (P
 // cells, 0: unknown) or the grid's edge makes general get gen_cost times as
 // many segments, and the other stripes' first and last segments are shortened
 // by the time of their general rows.  Returns the number of blocks.
-inline long chain_layout(ChainArgs& a, int K, long resident, int P, float gen_cost) {
-  const int hb = (K + 3) / 4 * 4, outw = kChainCols - 2 * hb;
+inline long chain_layout(ChainArgs& a, int K, long blocks, int P, float gen_cost) {
+  const int hb = chain_halo(K, 1), outw = kChainCols - 2 * hb;
   a.n_stripes = (a.ny + outw - 1) / outw;
   auto general = [&](int s) {
     const int lo = s * outw - hb, hi = lo + kChainCols - 1;
@@ -108,7 +114,7 @@ inline long chain_layout(ChainArgs& a, int K, long resident, int P, float gen_co
   while (ghi < a.n_stripes - glo && general(a.n_stripes - 1 - ghi)) ++ghi;
   const int n_int = a.n_stripes - glo - ghi, n_gen = glo + ghi, mn = 4 * K;
   const double G = gen_cost >= 1.f ? gen_cost : 1.0;
-  const long n_segs = std::max(1L, (long)((double)resident / (n_int + G * n_gen)));
+  const long n_segs = std::max(1L, (long)((double)blocks / (n_int + G * n_gen)));
   const long n_segs_g = std::max(1L, (long)(G * n_segs));
   a.seg_rows_g = std::max((int)((a.nx + n_segs_g - 1) / n_segs_g), mn);
   a.n_segs_g = (a.nx + a.seg_rows_g - 1) / a.seg_rows_g;
@@ -127,9 +133,9 @@ inline long chain_layout(ChainArgs& a, int K, long resident, int P, float gen_co
   return (long)n_int * ns + (long)n_gen * a.n_segs_g;
 }
 
-// one pass of kChainLv*nc steps (fd2d_chain.cu)
-int launch_chain(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int nc, int* status,
-                 float gen_cost, cudaStream_t st);
+// one pass of k steps, 4 or 8, over arrays of `pitch` columns a row (fd2d_chain.cu)
+int launch_chain(const fdtd2d_params& p, int pitch, const float* naz, const float* nbz, const FieldSet& in,
+                 const FieldSet& out, float* ez, int t0, int k, int* status, float gen_cost, cudaStream_t st);
 
 namespace {
 
@@ -147,23 +153,23 @@ struct ChainRow {
   F4 dz, iz, hx, hy, ihx, ihy, ez;
 };
 
-template <int NC, bool LOSSY, bool PML>
+template <int LV, int NC, bool LOSSY, bool PML>
 __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ ChainArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
-  constexpr int W = kChainCols, LV = kChainLv, RF = kChainRf, K = LV * NC, HB = (K + 3) / 4 * 4;  // halo columns: whole lanes
-  constexpr int NF = chain_fields(LOSSY, PML), NM = LOSSY ? 2 : 1, MT = chain_mat(NC);
+  constexpr int W = kChainCols, RF = chain_rf(LV), K = LV * NC, HB = chain_halo(LV, NC);
+  constexpr int NF = chain_fields(LOSSY, PML), NM = LOSSY ? 2 : 1, MT = chain_mat(LV, NC);
   constexpr int F_IZ = 3, F_IHX = 3 + (LOSSY ? 1 : 0), F_IHY = F_IHX + 1;
   extern __shared__ float4 chain_sm[];
   int stripe, i_s, i_e;
   if (!chain_work(a, blockIdx.x, stripe, i_s, i_e)) return;  // the whole block
 
   const int lane = threadIdx.x & 31, cw = threadIdx.x >> 5;
-  const int nx = a.nx, ny = a.ny;
+  const int nx = a.nx, ny = a.ny, pitch = a.pitch;
   const int j0 = stripe * (W - 2 * HB) - HB + lane * 4;
-  const bool vin = j0 >= 0 && j0 + 4 <= ny;  // ny % 4 == 0: a lane's vector is wholly in or out
+  const bool vin = j0 >= 0 && j0 + 4 <= pitch;  // pitch % 4 == 0: a lane's vector is wholly in or out of the arrays
   const bool vout = vin && lane * 4 >= HB && lane * 4 < W - HB;
   float* const sm = reinterpret_cast<float*>(chain_sm) + lane * 4;
-  float* const links = sm + kChainIn * NF * W;                      // [NC-1][RF][NF][W]
+  float* const links = sm + RF * NF * W;                      // [NC-1][RF][NF][W]
   float* const mring = links + (NC - 1) * RF * NF * W;              // [MT][NM][W], row r in slot r mod MT
   float* const cc = mring + MT * NM * W;                            // [5][W] gy2/2, gy3, fy1, fy2, fy3
   const float* const from = cw == 0 ? sm : links + (cw - 1) * RF * NF * W;  // rows into this warp
@@ -190,7 +196,8 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
   }
   const bool cint = __all_sync(kAll, col_ok);
   const bool src_here = a.src_kind != FDTD_SRC_NONE && a.src_j >= j0 - lane * 4 && a.src_j < j0 - lane * 4 + W;
-  const bool col0 = j0 == 0, last_col = j0 + 4 == ny;
+  const bool col0 = j0 == 0;
+  const int h_cols = ny - 1 - j0;  // of this lane's columns that H updates
 
   // bit l: row b+l may be touched by an interior iteration
   auto rows_ok = [&](int b) -> unsigned {
@@ -208,7 +215,7 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
   // checks the grid's size): half the address arithmetic
   auto fetch = [&](int row, int slot, int mslot) {
     const bool ok = vin && row >= 0 && row < nx;
-    const unsigned off = ok ? (unsigned)row * (unsigned)ny + (unsigned)j0 : 0u;
+    const unsigned off = ok ? (unsigned)row * (unsigned)pitch + (unsigned)j0 : 0u;
     float* const f = sm + slot * NF * W;
     chain_cp16(f + 0 * W, a.in.dz, off, ok);
     chain_cp16(f + 1 * W, a.in.hx, off, ok);
@@ -233,12 +240,11 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
   __syncthreads();
   const int first = i_s - K;
   const int b0 = (first >= 0 ? first / RF : -((RF - 1 - first) / RF)) * RF;  // first row, of a block of RF
-  int rb = b0 - kChainLag * cw;                                              // this warp's first level's row
-  int ms = ((rb - (LV - 1)) % MT + MT) % MT + LV - 1;                        // material slot of row rb, in LV-1 .. MT+LV-2
-  int par = 0;                                                               // half of the input ring that holds the block's rows
+  int rb = b0 - chain_lag(LV) * cw;                     // this warp's first level's row
+  int ms = ((rb - (LV - 1)) % MT + MT) % MT + LV - 1;  // material slot of row rb, in LV-1 .. MT+LV-2
   if (cw == 0) {
 #pragma unroll
-    for (int k = 0; k < kChainIn - 1; ++k) fetch(rb + k, k, (ms + k) % MT);
+    for (int k = 0; k < RF - 1; ++k) fetch(rb + k, k, (ms + k) % MT);
   }
   bool fin = true;
 
@@ -249,11 +255,10 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
     constexpr bool INT = decltype(inttag)::value;
     const int r = rb + I;
     const float* f = from + I * NF * W;
-    if (cw == 0) {  // row r+5 starts its way in, into row r-1's slot; row r's copies complete
-      const int mf = ms + I + kChainIn - 1;
-      fetch(r + kChainIn - 1, I > 0 ? par + I - 1 : RF - par + RF - 1, mf >= MT ? mf - MT : mf);
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(kChainIn - 1) : "memory");
-      f += par * NF * W;
+    if (cw == 0) {  // row r+RF-1 starts its way in, into row r-1's slot; row r's copies complete
+      const int mf = ms + I + RF - 1;
+      fetch(r + RF - 1, (I + RF - 1) % RF, mf >= MT ? mf - MT : mf);
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(RF - 1) : "memory");
     }
     {
       ChainRow& q = R[I];
@@ -346,12 +351,13 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
           nhx = fma4(0.5f, cx, p.hx);
           nhy = fma4(-0.5f, cy, p.hy);
         }
-        // row nx-1 and column ny-1 (the last of its lane) are not updated
+        // row nx-1 and column ny-1 are not updated
+        const int n = in ? h_cols : 0;
         auto take = [&](F4& x, const F4& nw) {
-          x.a.x = in ? nw.a.x : x.a.x;
-          x.a.y = in ? nw.a.y : x.a.y;
-          x.b.x = in ? nw.b.x : x.b.x;
-          x.b.y = in && !last_col ? nw.b.y : x.b.y;
+          x.a.x = n > 0 ? nw.a.x : x.a.x;
+          x.a.y = n > 1 ? nw.a.y : x.a.y;
+          x.b.x = n > 2 ? nw.b.x : x.b.x;
+          x.b.y = n > 3 ? nw.b.y : x.b.y;
         };
         take(p.hx, nhx);
         take(p.hy, nhy);
@@ -376,7 +382,7 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
     } else {
       const int row = r - LV;
       if (vout && row >= i_s && row < i_e) {
-        const unsigned off = (unsigned)row * (unsigned)ny + (unsigned)j0;
+        const unsigned off = (unsigned)row * (unsigned)pitch + (unsigned)j0;
         auto st = [&](float* p, const F4& v) { __stcs(reinterpret_cast<float4*>(p + off), to4(v)); };
         st(a.out.dz, c.dz);
         st(a.out.hx, c.hx);
@@ -395,15 +401,17 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
       }
     }
   };
-  static_assert(RF == 3, "block() names the iterations of a block");
+  static_assert(RF <= 5, "block() names the iterations of a block");
   auto block = [&](auto inttag) {
     iterate(std::integral_constant<int, 0>{}, inttag);
     iterate(std::integral_constant<int, 1>{}, inttag);
     iterate(std::integral_constant<int, 2>{}, inttag);
+    if constexpr (RF > 3) iterate(std::integral_constant<int, 3 % RF>{}, inttag);
+    if constexpr (RF > 4) iterate(std::integral_constant<int, 4 % RF>{}, inttag);
   };
 
   // ---- down the segment: the last warp's last level has to complete row i_e-1
-  const int n_blk = (i_e - 1 + LV - (RF - 1) + kChainLag * (NC - 1) - b0 + RF - 1) / RF + 1;
+  const int n_blk = (i_e - 1 + LV - (RF - 1) + chain_lag(LV) * (NC - 1) - b0 + RF - 1) / RF + 1;
   int gb = rb - LV;  // rows gb .. gb+63 are in gm
   unsigned long long gm = cint ? rows_ok(gb) | (unsigned long long)rows_ok(gb + 32) << 32 : 0ull;
   constexpr unsigned long long kTouch = (1ull << (LV + RF)) - 1;  // rows rb-LV .. rb+RF-1 that a block touches
@@ -420,7 +428,6 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
     else block(std::false_type{});
     rb += RF;
     ms = ms + RF >= MT + LV - 1 ? ms + RF - MT : ms + RF;
-    par = RF - par;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (a.status && __any_sync(kAll, !fin) && lane == 0) raise_status(a.status, ST_NONFINITE);

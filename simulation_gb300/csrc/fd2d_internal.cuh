@@ -24,6 +24,13 @@ int launch_fourier(int t, const fdtd2d_params& p, const fdtd2d_state& s, cudaStr
 int launch_step3(int t, const fdtd2d_params& p, const fdtd2d_state& s, cudaStream_t st);
 int launch_dielectric(int nx, int ny, int npml, double rgrid, double dt, double epsr, double sigma, float* naz,
                       float* nbz, cudaStream_t st);
+struct FieldSet;
+// fields (and materials) between arrays of ny and of `pitch` columns a row; pad
+// columns are zero
+int launch_pad(const FieldSet& in, const FieldSet& out, const float* naz, float* naz_p, const float* nbz, float* nbz_p,
+               int nx, int ny, int pitch, cudaStream_t st);
+int launch_unpad(const FieldSet& in, const FieldSet& out, const float* ez_p, float* ez, int nx, int ny, int pitch,
+                 cudaStream_t st);
 int launch_check_finite(const float* x, size_t n, int* status, cudaStream_t st);
 
 // One pass of the fused streaming kernel (fd2d_march.cu): reads the level-0

@@ -525,4 +525,52 @@ int launch_check_finite(const float* x, size_t n, int* status, cudaStream_t st) 
   return fdtd_host::check_launch();
 }
 
+// Copies of up to 9 arrays between rows of `from` and of `to` columns; columns
+// past ny are written as 0.  HBM-bound: one read and one write of each value,
+// coalesced; blockIdx.z picks the array.
+struct PadArgs {
+  const float* src[9];
+  float* dst[9];
+  int nx, ny, from, to;
+};
+__global__ void k_repitch(const PadArgs a) {
+  const float* __restrict__ s = a.src[blockIdx.z];
+  float* __restrict__ d = a.dst[blockIdx.z];
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= a.to) return;
+  for (int i = blockIdx.y * 8; i < min(a.nx, (int)blockIdx.y * 8 + 8); ++i)
+    d[(size_t)i * a.to + j] = j < a.ny ? s[(size_t)i * a.from + j] : 0.f;
+}
+
+static int repitch(const float* const (&src)[9], float* const (&dst)[9], int nx, int ny, int from, int to,
+                   cudaStream_t st) {
+  PadArgs a{};
+  int n = 0;
+  for (int k = 0; k < 9; ++k)
+    if (src[k] && dst[k]) {
+      a.src[n] = src[k];
+      a.dst[n++] = dst[k];
+    }
+  a.nx = nx;
+  a.ny = ny;
+  a.from = from;
+  a.to = to;
+  const int rows = (nx + 7) / 8;
+  if (rows > 65535) return FDTD_ERR_SIZE;
+  k_repitch<<<dim3((to + 255) / 256, rows, n), 256, 0, st>>>(a);
+  return fdtd_host::check_launch();
+}
+
+int launch_pad(const FieldSet& in, const FieldSet& out, const float* naz, float* naz_p, const float* nbz, float* nbz_p,
+               int nx, int ny, int pitch, cudaStream_t st) {
+  return repitch({in.dz, in.iz, in.hx, in.hy, in.ihx, in.ihy, naz, nbz, nullptr},
+                 {out.dz, out.iz, out.hx, out.hy, out.ihx, out.ihy, naz_p, nbz_p, nullptr}, nx, ny, ny, pitch, st);
+}
+
+int launch_unpad(const FieldSet& in, const FieldSet& out, const float* ez_p, float* ez, int nx, int ny, int pitch,
+                 cudaStream_t st) {
+  return repitch({in.dz, in.iz, in.hx, in.hy, in.ihx, in.ihy, ez_p, nullptr, nullptr},
+                 {out.dz, out.iz, out.hx, out.hy, out.ihx, out.ihy, ez, nullptr, nullptr}, nx, ny, pitch, ny, st);
+}
+
 }  // namespace fdtd

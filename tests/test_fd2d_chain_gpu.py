@@ -1,4 +1,5 @@
-"""The chained passes of 4 and 8 steps (large grids) against the per-function
+"""The chained passes of 4 and 8 steps (large grids; padded copies where ny is
+no multiple of 4) against the per-function
 kernels, bitwise: sizes around the stripes and segments, with and without loss
 and absorbing layer, sources at stripe and segment borders, step counts that
 take every pass length, and the march on the same grid."""
@@ -10,7 +11,8 @@ from tests.test_fd2d_tile_gpu import _equal, _sim
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny", [(1024, 1400), (1100, 1344), (8200, 132), (70, 16384), (2049, 1012), (1500, 1504)])
+@pytest.mark.parametrize("nx,ny", [(1024, 1400), (1100, 1344), (8200, 132), (70, 16384), (2049, 1012), (1500, 1504),
+                                   (1501, 1203), (1300, 1345), (1024, 1402)])
 @pytest.mark.parametrize("lossy,npml", [(False, 0), (False, 20), (True, 0), (True, 20)])
 def test_sizes(cuda_lib, nx, ny, lossy, npml):
     mk = lambda: _sim(nx, ny, lossy, npml, (nx // 2, ny // 2))  # noqa: E731
