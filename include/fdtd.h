@@ -332,6 +332,9 @@ int fdtd_gemm_bf16(const fdtd_gemm_desc* d, int* status, fdtd_stream_t stream);
 /* lift from cin <= 8 input channels per position: x0 = in P^T + p */
 int fno_lift_fwd(long long rows, int C, int cin, const float* in, const float* P, const float* p, void* x0,
                  fdtd_stream_t stream);
+/* fno_lift_bwd32 takes dx0 in FP32 (rounded to BF16 as it is read); C % 8 == 0, C <= 2048, dx0 16-byte aligned */
+int fno_lift_bwd32(long long rows, int C, int cin, const float* in, const float* dx0, float* dP, float* dp,
+                   fdtd_stream_t stream);
 int fno_lift_bwd(long long rows, int C, int cin, const float* in, const void* dx0, float* dP, float* dp,
                  fdtd_stream_t stream);
 /* Propagation frame of a slab profile: feat [n][nbins][6] = (eps_r-1)/eps_scale of
@@ -368,6 +371,11 @@ int fno_small_matmul(int batch, int M, int N, int K, const float* A, const float
 int fno_build_rbig_rect(int M, int Co, int Ci, const float* Rr, const float* Ri, void* Rbig, fdtd_stream_t stream);
 int fno_gelu_fwd(long long n, const float* z, void* y, void* pre, fdtd_stream_t stream);
 int fno_gelu_bwd(long long n, const void* dy16, const float* dy32, const void* pre, void* dz, fdtd_stream_t stream);
+/* the same with the bias gradient, over rows x C values: dz, and dsum[c] += sum of dz[.][c].  One of
+ * dy16, dy32 [rows][C] and dh [rows/N][C] (the gradient of the mean over N positions) is given; C % 8 == 0,
+ * C <= 2048, arrays 16-byte aligned */
+int fno_gelu_bwd_sum(long long rows, int C, int N, const void* dy16, const float* dy32, const float* dh, const void* pre,
+                     void* dz, float* dsum, fdtd_stream_t stream);
 int fno_meanpool(int B, int N, int C, const void* x, void* h, fdtd_stream_t stream);
 int fno_meanpool_bwd(int B, int N, int C, const float* dh, void* dx, fdtd_stream_t stream);
 int fno_colsum(long long rows, int C, const void* x16, const float* x32, float* out, fdtd_stream_t stream);

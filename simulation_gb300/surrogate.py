@@ -363,9 +363,11 @@ class FNO:
         gemm(dz1, s["h"], a_mn=True, b_mn=True, out=self.g["H1"])               # dH1 = dz1^T h
         _call("fno_colsum", Bn, H, dz1.data_ptr(), None, self.g["hb1"].data_ptr())
         dh = gemm(dz1, self.w16["H1"], b_mn=True)                               # dh = dz1 H1  [B][C]
-        dx16 = torch.empty((Bn, N, C), dtype=BF, device=dev)
-        _call("fno_meanpool_bwd", Bn, N, C, dh.data_ptr(), dx16.data_ptr())
-        dx32 = None
+        wide = C % 8 == 0 and C <= 2048  # the fused kernels' channel groups
+        dx16 = dx32 = None
+        if not wide:
+            dx16 = torch.empty((Bn, N, C), dtype=BF, device=dev)
+            _call("fno_meanpool_bwd", Bn, N, C, dh.data_ptr(), dx16.data_ptr())
         parts = torch.empty((Bn, C, C), dtype=torch.float32, device=dev)
         dG = torch.empty((Bn, C, 2 * M), dtype=torch.float32, device=dev)
         dGm = torch.empty((M, Bn, 2 * C), dtype=BF, device=dev)
@@ -376,11 +378,13 @@ class FNO:
         psi_b = self.psi16.unsqueeze(0).expand(Bn, -1, -1)
         for l in reversed(range(self.L)):
             x, pre, Fm = s["x"][l], s["pre"][l], s["Fm"][l]
-            if dx32 is None:
-                _call("fno_gelu_bwd", dz.numel(), dx16.data_ptr(), None, pre.data_ptr(), dz.data_ptr())
+            p16, p32 = None if dx16 is None else dx16.data_ptr(), None if dx32 is None else dx32.data_ptr()
+            if wide:
+                _call("fno_gelu_bwd_sum", Bn * N, C, N, None, p32, dh.data_ptr() if p32 is None else None,
+                      pre.data_ptr(), dz.data_ptr(), self.g[f"L{l}.b"].data_ptr())
             else:
-                _call("fno_gelu_bwd", dz.numel(), None, dx32.data_ptr(), pre.data_ptr(), dz.data_ptr())
-            _call("fno_colsum", Bn * N, C, dz.data_ptr(), None, self.g[f"L{l}.b"].data_ptr())
+                _call("fno_gelu_bwd", dz.numel(), p16 if p32 is None else None, p32, pre.data_ptr(), dz.data_ptr())
+                _call("fno_colsum", Bn * N, C, dz.data_ptr(), None, self.g[f"L{l}.b"].data_ptr())
             # dW = sum_b dz_b^T x_b  (per-sample products, then summed)
             gemm(dz, x, a_mn=True, b_mn=True, out=parts)
             _call("fno_sum_parts", Bn, C * C, parts.data_ptr(), self.g[f"L{l}.W"].data_ptr())
@@ -395,6 +399,10 @@ class FNO:
             nd = torch.empty((Bn, N, C), dtype=torch.float32, device=dev)
             gemm(dz, self.w16[f"L{l}.W"], b_mn=True, out=nd, second=(self.phi16, dF, True, False))
             dx32 = nd
+        if wide:
+            _call("fno_lift_bwd32", Bn * N, C, self.cin, s["inp"].data_ptr(), dx32.data_ptr(), self.g["P"].data_ptr(),
+                  self.g["pb"].data_ptr())
+            return
         dx0 = torch.empty((Bn, N, C), dtype=BF, device=dev)
         _call("fno_to_bf16", dx32.numel(), dx32.data_ptr(), dx0.data_ptr())
         _call("fno_lift_bwd", Bn * N, C, self.cin, s["inp"].data_ptr(), dx0.data_ptr(), self.g["P"].data_ptr(),

@@ -1,0 +1,57 @@
+"""The fused backward kernels of the surrogate against plain FP32/FP64 torch:
+GELU backward with the bias sum from each of its three sources, and the lift's
+backward from FP32 gradients, at row counts and widths off the blocks' shape."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _gelu_grad(z):
+    u = np.sqrt(2 / np.pi) * (z + 0.044715 * z ** 3)
+    t = torch.tanh(u)
+    return 0.5 * (1 + t) + 0.5 * z * (1 - t * t) * np.sqrt(2 / np.pi) * (1 + 3 * 0.044715 * z * z)
+
+
+@pytest.mark.parametrize("C,B,N", [(8, 1, 1), (24, 3, 7), (128, 5, 33), (128, 64, 512), (264, 2, 129), (2048, 2, 5)])
+@pytest.mark.parametrize("src", ["dy16", "dy32", "dh"])
+def test_gelu_bwd_sum(cuda_lib, C, B, N, src):
+    from simulation_gb300 import surrogate as S
+    g = torch.Generator().manual_seed(C + N)
+    rows = B * N
+    pre = torch.randn((rows, C), generator=g).cuda().bfloat16()
+    dy = torch.randn((rows, C), generator=g).cuda()
+    dh = torch.randn((B, C), generator=g).cuda()
+    dz = torch.empty((rows, C), dtype=torch.bfloat16, device="cuda")
+    db = torch.ones(C, device="cuda")
+    d16 = dy.bfloat16()
+    S._call("fno_gelu_bwd_sum", rows, C, N, d16.data_ptr() if src == "dy16" else None,
+            dy.data_ptr() if src == "dy32" else None, dh.data_ptr() if src == "dh" else None, pre.data_ptr(),
+            dz.data_ptr(), db.data_ptr())
+    ref_d = {"dy16": d16.double(), "dy32": dy.double(),
+             "dh": (dh / N).bfloat16().double().repeat_interleave(N, 0)}[src]
+    ref = ref_d * _gelu_grad(pre.double())
+    torch.cuda.synchronize()
+    # BF16 rounding (2^-9) of the result, and the hardware tanh (2^-11) in it
+    assert float((dz.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max())
+    # the sum is of the stored values, in FP32: rows rounding errors of the running sum at most
+    want = 1 + dz.double().sum(0)
+    scale = dz.double().abs().sum(0) + 1
+    assert float(((db.double() - want).abs() / scale).max()) <= 1e-6
+
+
+@pytest.mark.parametrize("cin", [1, 6, 8])
+@pytest.mark.parametrize("rows,C", [(1, 8), (77, 24), (4096, 128), (513, 264)])
+def test_lift_bwd32(cuda_lib, rows, C, cin):
+    from simulation_gb300 import surrogate as S
+    g = torch.Generator().manual_seed(rows + cin)
+    x = torch.randn((rows, cin), generator=g).cuda()
+    dx = torch.randn((rows, C), generator=g).cuda()
+    dP, dp = torch.zeros((C, cin), device="cuda"), torch.zeros(C, device="cuda")
+    S._call("fno_lift_bwd32", rows, C, cin, x.data_ptr(), dx.data_ptr(), dP.data_ptr(), dp.data_ptr())
+    d = dx.bfloat16().double()
+    torch.cuda.synchronize()
+    lim = 1e-6 * (d.abs().T @ x.double().abs() + 1)
+    assert bool(((dP.double() - d.T @ x.double()).abs() <= lim).all())
+    assert bool(((dp.double() - d.sum(0)).abs() <= 1e-6 * (d.abs().sum(0) + 1)).all())
