@@ -165,6 +165,7 @@ _SIGS = {
     "fno_small_matmul": ([C.c_int, C.c_int, C.c_int, C.c_int, F, F, F, P], C.c_int),
     "fno_build_rbig_rect": ([C.c_int, C.c_int, C.c_int, F, F, P, P], C.c_int),
     "fno_gelu_fwd": ([C.c_longlong, F, P, P, P], C.c_int),
+    "fno_layer_fwd": ([C.c_int] * 5 + [P, P, F, P, P, P, P, P, P, P, P], C.c_int),
     "fno_gelu_bwd": ([C.c_longlong, P, F, P, P, P], C.c_int),
     "fno_gelu_bwd_sum": ([C.c_longlong, C.c_int, C.c_int, P, F, F, P, P, F, P], C.c_int),
     "fno_lift_bwd32": ([C.c_longlong, C.c_int, C.c_int, F, F, F, F, P], C.c_int),

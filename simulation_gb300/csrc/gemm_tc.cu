@@ -23,14 +23,9 @@
 // backward pass need MN-major), selected per call.  Every wait on an mbarrier
 // is bounded (about 2 s): on expiry the kernel records FDTD_STATUS_TIMEOUT in
 // the status word and finishes without further waits.
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cudaTypedefs.h>
-
 #include <algorithm>
-#include <mutex>
 
-#include "fdtd_common.cuh"
+#include "tc_common.cuh"
 
 namespace fdtd {
 namespace {
@@ -61,75 +56,6 @@ struct GemmArgs {
   int a2_mn, b2_mn, a2_shared, b2_shared;
   int* status;
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t a, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t a, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-
-// bounded wait on an mbarrier phase; false (and TIMEOUT recorded) on expiry
-__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, int* status) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (clock64() - t0 > 4000000000LL) {
-      raise_status(status, ST_TIMEOUT);
-      return false;
-    }
-  }
-}
-
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, int c0, int c1, int c2,
-                                            uint32_t mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-      "[%5];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(c0), "r"(c1), "r"(c2), "r"(mbar)
-      : "memory");
-}
-
-// shared-memory matrix descriptor (tcgen05): start address, leading and
-// stride byte offsets (16-byte units), descriptor version 1, 128B swizzle
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-// instruction descriptor, kind::f16: BF16 A and B, FP32 accumulator, M x N
-__host__ __device__ constexpr uint32_t instr_desc(int m, int n, int a_mn, int b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
-         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-// GELU, tanh form (Hendrycks & Gimpel 2016): 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))
-// with the hardware tanh approximation
-__device__ __forceinline__ float tanh_hw(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float gelu(float z) {
-  const float u = 0.7978845608028654f * fmaf(0.044715f * z, z * z, z);
-  return 0.5f * z * (1.0f + tanh_hw(u));
-}
 
 // Persistent, warp-specialised kernel: warps 0-7 drain accumulators
 // (epilogue), warp 8 is the TMA producer, warp 9 issues the MMAs.  Two TMEM
@@ -229,7 +155,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   } else if (warp == EPI_WARPS + 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const uint32_t lead = elect_lane();
       const uint32_t idesc1 = instr_desc(BM, BN, a.a_mn, a.b_mn);
       const uint32_t idesc2 = instr_desc(BM, BN, a.a2_mn, a.b2_mn);
       long long g = 0;
@@ -237,12 +164,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       bool ok = true;
       for (long long t = blockIdx.x; t < total && ok; t += gridDim.x, ++i) {
         const int b = i & 1;
-        if (i >= 2 && !(ok = mbar_wait(smem_u32(&tempty[b]), (uint32_t)(((i >> 1) - 1) & 1), a.status))) break;
+        if (i >= 2 && !(ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&tempty[b]), (uint32_t)(((i >> 1) - 1) & 1), a.status)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t dacc = tmem + (uint32_t)(b * BN);
         for (int kb = 0; kb < kblocks; ++kb, ++g) {
           const int s = (int)(g % STAGES);
-          if (!(ok = mbar_wait(smem_u32(&full[s]), (uint32_t)((g / STAGES) & 1), a.status))) break;
+          if (!(ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), (uint32_t)((g / STAGES) & 1), a.status)))) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t sa = smem_u32(tiles + s * STAGE_BYTES);
           const uint32_t sb = sa + A_BYTES;
@@ -257,20 +184,12 @@ __global__ void __launch_bounds__(THREADS, 1)
             const uint64_t bd =
                 bmn ? smem_desc(sb + kk * 2048, a.lbo_mn, a.sbo_mn) : smem_desc(sb + kk * 32, 16, 1024);
             const uint32_t acc = (kb > 0 || kk > 0) ? 1u : 0u;
-            asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dacc),
-                "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                : "memory");
+            mma_bf16(lead, dacc, ad, bd, idesc, acc);
           }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_u32(&empty[s]))
-                       : "memory");
+          mma_commit(lead, smem_u32(&empty[s]));
         }
         if (ok)
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_u32(&tfull[b]))
-                       : "memory");
+          mma_commit(lead, smem_u32(&tfull[b]));
       }
     }
   } else {
@@ -294,16 +213,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int c0 = c_begin; c0 < c_end; c0 += 32) {
         uint32_t r[32];
         const uint32_t taddr = tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)(b * BN + c0);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-              "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-              "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-              "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(taddr)
-            : "memory");
+        tmem_ld32(taddr, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (c0 + 32 >= c_end) {
           // this warp's part of the accumulator has been read: release it
@@ -415,36 +325,6 @@ __global__ void __launch_bounds__(THREADS, 1)
 }
 
 // ----------------------------------------------------------------- host
-PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-std::mutex g_encode_mu;
-
-int get_encode() {
-  std::lock_guard<std::mutex> lk(g_encode_mu);
-  if (g_encode) return FDTD_OK;
-  void* fn = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q);
-  if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn) {
-    fdtd_host::note_cuda_error(e);
-    return FDTD_ERR_CUDA;
-  }
-  g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  return FDTD_OK;
-}
-
-// 3D tensor map over a BF16 operand: dims {inner, outer, batch}
-int make_map(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t outer, uint64_t batch, uint64_t ld_elems,
-             uint64_t stride_elems, uint32_t box_inner, uint32_t box_outer) {
-  cuuint64_t dims[3] = {inner, outer, batch};
-  cuuint64_t strides[2] = {ld_elems * 2, stride_elems * 2};
-  cuuint32_t box[3] = {box_inner, box_outer, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  const CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
-                              es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? FDTD_OK : FDTD_ERR_ARG;
-}
-
 template <int BN, int STAGES>
 size_t smem_bytes() {
   return 1024 + (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 8 * (2 * STAGES + 6) + sizeof(float) * BN;
@@ -486,8 +366,7 @@ extern "C" int fdtd_gemm_bf16(const fdtd_gemm_desc* d, int* status, fdtd_stream_
   if (d->act < 0 || d->act > 1) return FDTD_ERR_ARG;
   if ((d->a_mn_major ? d->lda < d->M : d->lda < d->K) || (d->b_mn_major ? d->ldb < d->N : d->ldb < d->K))
     return FDTD_ERR_SIZE;
-  int rc = get_encode();
-  if (rc) return rc;
+  int rc = FDTD_OK;
   const int BN = (d->N <= 64) ? 64 : 128;
   CUtensorMap ta, tb;
   // an operand with batch stride 0 is shared: one batch slice in its map

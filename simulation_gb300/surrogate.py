@@ -258,8 +258,8 @@ class FNO:
         self.rbig0f = torch.empty((M, 2 * C, 2 * KIN), dtype=BF, device=self.dev)
         _call("fno_build_rbig_rect", M, C, KIN, rr.data_ptr(), ri.data_ptr(), self.rbig0f.data_ptr())
 
-    def _first_layer_folded(self, inp: torch.Tensor, phi_b: torch.Tensor) -> torch.Tensor:
-        """x1 of the first spectral layer straight from the packed inputs."""
+    def _first_modes_folded(self, inp: torch.Tensor):
+        """The packed inputs [B][N][KPW] and their mode coefficients [M][B][2 KIN]."""
         Bn, N, C, M, KIN = inp.shape[0], self.N, self.C, self.M, self.KIN
         dev = self.dev
         # the 64-wide operand lives per (stream, batch size): its zero padding is
@@ -278,6 +278,12 @@ class FNO:
         gemm(inpT, self.phi16, a_mn=True, out=F.view(Bn * KIN, 2 * M))
         Fm = torch.empty((M, Bn, 2 * KIN), dtype=BF, device=dev)
         _call("fno_dft_to_modes", Bn, KIN, M, F.data_ptr(), Fm.data_ptr())
+        return inp16, Fm
+
+    def _first_layer_folded(self, inp: torch.Tensor) -> torch.Tensor:
+        """x1 of the first spectral layer straight from the packed inputs."""
+        Bn, N, C, M, dev = inp.shape[0], self.N, self.C, self.M, self.dev
+        inp16, Fm = self._first_modes_folded(inp)
         Gm = torch.empty((M, Bn, 2 * C), dtype=torch.float32, device=dev)
         gemm(Fm, self.rbig0f, out=Gm)
         G = torch.empty((Bn, C, 2 * M), dtype=BF, device=dev)
@@ -285,6 +291,47 @@ class FNO:
         x = torch.empty((Bn, N, C), dtype=BF, device=dev)
         gemm(inp16, self.w0f16, out=x, bias=self.p["L0.b"], gelu=True, second=(self.psi16, G, False, False))
         return x
+
+    # ------------------------------------------------------------ fused layers
+    def _fused(self, Bn: int) -> bool:
+        """Whether ``fno_layer_fwd`` takes this network and batch."""
+        return self.C == 128 and self.M == 32 and self.N >= 128 and self.N & (self.N - 1) == 0 and Bn <= 65535
+
+    def _layers_fused(self, inp: torch.Tensor, saved: dict | None) -> torch.Tensor:
+        """h [B][C], the mean of the last layer's output: two launches a layer,
+        the mode product and ``fno_layer_fwd``."""
+        Bn, N, C, M, dev = inp.shape[0], self.N, self.C, self.M, self.dev
+        folded = saved is None and self.fold and self.cin + 1 <= self.KIN
+        if folded:
+            x, Fm = self._first_modes_folded(inp)
+        else:
+            x = torch.empty((Bn, N, C), dtype=BF, device=dev)
+            _call("fno_lift_fwd", Bn * N, C, self.cin, inp.data_ptr(), self.p["P"].data_ptr(),
+                  self.p["pb"].data_ptr(), x.data_ptr())
+            F = gemm(x, self.phi16.unsqueeze(0).expand(Bn, -1, -1), a_mn=True)
+            Fm = torch.empty((M, Bn, 2 * C), dtype=BF, device=dev)
+            _call("fno_dft_to_modes", Bn, C, M, F.data_ptr(), Fm.data_ptr())
+        Gm = torch.empty((M, Bn, 2 * C), dtype=BF, device=dev)
+        h = torch.empty((Bn, C), dtype=BF, device=dev)
+        for l in range(self.L):
+            first, last = folded and l == 0, l == self.L - 1
+            gemm(Fm, self.rbig0f if first else self.rbig[l], out=Gm)
+            w = self.w0f16 if first else self.w16[f"L{l}.W"]
+            pre = None
+            if saved is not None:
+                pre = torch.empty((Bn, N, C), dtype=BF, device=dev)
+                for k, v in (("x", x), ("pre", pre), ("Fm", Fm)):
+                    saved[k].append(v)
+            xn = fn = None
+            if not last:
+                xn = torch.empty((Bn, N, C), dtype=BF, device=dev)
+                fn = torch.empty((M, Bn, 2 * C), dtype=BF, device=dev)
+            _call("fno_layer_fwd", Bn, N, C, M, w.shape[1], x.data_ptr(), w.data_ptr(), self.p[f"L{l}.b"].data_ptr(),
+                  self.psi16.data_ptr(), Gm.data_ptr(), None if last else xn.data_ptr(),
+                  None if last else fn.data_ptr(), h.data_ptr() if last else None,
+                  None if pre is None else pre.data_ptr(), None)
+            x, Fm = xn, fn
+        return h
 
     def state_dict(self):
         return {k: v.detach().cpu().clone() for k, v in self.p.items()}
@@ -299,17 +346,19 @@ class FNO:
         """inp [B][N][cin] float32 (device) -> network output y [B][D] float32."""
         Bn, N, C, M = inp.shape[0], self.N, self.C, self.M
         dev = self.dev
-        phi_b = self.phi16.unsqueeze(0).expand(Bn, -1, -1)  # stride 0 over the batch
         folded = not keep and self.fold and self.cin + 1 <= self.KIN
+        if folded and self._folded_stale:
+            self._refresh_folded()
+        saved = {"inp": inp, "x": [], "pre": [], "Fm": []}
+        if self._fused(Bn) and self.L > 0:
+            return self._head(self._layers_fused(inp, saved if keep else None), saved if keep else None)
+        phi_b = self.phi16.unsqueeze(0).expand(Bn, -1, -1)  # stride 0 over the batch
         if folded:
-            if self._folded_stale:
-                self._refresh_folded()
-            x = self._first_layer_folded(inp, phi_b)
+            x = self._first_layer_folded(inp)
         else:
             x = torch.empty((Bn, N, C), dtype=BF, device=dev)
             _call("fno_lift_fwd", Bn * N, C, self.cin, inp.data_ptr(), self.p["P"].data_ptr(),
                   self.p["pb"].data_ptr(), x.data_ptr())
-        saved = {"inp": inp, "x": [], "pre": [], "Fm": []}
         F = torch.empty((Bn, C, 2 * M), dtype=torch.float32, device=dev)
         Fm = torch.empty((M, Bn, 2 * C), dtype=BF, device=dev)
         Gm = torch.empty((M, Bn, 2 * C), dtype=torch.float32, device=dev)
@@ -334,13 +383,18 @@ class FNO:
             x = xn
         h = torch.empty((Bn, C), dtype=BF, device=dev)
         _call("fno_meanpool", Bn, N, C, x.data_ptr(), h.data_ptr())
+        return self._head(h, saved if keep else None)
+
+    def _head(self, h: torch.Tensor, saved: dict | None) -> torch.Tensor:
+        """y [B][D] from the pooled activations h [B][C]."""
+        Bn, dev = h.shape[0], self.dev
         a1 = torch.empty((Bn, self.H), dtype=BF, device=dev)
         z1 = torch.empty((Bn, self.H), dtype=BF, device=dev)
         gemm(h, self.w16["H1"], out=a1, bias=self.p["hb1"], gelu=True, pre=z1)
         o = torch.empty((Bn, self.D), dtype=torch.float32, device=dev)
         gemm(a1, self.w16["H2"], out=o, bias=self.p["hb2"])
-        if keep:
-            saved.update(h=h, a1=a1, z1=z1, xL=x)
+        if saved is not None:
+            saved.update(h=h, a1=a1, z1=z1)
             self._saved = saved
         return o
 
