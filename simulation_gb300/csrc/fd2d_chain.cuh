@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
       const F4 curl = {make_float2(__fadd_rn(d.a.x, hl), __fadd_rn(d.a.y, q.hx.a.x)),
                        make_float2(__fadd_rn(d.b.x, q.hx.a.y), __fadd_rn(d.b.y, q.hx.b.x))};
       if (INT) {
-        q.dz = add4(q.dz, mul4(0.5f, curl));
+        q.dz = sub4(q.dz, mul4(-0.5f, curl));
       } else {
         F4 nd;
         const bool in = row >= 1 && row < nx;
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
           // gx2*(gy2/2) is (gx2*gy2)/2 exactly
           nd = fma4(mul4(gx3, chain_lds(cc + 1 * W)), q.dz, mul4(mul4(gx2, chain_lds(cc + 0 * W)), curl));
         } else {
-          nd = add4(q.dz, mul4(0.5f, curl));
+          nd = sub4(q.dz, mul4(-0.5f, curl));
         }
         q.dz.a.x = in && !col0 ? nd.a.x : q.dz.a.x;
         q.dz.a.y = in ? nd.a.y : q.dz.a.y;
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
         if (PML) {
           p.ihx = add4(p.ihx, cx);
           p.ihy = add4(p.ihy, cy);
-          p.hx = add4(p.hx, mul4(0.5f, cx));
+          p.hx = sub4(p.hx, mul4(-0.5f, cx));
           p.hy = sub4(p.hy, mul4(0.5f, cy));
         } else {
           p.hx = fma4(0.5f, cx, p.hx);

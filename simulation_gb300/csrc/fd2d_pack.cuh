@@ -8,6 +8,9 @@
 namespace fdtd {
 namespace {
 
+// A packed product is not added with add4: the compiler joins the two to one
+// fma, which rounds a subnormal 0.5*x differently.  x + 0.5*y is written
+// sub4(x, mul4(-0.5f, y)).
 struct F4 {  // four cells of a lane as two packed pairs
   float2 a, b;
 };

@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
         if (PML) {
           ihx_set(r, add4(ihx_get(r), cx));
           at(A_IHY, r) = to4(add4(f4(at(A_IHY, r)), cy));
-          hx[r] = add4(hx[r], mul4(0.5f, cx));
+          hx[r] = sub4(hx[r], mul4(-0.5f, cx));
           hy[r] = sub4(hy[r], mul4(0.5f, cy));
         } else {
           hx[r] = fma4(0.5f, cx, hx[r]);
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
                        make_float2(__fadd_rn(d.b.x, hx[r].a.y), __fadd_rn(d.b.y, hx[r].b.x))};
       hup = hy[r];
       if (INT) {
-        dz[r] = add4(dz[r], mul4(0.5f, curl));
+        dz[r] = sub4(dz[r], mul4(-0.5f, curl));
       } else {
         F4 nd;
         if (PML) {
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
           // gx2*(gy2/2) is (gx2*gy2)/2 exactly
           nd = fma4(mul4(make_float2(k.z, k.w), gy3), dz[r], mul4(mul4(make_float2(k.x, k.y), gy2), curl));
         } else {
-          nd = add4(dz[r], mul4(0.5f, curl));
+          nd = sub4(dz[r], mul4(-0.5f, curl));
         }
         nd.a.x = j0 != 0 ? nd.a.x : dz[r].a.x;  // column 0 is not updated
         if (MASK) {                            // nor is row 0

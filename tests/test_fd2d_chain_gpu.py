@@ -41,3 +41,14 @@ def test_nonfinite(cuda_lib):
     a.step(16)
     with pytest.raises(_lib.FdtdError):
         a.check()
+
+
+@pytest.mark.parametrize("lossy,npml", [(False, 0), (False, 12), (True, 12)])
+def test_subnormal_fields(cuda_lib, lossy, npml):
+    mk = lambda: _sim(1024, 1400, lossy, npml, None)  # noqa: E731
+    a, b = mk(), mk()
+    for s in (a, b):
+        s.dz.mul_(1e-37)
+    a.step(24)
+    b.step_per_function(24)
+    _equal(a, b, "subnormal")

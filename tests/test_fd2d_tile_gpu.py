@@ -78,3 +78,15 @@ def test_nonfinite_and_two_streams(cuda_lib):
         r.step_per_function(100)
     for s, r in zip(sims, refs):
         _equal(s, r, "streams")
+
+
+@pytest.mark.parametrize("lossy,npml", [(False, 0), (False, 12), (True, 12)])
+def test_subnormal_fields(cuda_lib, lossy, npml):
+    """fields around the smallest normal number: every product is rounded by itself"""
+    mk = lambda: _sim(400, 512, lossy, npml, None)  # noqa: E731
+    a, b = mk(), mk()
+    for s in (a, b):
+        s.dz.mul_(1e-37)
+    a.step(24)
+    b.step_per_function(24)
+    _equal(a, b, "subnormal")
