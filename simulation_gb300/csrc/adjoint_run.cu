@@ -6,17 +6,25 @@
 // fd2d/python/fd2d_3_4.py:131-136 and a point source after the D update.
 //
 // Schedule (all in the caller's workspace, nothing allocated):
-//   forward   fused passes of up to 4 steps from zero fields; each segment
-//             of `checkpoint` steps starts from a stored state (the previous
-//             segment's last pass writes it directly) and the probe's Ez is
-//             recorded every step; J is summed on the device in double;
-//   reverse   segments last first.  A segment's states are recomputed from
+//   forward   from zero fields, a segment of `checkpoint` steps at a time: one
+//             launch of the on-chip loop where the grid's tiles fit the SMs,
+//             else fused passes of up to 4 steps; each segment starts from a
+//             stored state (the one before writes it directly) and the probe's
+//             Ez is recorded every step; J is summed on the device in double;
+//   reverse   segments last first.  Where the tiles fit: the segment runs
+//             again from its checkpoint, recording what the reverse needs of
+//             it (the design box and the probe), and is undone on the chip,
+//             one launch each.  Else a segment's states are recomputed from
 //             its checkpoint by recording passes (one pass of 4 steps stores
 //             dz, iz, hx, hy after each of its steps), on a second stream,
 //             one segment ahead of the sweep (two record buffers, events
 //             order their reuse); the sweep runs one fused reverse kernel per
 //             two steps (one step for an odd segment's first), the adjoint
 //             fields ping-ponging between two sets.
+// At 1024^2, 1500 steps, checkpoint 64, a lossless 256^2 box: 15.4 ms on the
+// chip (forward 4.7, recording runs 5.0, reverse 5.4) against 38.5 streaming,
+// whose reverse reads two recorded states and the adjoints of every tile from
+// L2 in each launch (33 us for two steps; 7.2 here, exchanges included).
 // Results do not depend on the checkpoint interval or on the overlap: every
 // recorded state is bitwise the forward's, and each reverse step does the
 // same per-cell arithmetic (fdtd2d_adjoint_step's two kernels give the same
@@ -26,6 +34,7 @@
 #include <vector>
 
 #include "fd2d_internal.cuh"
+#include "fd2d_tile.h"
 
 namespace fdtd {
 int launch_adjoint_fused(const fdtd2d_params& p, int t, const fdtd2d_fields& fwd, const fdtd2d_fields& adj_in,
@@ -205,6 +214,17 @@ int check_ws(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, void* ws, s
   return FDTD_OK;
 }
 
+// The on-chip loop's layout for this grid, when it has one (its flags go to
+// the Ez slot, which its runs leave alone).
+bool tile_layout(const fdtd2d_params* p, const Layout& L, TilePlan& pl, int max_V = 5) {
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  return tile_plan(p->nx, p->ny, p->nbz != nullptr, true, std::min(nsm, kTileMaxBlocks), pl, max_V) &&
+         (size_t)pl.n_ti * pl.n_tj * 128 <= L.slot;
+}
+
 int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* trace, double* J, void* ws,
                 cudaStream_t st) {
   const Layout L = layout(p0, a, ws);
@@ -216,9 +236,18 @@ int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* 
   if (rc) return rc;
   if ((rc = cuda_rc(cudaMemsetAsync(trace, 0, (size_t)a->nsteps * sizeof(float), st)))) return rc;
   float* ez = at(L, L.ez);
+  TilePlan pl;
+  const bool tile = tile_layout(&p, L, pl);
   for (int c = 0; c < L.ncp; ++c) {
     const int t_start = c * L.cp;
     const int len = std::min(L.cp, a->nsteps - t_start);
+    if (tile && len >= kTileMinSteps) {
+      const FieldSet out = set_of(ckpt(&p, L, c + 1));
+      if ((rc = launch_tile(p, set_of(ckpt(&p, L, c)), out, set_of(xbuf(&p, L, 0)), out, nullptr, t_start, len,
+                            nullptr, trace, (unsigned*)ez, pl, st)))
+        return rc;
+      continue;
+    }
     const int kk = march_default_steps(p.nx, p.ny);
     const int npass = (len + kk - 1) / kk;
     fdtd2d_fields in = ckpt(&p, L, c);
@@ -256,17 +285,56 @@ int recompute(const fdtd2d_params* p, const Layout& L, int c, int len, int b, cu
   return FDTD_OK;
 }
 
+// The reverse sweep on the chip: segments last first, each run forward again
+// from its checkpoint to record the design box's dz' - iz and the probe's ez
+// (cp steps of at most a grid each, in the room of six recorded states a step),
+// then undone in one launch, all on the caller's stream.
+int run_reverse_tile(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* grad_naz, float* grad_nbz,
+                     const Layout& L, const TilePlan& fwd, const TilePlan& rev, cudaStream_t st) {
+  fdtd2d_params p = *p0;
+  p.probe_i = a->probe_i;
+  p.probe_j = a->probe_j;
+  TileAdj adj;
+  adj.box = a->box;
+  adj.jb = a->box.j0 & ~3;
+  adj.njp = ((a->box.j0 + a->box.nj + 3) & ~3) - adj.jb;
+  adj.rec = at(L, L.rec0);
+  adj.probe_w = a->probe_weight;
+  adj.grad_naz = grad_naz;
+  adj.grad_nbz = grad_nbz;
+  float* probe = adj.rec + (size_t)L.cp * adj.box.ni * adj.njp;  // [cp]
+  unsigned* flags = (unsigned*)at(L, L.ez);
+  const FieldSet x0 = set_of(xbuf(&p, L, 0)), x1 = set_of(xbuf(&p, L, 1));
+  int cur = 0;
+  for (int c = L.ncp - 1; c >= 0; --c) {
+    const int t_start = c * L.cp, len = std::min(L.cp, a->nsteps - t_start);
+    float* pz = probe - t_start;  // indexed by step
+    int rc = launch_tile(p, set_of(ckpt(&p, L, c)), x1, x0, x1, nullptr, t_start, len, nullptr, pz, flags, fwd, st,
+                         kTileRec, &adj);
+    if (rc) return rc;
+    const FieldSet out = set_of(adjbuf(&p, L, 1 - cur));
+    rc = launch_tile(p, set_of(adjbuf(&p, L, cur)), out, x0, out, nullptr, t_start + len, len, nullptr, pz, flags, rev,
+                     st, kTileRev, &adj);
+    if (rc) return rc;
+    cur = 1 - cur;
+  }
+  return FDTD_OK;
+}
+
 int run_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz, float* grad_nbz,
                 void* ws, cudaStream_t main) {
   const Layout L = layout(p, a, ws);
-  Side* side = nullptr;
-  int rc = side_of_device(&side);
-  if (rc) return rc;
-  cudaStream_t ss = side->stream;
+  int rc;
   const size_t gb = (size_t)a->box.ni * a->box.nj * sizeof(float);
   if ((rc = zero_fields(p, adjbuf(p, L, 0), main))) return rc;
   if ((rc = cuda_rc(cudaMemsetAsync(grad_naz, 0, gb, main)))) return rc;
   if (grad_nbz && (rc = cuda_rc(cudaMemsetAsync(grad_nbz, 0, gb, main)))) return rc;
+  TilePlan fwd, rev;
+  if (L.cp >= kTileMinSteps && tile_layout(p, L, fwd) && tile_layout(p, L, rev, tile_rev_max_V(p->nbz != nullptr)))
+    return run_reverse_tile(p, a, grad_naz, grad_nbz, L, fwd, rev, main);
+  Side* side = nullptr;
+  if ((rc = side_of_device(&side))) return rc;
+  cudaStream_t ss = side->stream;
   // the side stream starts after everything before this call on the caller's stream
   if ((rc = cuda_rc(cudaEventRecord(side->fork, main)))) return rc;
   if ((rc = cuda_rc(cudaStreamWaitEvent(ss, side->fork, 0)))) return rc;

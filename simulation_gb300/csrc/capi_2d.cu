@@ -3,7 +3,7 @@
 
 #include "fd2d_chain.cuh"
 #include "fd2d_internal.cuh"
-#include "fd2d_tile.cuh"
+#include "fd2d_tile.h"
 
 namespace {
 
@@ -267,7 +267,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
 
   TilePlan tile;
   // (a call's load and store of the tiles, 15 us at 1024^2, is two march passes: not worth it below 4 steps)
-  if (nsteps >= 4 && workspace && ((uintptr_t)workspace & 255u) == 0 && workspace_bytes >= tile_workspace_bytes(p) &&
+  if (nsteps >= kTileMinSteps && workspace && ((uintptr_t)workspace & 255u) == 0 && workspace_bytes >= tile_workspace_bytes(p) &&
       tile_ok(p, steps_per_pass, tile)) {
     const FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
     unsigned* flags = (unsigned*)((char*)workspace + slot_bytes(p) * nslots(p));

@@ -12,9 +12,9 @@ namespace fdtd {
 // 2: 0.75, 5: 1.7), loss adds 0.1 V; an exchange 2.1 + 0.52 V (fence, flag and
 // read latencies, and the halo's traffic), once in T steps.  100^2 runs 1.2 a
 // step with V = 1, T = 4 (6.2 marching), 1024^2 3.3 with V = 5, T = 4 (10.5).
-bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& best) {
+bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& best, int max_V) {
   double best_cost = 1e30;
-  for (int V = 1; V <= 5; ++V)
+  for (int V = 1; V <= max_V; ++V)
     for (int T = 2; T <= 8; ++T) {
       TilePlan pl;
       pl.V = V;
@@ -39,36 +39,10 @@ bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& b
 
 namespace {
 
-template <int V, bool LOSSY, bool PML>
-int launch_t(const TileArgs& a, cudaStream_t st) {
-  auto kern = k_tile<V, LOSSY, PML>;
-  const size_t smem = tile_smem_bytes(V, LOSSY, PML);
-  cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(a.n_ti * a.n_tj, 1, 1);
-    cfg.blockDim = dim3(kTileWarps * 32, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;  // all blocks resident: they wait on one another
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, a);
-  }
-  if (e != cudaSuccess) {
-    fdtd_host::note_cuda_error(e);
-    return FDTD_ERR_CUDA;
-  }
-  return fdtd_host::check_launch();
-}
-
 template <int V>
 int launch_v(const TileArgs& a, bool lossy, bool pml, cudaStream_t st) {
-  if (lossy) return pml ? launch_t<V, true, true>(a, st) : launch_t<V, true, false>(a, st);
-  return pml ? launch_t<V, false, true>(a, st) : launch_t<V, false, false>(a, st);
+  if (lossy) return pml ? launch_t<V, true, true, kTileFwd>(a, st) : launch_t<V, true, false, kTileFwd>(a, st);
+  return pml ? launch_t<V, false, true, kTileFwd>(a, st) : launch_t<V, false, false, kTileFwd>(a, st);
 }
 
 bool al16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
@@ -77,7 +51,7 @@ bool al16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, const FieldSet& x0, const FieldSet& x1,
                 float* ez, int t0, int nsteps, int* status, float* probe_ez, unsigned* flags, const TilePlan& pl,
-                cudaStream_t st) {
+                cudaStream_t st, int mode, const TileAdj* adj) {
   TileArgs a{};
   a.nx = p.nx;
   a.ny = p.ny;
@@ -100,6 +74,7 @@ int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out,
   a.probe_j = p.probe_j;
   a.probe_ez = probe_ez;
   a.flags = flags;
+  if (adj) a.adj = *adj;
   a.T = pl.T;
   a.hc = pl.hc;
   a.n_ti = pl.n_ti;
@@ -118,6 +93,10 @@ int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out,
       fdtd_host::note_cuda_error(e);
       return FDTD_ERR_CUDA;
     }
+  }
+  if (mode != kTileFwd) {
+    if (!pml || !v || !adj) return FDTD_ERR_ARG;
+    return mode == kTileRec ? launch_tile_rec(a, pl.V, lossy, st) : launch_tile_rev(a, pl.V, lossy, st);
   }
   switch (pl.V) {
     case 1: return launch_v<1>(a, lossy, pml, st);

@@ -27,12 +27,20 @@
 //
 // Same step order and per-cell formulas as the per-function kernels: results
 // are bitwise equal to theirs.
+//
+// The adjoint's reverse sweep runs in the same frame (kTileRev): the adjoint
+// fields take the fields' places, an undone step reaches one cell in each
+// direction as a step does, and the two values that cross strips are the
+// adjoint of cy downwards and that of the D update's curl upwards.  All it
+// needs of the forward run is dz' - iz in the design box and ez at the probe,
+// which a forward run in mode kTileRec leaves per step.
 #pragma once
 
 #include <type_traits>
 
 #include "fd2d_internal.cuh"
 #include "fd2d_pack.cuh"
+#include "fd2d_tile.h"
 
 namespace fdtd {
 
@@ -54,6 +62,7 @@ struct TileArgs {
   int probe_i, probe_j;
   float* probe_ez;
   unsigned* flags;    // one per block, 32 words apart, zero at the start
+  TileAdj adj;        // modes kTileRec and kTileRev
   int T;              // steps between exchanges = halo rows
   int hc;             // halo columns on each side: T rounded up to whole lanes, or 0 with one tile per row
   int n_ti, n_tj;
@@ -61,30 +70,24 @@ struct TileArgs {
   int vec;            // ny % 4 == 0 and all arrays 16-byte aligned
 };
 
-struct TilePlan {
-  int V = 0, T = 0, hc = 0, n_ti = 0, n_tj = 0, own_r = 0, own_c = 0;
-};
-constexpr int kTileMaxBlocks = 152;                       // one per SM
-constexpr size_t kTileFlagBytes = kTileMaxBlocks * 128;  // flags of the largest launch
-
 // shared memory of a block, in float4: arrays of 16*V rows of 32 float4 (naz,
 // [ihy], [nbz, iz]), the strips' edge rows, the column and row coefficients
 // (at 5 rows a warp ihx moves there too: with it in registers the general
 // steps spill)
 __host__ __device__ constexpr bool tile_ihx_smem(int V, bool pml) { return pml && V >= 5; }
-__host__ __device__ constexpr int tile_arrays(int V, bool lossy, bool pml) {
-  return 1 + (pml ? 1 : 0) + (lossy ? 2 : 0) + (tile_ihx_smem(V, pml) ? 1 : 0);
+__host__ __device__ constexpr int tile_arrays(int V, bool lossy, bool pml, int mode) {
+  return 1 + (pml ? 1 : 0) + (lossy ? 2 : 0) + (tile_ihx_smem(V, pml) ? 1 : 0) +
+         (mode == kTileRev ? (lossy ? 2 : 1) : 0);  // the box's gradients
 }
-__host__ __device__ constexpr size_t tile_smem_bytes(int V, bool lossy, bool pml) {
-  return sizeof(float4) * ((size_t)kTileWarps * V * 32 * tile_arrays(V, lossy, pml) + 2 * kTileWarps * 32 + 5 * 32 +
+__host__ __device__ constexpr size_t tile_smem_bytes(int V, bool lossy, bool pml, int mode) {
+  return sizeof(float4) * ((size_t)kTileWarps * V * 32 * tile_arrays(V, lossy, pml, mode) + 2 * kTileWarps * 32 + 5 * 32 +
                            3 * kTileWarps * V);
 }
 
-// defined in fd2d_tile.cu
-bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& best);
-int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, const FieldSet& x0, const FieldSet& x1,
-                float* ez, int t0, int nsteps, int* status, float* probe_ez, unsigned* flags, const TilePlan& pl,
-                cudaStream_t st);
+// defined in fd2d_tile_rec.cu
+int launch_tile_rec(const TileArgs& a, int V, bool lossy, cudaStream_t st);
+// defined in fd2d_tile_rev.cu
+int launch_tile_rev(const TileArgs& a, int V, bool lossy, cudaStream_t st);
 
 // what a strip of a tile has to handle in its steps
 constexpr int kTileInt = 0;    // unit coefficients
@@ -143,13 +146,15 @@ __device__ __forceinline__ bool tile_finite(const float4& v) {
   return isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w);
 }
 
-template <int V, bool LOSSY, bool PML>
+template <int V, bool LOSSY, bool PML, int MODE>
 __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int W = kTileWarps, R = W * V;
   constexpr bool IHXS = tile_ihx_smem(V, PML);
-  constexpr int NARR = tile_arrays(V, LOSSY, PML);
-  constexpr int A_NAZ = 0, A_IHY = 1, A_NBZ = PML ? 2 : 1, A_IZ = A_NBZ + 1, A_IHX = NARR - 1;
+  constexpr int NARR = tile_arrays(V, LOSSY, PML, MODE);
+  constexpr bool REC = MODE == kTileRec, REV = MODE == kTileRev;
+  constexpr int A_NAZ = 0, A_IHY = 1, A_NBZ = PML ? 2 : 1, A_IZ = A_NBZ + 1, A_IHX = A_NBZ + (LOSSY ? 2 : 0),
+                A_G = A_IHX + (IHXS ? 1 : 0), A_GB = A_G + 1;
   extern __shared__ float4 tsm[];
   __shared__ int s_dead;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -244,11 +249,182 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
   const bool masks = i0 <= 0 || i0 + V - 1 >= nx - 1 || __any_sync(kAll, j0 < ny && j0 + 4 > ny);
   const bool unit = __all_sync(kAll, col_ok && row_ok && j0 != 0 && !last_col);
   const int kind = src_here || probe_here ? kTilePoint : masks ? kTileEdge : unit ? kTileInt : kTileGen;
-  xh[w * 32 + lane] = to4(hy[V - 1]);
+  // owned cells of the design box, in whole lanes
+  [[maybe_unused]] const int bc = j0 - a.adj.jb;
+  [[maybe_unused]] const bool box_c = (REC || REV) && own_c && bc >= 0 && bc < a.adj.njp;
+  [[maybe_unused]] auto box_row = [&](int i) {
+    return i >= oi0 && i < oi1 && i >= a.adj.box.i0 && i < a.adj.box.i0 + a.adj.box.ni;
+  };
+  [[maybe_unused]] auto rec_at = [&](int s, int i) {  // dz' - iz of the lane's cells at the s-th step of the run
+    return reinterpret_cast<float4*>(a.adj.rec + ((size_t)s * a.adj.box.ni + (i - a.adj.box.i0)) * a.adj.njp + bc);
+  };
+  if constexpr (REV) {
+#pragma unroll
+    for (int r = 0; r < V; ++r) {
+      const int i = i0 + r;
+      auto grad = [&](const float* g) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (g && box_c && box_row(i))
+          for (int c = 0; c < 4; ++c) {
+            const int bj = j0 + c - a.adj.box.j0;
+            if (bj >= 0 && bj < a.adj.box.nj) v[c] = g[(size_t)(i - a.adj.box.i0) * a.adj.box.nj + bj];
+          }
+        return make_float4(v[0], v[1], v[2], v[3]);
+      };
+      at(A_G, r) = grad(a.adj.grad_naz);
+      if (LOSSY) at(A_GB, r) = grad(a.adj.grad_nbz);
+    }
+    __syncthreads();  // the columns' and rows' coefficients
+  }
+  // how many of the lane's columns of row i have an H update (rows 0 .. nx-2, columns 0 .. ny-2)
+  [[maybe_unused]] auto h_cols = [&](int i) { return i >= 0 && i <= nx - 2 ? ny - 1 - j0 : 0; };
+  [[maybe_unused]] auto first = [&](const F4& v, const F4& o, int n) {  // the first n of v, then o's
+    return F4{make_float2(n <= 0 ? o.a.x : v.a.x, n <= 1 ? o.a.y : v.a.y),
+              make_float2(n <= 2 ? o.b.x : v.b.x, n <= 3 ? o.b.y : v.b.y)};
+  };
+  // REV: the adjoint of cy on strip row r, from the adjoints of hy and ihy
+  [[maybe_unused]] auto lam_cy = [&](int r) {
+    const float4 k = rc[(w * V + r) * 3 + 1];
+    const float2 nfx2 = make_float2(k.z, k.w);
+    const F4 t = fma4(mul4(nfx2, f4(cc[2 * 32 + lane])), hy[r], f4(at(A_IHY, r)));
+    return first(fma4(make_float2(0.5f * k.z, 0.5f * k.w), hy[r], t), F4{}, h_cols(i0 + r));
+  };
+  // the row that the strip below needs: hy, or the adjoint of cy
+  auto publish = [&] {
+    if constexpr (REV) xh[w * 32 + lane] = to4(lam_cy(V - 1));
+    else xh[w * 32 + lane] = to4(hy[V - 1]);
+  };
+  publish();
   __syncthreads();
 
+  // ---- one step undone, step t0-s
+  [[maybe_unused]] auto unstep = [&](auto kind_tag, const int s) {
+    constexpr int KIND = decltype(kind_tag)::value;
+    constexpr bool INT = KIND == kTileInt, MASK = KIND >= kTileEdge, POINT = KIND == kTilePoint;
+    F4 gy2, gy3, fy1, fy2, fy3;
+    if (!INT) {
+      gy2 = f4(cc[0 * 32 + lane]);
+      gy3 = f4(cc[1 * 32 + lane]);
+      fy1 = f4(cc[2 * 32 + lane]);
+      fy2 = f4(cc[3 * 32 + lane]);
+      fy3 = f4(cc[4 * 32 + lane]);
+    }
+    F4 cup = f4(w > 0 ? xh[(w - 1) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f));
+#pragma unroll
+    for (int r = 0; r < V; ++r) {
+      const int i = i0 + r;
+      const bool boxed = box_c && box_row(i);
+      float4 diff = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (boxed) diff = __ldg(rec_at(a.nsteps - 1 - s, i));
+      // adjoints of cx and cy; the H update undone but for the D adjoint's terms
+      F4 cx, cy;
+      if (INT) {
+        cx = fma4(0.5f, hx[r], ihx_get(r));
+        cy = fma4(-0.5f, hy[r], f4(at(A_IHY, r)));
+      } else {
+        const float4 k = rc[(w * V + r) * 3 + 1];
+        const float2 fx3 = *reinterpret_cast<const float2*>(&rc[(w * V + r) * 3 + 2]);
+        const float2 fx1 = make_float2(k.x, k.y), nfx2 = make_float2(k.z, k.w);
+        const F4 ix = ihx_get(r), iy = f4(at(A_IHY, r));
+        F4 nix = fma4(mul4(fx1, fy2), hx[r], ix), niy = fma4(mul4(nfx2, fy1), hy[r], iy);
+        cx = fma4(mul4(0.5f, fy2), hx[r], nix);
+        cy = fma4(make_float2(0.5f * k.z, 0.5f * k.w), hy[r], niy);
+        F4 nhx = mul4(fy3, hx[r]), nhy = mul4(fx3, hy[r]);
+        if (MASK) {
+          const int n = h_cols(i);
+          cx = first(cx, F4{}, n);
+          cy = first(cy, F4{}, n);
+          nix = first(nix, ix, n);
+          niy = first(niy, iy, n);
+          nhx = first(nhx, hx[r], n);
+          nhy = first(nhy, hy[r], n);
+        } else {  // column ny-1, the last of its lane
+          cx.b.y = last_col ? 0.f : cx.b.y;
+          cy.b.y = last_col ? 0.f : cy.b.y;
+          nix.b.y = last_col ? ix.b.y : nix.b.y;
+          niy.b.y = last_col ? iy.b.y : niy.b.y;
+          nhx.b.y = last_col ? hx[r].b.y : nhx.b.y;
+          nhy.b.y = last_col ? hy[r].b.y : nhy.b.y;
+        }
+        ihx_set(r, nix);
+        at(A_IHY, r) = to4(niy);
+        hx[r] = nhx;
+        hy[r] = nhy;
+      }
+      // adjoint of ez, then the E update undone
+      float cl = __shfl_up_sync(kAll, cx.b.y, 1);
+      cl = lane == 0 ? 0.f : cl;  // column 0, or a halo's edge
+      F4 lez = {make_float2(__fsub_rn(cx.a.x, cl), __fsub_rn(cx.a.y, cx.a.x)),
+                make_float2(__fsub_rn(cx.b.x, cx.a.y), __fsub_rn(cx.b.y, cx.b.x))};
+      lez = sub4(add4(lez, cy), cup);
+      cup = cy;
+      if (POINT && probe_here && i == a.probe_i) {
+        const float e = __ldg(a.probe_ez + a.t0 - 1 - s);
+        auto seed = [&](float& x, int j) {
+          if (j == a.probe_j) x = __fmaf_rn(a.adj.probe_w, e, x);
+        };
+        seed(lez.a.x, j0);
+        seed(lez.a.y, j0 + 1);
+        seed(lez.b.x, j0 + 2);
+        seed(lez.b.y, j0 + 3);
+      }
+      const F4 na = f4(at(A_NAZ, r));
+      if (LOSSY) {
+        const F4 liz = f4(at(A_IZ, r));
+        lez = fma4(f4(at(A_NBZ, r)), liz, lez);
+        const F4 nna = {make_float2(-na.a.x, -na.a.y), make_float2(-na.b.x, -na.b.y)};
+        at(A_IZ, r) = to4(fma4(nna, lez, liz));
+        if (boxed) at(A_GB, r) = to4(fma4(liz, mul4(na, f4(diff)), f4(at(A_GB, r))));
+      }
+      if (boxed) at(A_G, r) = to4(fma4(lez, f4(diff), f4(at(A_G, r))));
+      const F4 T = fma4(na, lez, dz[r]);
+      // the D update undone; dg is the adjoint of its curl, ndg = -dg (the sums below as in sub4's comment)
+      F4 dg, ndg;
+      if (INT) {
+        dz[r] = T;
+        dg = mul4(0.5f, T);
+        ndg = mul4(-0.5f, T);
+      } else {
+        const float4 k = rc[(w * V + r) * 3];
+        F4 nd = mul4(mul4(make_float2(k.z, k.w), gy3), T);
+        dg = mul4(mul4(make_float2(k.x, k.y), gy2), T);
+        ndg = mul4(mul4(make_float2(-k.x, -k.y), gy2), T);
+        if (j0 == 0) {  // column 0 has no D update
+          nd.a.x = T.a.x;
+          dg.a.x = ndg.a.x = 0.f;
+        }
+        if (MASK && i < 1) {  // nor has row 0
+          nd = T;
+          dg = ndg = F4{};
+        }
+        if (POINT && src_here && a.src_kind == FDTD_SRC_HARD && i == a.src_i) {
+          auto cut = [&](float& x, float& y, float& z, int j) {
+            if (j == a.src_j) x = y = z = 0.f;
+          };
+          cut(nd.a.x, dg.a.x, ndg.a.x, j0);
+          cut(nd.a.y, dg.a.y, ndg.a.y, j0 + 1);
+          cut(nd.b.x, dg.b.x, ndg.b.x, j0 + 2);
+          cut(nd.b.y, dg.b.y, ndg.b.y, j0 + 3);
+        }
+        dz[r] = nd;
+      }
+      float nr = __shfl_down_sync(kAll, ndg.a.x, 1);
+      nr = lane == 31 ? 0.f : nr;
+      const F4 nj = {make_float2(ndg.a.y, ndg.b.x), make_float2(ndg.b.y, nr)};
+      hx[r] = sub4(sub4(hx[r], dg), nj);
+      hy[r] = sub4(hy[r], ndg);
+      if (r == 0) xe[w * 32 + lane] = to4(dg);
+      else hy[r - 1] = sub4(hy[r - 1], dg);
+    }
+    __syncthreads();
+    hy[V - 1] = sub4(hy[V - 1], f4(w < W - 1 ? xe[(w + 1) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f)));
+    if (INT) xh[w * 32 + lane] = to4(fma4(-0.5f, hy[V - 1], f4(at(A_IHY, V - 1))));
+    else publish();
+    __syncthreads();
+  };
+
   // ---- one time step, t0+s+1; LAST stores ez
-  auto step = [&](auto kind_tag, const int s, const bool last) {
+  [[maybe_unused]] auto step = [&](auto kind_tag, const int s, const bool last) {
     constexpr int KIND = decltype(kind_tag)::value;
     constexpr bool INT = KIND == kTileInt, MASK = KIND >= kTileEdge, POINT = KIND == kTilePoint;
     // the columns' coefficients for this step (read per row they bound it: shared memory)
@@ -370,9 +546,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
       const F4 na = f4(at(A_NAZ, r));
       if (LOSSY) {
         const F4 iz = f4(at(A_IZ, r));
-        e = mul4(na, sub4(dz[r], iz));
+        const F4 diff = sub4(dz[r], iz);
+        if (REC && box_c && box_row(i)) __stcg(rec_at(s, i), to4(diff));
+        e = mul4(na, diff);
         at(A_IZ, r) = to4(fma4(f4(at(A_NBZ, r)), e, iz));
       } else {
+        if (REC && box_c && box_row(i)) __stcg(rec_at(s, i), to4(dz[r]));
         e = mul4(na, dz[r]);
       }
       if (POINT && probe_here && i == a.probe_i && own_c && i >= oi0 && i < oi1) {
@@ -478,7 +657,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
           if (LOSSY) at(A_IZ, r) = tile_ld(x.iz, row, j0, ny, false);
         }
     }
-    xh[w * 32 + lane] = to4(hy[V - 1]);
+    publish();
     __syncthreads();
   };
 
@@ -489,7 +668,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
   for (int s = 0, e = 0; s < a.nsteps;) {
     const int m = min(T, a.nsteps - s);
     auto run = [&](auto kind_tag) {
-      for (int q = 0; q < m; ++q) step(kind_tag, s + q, s + q + 1 == a.nsteps);
+      for (int q = 0; q < m; ++q) {
+        if constexpr (REV) unstep(kind_tag, s + q);
+        else step(kind_tag, s + q, s + q + 1 == a.nsteps);
+      }
     };
     if (kind == kTileInt) run(std::integral_constant<int, kTileInt>{});
     else if (kind == kTileGen) run(std::integral_constant<int, kTileGen>{});
@@ -527,8 +709,46 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
       }
       if (LOSSY) st(a.out.iz, at(A_IZ, r));
     }
+    if constexpr (REV) {
+      auto put = [&](float* g, const float4& v4) {
+        const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+        if (g && box_c && box_row(i))
+          for (int c = 0; c < 4; ++c) {
+            const int bj = j0 + c - a.adj.box.j0;
+            if (bj >= 0 && bj < a.adj.box.nj) g[(size_t)(i - a.adj.box.i0) * a.adj.box.nj + bj] = v[c];
+          }
+      };
+      put(a.adj.grad_naz, at(A_G, r));
+      if (LOSSY) put(a.adj.grad_nbz, at(A_GB, r));
+    }
   }
   if (a.status && !fin) raise_status(a.status, ST_NONFINITE);
+}
+
+template <int V, bool LOSSY, bool PML, int MODE>
+int launch_t(const TileArgs& a, cudaStream_t st) {
+  auto kern = k_tile<V, LOSSY, PML, MODE>;
+  const size_t smem = tile_smem_bytes(V, LOSSY, PML, MODE);
+  cudaError_t e = cudaSuccess;
+  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.n_ti * a.n_tj, 1, 1);
+    cfg.blockDim = dim3(kTileWarps * 32, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;  // all blocks resident: they wait on one another
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, a);
+  }
+  if (e != cudaSuccess) {
+    fdtd_host::note_cuda_error(e);
+    return FDTD_ERR_CUDA;
+  }
+  return fdtd_host::check_launch();
 }
 
 }  // namespace

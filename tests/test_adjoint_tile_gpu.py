@@ -1,0 +1,55 @@
+"""The adjoint on the chip (checkpoint intervals of 4 and more where the tiles
+fit the SMs) against the streaming kernels (interval 3), bitwise: boxes off the
+groups of four and over tile borders, with and without loss, both gradients,
+partial last segments, hard and soft sources, probes inside the box."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(nx, ny, npml, lossy, box, src, probe, kind, ns, cp):
+    from simulation_gb300 import _lib
+    from simulation_gb300 import fd2d as G
+    s = G.SimTM2D(nx, ny, pml=G.pmlparam(nx, ny, npml), lossy=lossy,
+                  source=G.PointSource(*src, ("gauss", 12, 4.0), kind), ns=ns)
+    g = torch.Generator().manual_seed(nx)
+    i0, j0, ni, nj = box
+    s.naz.fill_(1.0)
+    s.naz[i0:i0 + ni, j0:j0 + nj] = 1.0 / (1.0 + 3.0 * torch.rand((ni, nj), generator=g)).cuda()
+    if lossy:
+        s.nbz.zero_()
+        s.nbz[i0:i0 + ni, j0:j0 + nj] = 0.02 * torch.rand((ni, nj), generator=g).cuda()
+    ap = _lib.AdjointParams2D(ns, cp, probe[0], probe[1], 2.0, _lib.Box2D(*box))
+    n = _lib.lib().fdtd2d_tm_adjoint_workspace_size(C.byref(s._p), C.byref(ap))
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    trace = torch.zeros(ns, device="cuda")
+    J = torch.zeros(1, dtype=torch.float64, device="cuda")
+    gn = torch.full((ni, nj), 7.0, device="cuda")
+    gb = torch.full((ni, nj), 7.0, device="cuda") if lossy else None
+    _lib.call("fdtd2d_tm_adjoint", C.byref(s._p), C.byref(ap), trace.data_ptr(), J.data_ptr(), gn.data_ptr(),
+              None if gb is None else gb.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream_ptr())
+    torch.cuda.synchronize()
+    return trace, J, gn, gb
+
+
+@pytest.mark.parametrize("nx,ny,box,src,probe", [
+    (40, 40, (10, 9, 18, 21), (12, 20), (30, 20)),          # one tile; the source and the probe in the box
+    (100, 128, (30, 40, 40, 50), (25, 64), (65, 64)),
+    (130, 260, (1, 1, 128, 258), (40, 130), (80, 131)),     # almost the whole grid
+    (300, 516, (60, 113, 170, 301), (50, 258), (90, 259)),
+    (700, 512, (300, 250, 99, 3), (290, 256), (330, 255)),
+    (1024, 1024, (384, 384, 256, 256), (344, 512), (390, 512)),
+])
+@pytest.mark.parametrize("lossy", [False, True])
+@pytest.mark.parametrize("kind", ["hard", "soft"])
+def test_against_streaming(cuda_lib, nx, ny, box, src, probe, lossy, kind):
+    a = _run(nx, ny, 8, lossy, box, src, probe, kind, 151, 32)  # segments of 32, 32, 32, 32, 23
+    b = _run(nx, ny, 8, lossy, box, src, probe, kind, 151, 3)
+    c = _run(nx, ny, 8, lossy, box, src, probe, kind, 151, 50)  # the last of one step
+    assert float(b[1]) > 0 and float(b[2].abs().max()) > 0
+    for x in (a, c):
+        for p, q in zip(x, b):
+            assert (p is None and q is None) or torch.equal(p, q)
