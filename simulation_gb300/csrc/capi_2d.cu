@@ -120,6 +120,16 @@ bool pad_ok(const fdtd2d_params* p, int steps_per_pass) {
   return p->ny % 4 != 0 && !ext_on(p) && steps_per_pass == 0 && chain_better(p->nx, p->ny) && p->nx <= 8 * 65535;
 }
 
+// Chained passes with the plane wave and the running DFT: the march's workspace
+// and, with the DFT on, room for the ez of kExtRecSteps steps.
+constexpr int kExtRecSteps = 16;
+bool chain_ext_ok(const fdtd2d_params* p, int steps_per_pass) {
+  return ext_on(p) && steps_per_pass == 0 && fused_params_ok(p) && chain_ext_better(p->nx, p->ny);
+}
+size_t chain_ext_workspace_bytes(const fdtd2d_params* p) {
+  return fused_workspace_bytes(p) + (p->nf > 0 ? kExtRecSteps * slot_bytes(p) : 0);
+}
+
 FieldSet workspace_set(const fdtd2d_params* p, void* workspace, size_t sb) {
   FieldSet ws{};
   char* base = (char*)workspace;
@@ -253,6 +263,7 @@ size_t fdtd2d_fast_workspace_size(const fdtd2d_params* p, int steps_per_pass) {
   if (!p || p->nx < 3 || p->ny < 3) return 0;
   TilePlan pl;
   if (tile_ok(p, steps_per_pass, pl)) return std::max(need, tile_workspace_bytes(p));
+  if (chain_ext_ok(p, steps_per_pass)) return chain_ext_workspace_bytes(p);
   return pad_ok(p, steps_per_pass) ? pad_workspace_bytes(p) : need;
 }
 
@@ -293,7 +304,8 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
   // pass schedule with an even number of passes, so the last pass writes the
   // caller's arrays (split one pass if needed).  Left to the library, large
   // grids take chained passes of 8 and 4 steps (fd2d_chain.cuh)
-  const bool chain = steps_per_pass == 0 && !ext_on(p) && !s->probe_ez && chain_better(p->nx, p->ny);
+  const bool chain = ext_on(p) ? chain_ext_ok(p, steps_per_pass) && workspace_bytes >= chain_ext_workspace_bytes(p)
+                               : steps_per_pass == 0 && !s->probe_ez && chain_better(p->nx, p->ny);
   const int K = steps_per_pass == 0 ? march_default_steps(p->nx, p->ny) : steps_per_pass;
   std::vector<int> sched;
   for (int rem = nsteps; rem > 0;) {
@@ -341,6 +353,16 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
   }
   int t = t0;
   int line_t0 = t0, line_n = 0;  // steps the incident-line tables hold
+  int rec_n = 0;                 // steps whose ez is recorded and not yet in the DFT
+  float* ez_rec = (float*)((char*)workspace + fused_workspace_bytes(p));
+  const size_t rec_slot = slot_bytes(p) / sizeof(float);
+  auto flush = [&]() -> int {
+    const int n = rec_n;
+    rec_n = 0;
+    if (n == 0) return FDTD_OK;
+    return launch_dft_rec((size_t)p->nx * p->ny, t - n, n, p->nf, p->dft_cos, p->dft_sin, ez_rec, rec_slot, s->r_pt,
+                          s->i_pt, st);
+  };
   for (size_t i = 0; i < sched.size(); ++i) {
     const FieldSet& in = (i % 2 == 0) ? user : ws;
     const FieldSet& out = (i % 2 == 0) ? ws : user;
@@ -351,7 +373,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
     int* status = (i + 1 == sched.size()) ? s->status : nullptr;
     // ez is a result of the call, not an input of the passes: only the last stores it
     float* ez = (i + 1 == sched.size()) ? s->ez : nullptr;
-    if (chain && (sched[i] == 8 || sched[i] == 4)) {
+    if (chain && !ext_on(p) && (sched[i] == 8 || sched[i] == 4)) {
       rc = launch_chain(*p, p->ny, p->naz, p->nbz, in, out, ez, t, sched[i], status, march_gen_cost(), st);
     } else if (!ext_on(p)) {
       rc = launch_march(*p, in, out, ez, t, sched[i], status, s->probe_ez, st);
@@ -367,11 +389,20 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
         ext.inc_e = inc_e + (size_t)(t - line_t0) * p->ny;
         ext.inc_h = inc_h + (size_t)(t - line_t0) * 2;
       }
-      rc = launch_march_ext(*p, in, out, ez, t, sched[i], status, ext, st);
+      const bool chained = chain && (sched[i] == 8 || sched[i] == 4);
+      if ((!chained || rec_n + sched[i] > kExtRecSteps) && (rc = flush())) return rc;
+      if (chained) {
+        rc = launch_chain_ext(*p, in, out, ez, t, sched[i], status, march_gen_cost(), ext, ez_rec + rec_n * rec_slot,
+                              rec_slot, st);
+        if (p->nf > 0) rec_n += sched[i];
+      } else {
+        rc = launch_march_ext(*p, in, out, ez, t, sched[i], status, ext, st);
+      }
     }
     if (rc) return rc;
     t += sched[i];
   }
+  if ((rc = flush())) return rc;
   if (copy_back) {
     const size_t b = (size_t)p->nx * p->ny * sizeof(float);
     float* pairs[6][2] = {{user.dz, ws.dz}, {user.hx, ws.hx}, {user.hy, ws.hy},

@@ -66,6 +66,12 @@ struct ChainArgs {
   // blocks 0 .. n_gen*n_segs_g-1: the general stripes at either edge, in shorter
   // segments; then the other stripes
   int n_stripes, n_gen_lo, n_gen_hi, n_segs, seg_first, seg_rows, n_segs_g, seg_rows_g;
+  // the EXT builds' plane wave and record of ez
+  int np;              // TF/SF box, 0: none
+  const float* inc_e;  // as in MarchExt
+  const float* inc_h;
+  float* ez_rec;       // ez of each of the pass's steps, for the running DFT; null: not wanted
+  size_t rec_slot;     // floats from one step's to the next
 };
 
 // floats of a block's shared memory: an input ring and a hand-over ring per
@@ -136,6 +142,11 @@ inline long chain_layout(ChainArgs& a, int K, long blocks, int P, float gen_cost
 // one pass of k steps, 4 or 8, over arrays of `pitch` columns a row (fd2d_chain.cu)
 int launch_chain(const fdtd2d_params& p, int pitch, const float* naz, const float* nbz, const FieldSet& in,
                  const FieldSet& out, float* ez, int t0, int k, int* status, float gen_cost, cudaStream_t st);
+// the same with the plane wave and the running DFT of `ext` (fd2d_chain_ext.cu); ez_rec: room for
+// the ez of k steps, rec_slot floats each (nf > 0)
+int launch_chain_ext(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int k,
+                     int* status, float gen_cost, const MarchExt& ext, float* ez_rec, size_t rec_slot,
+                     cudaStream_t st);
 
 namespace {
 
@@ -153,7 +164,8 @@ struct ChainRow {
   F4 dz, iz, hx, hy, ihx, ihy, ez;
 };
 
-template <int LV, int NC, bool LOSSY, bool PML>
+// EXT: the TF/SF box's corrections and the record of ez
+template <int LV, int NC, bool LOSSY, bool PML, bool EXT>
 __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ ChainArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int W = kChainCols, RF = chain_rf(LV), K = LV * NC, HB = chain_halo(LV, NC);
@@ -194,6 +206,17 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
 #pragma unroll
       for (int k = 0; k < 5; ++k) chain_sts(cc + k * W, f4(make_float4(v[k][0], v[k][1], v[k][2], v[k][3])));
   }
+  // TF/SF: the box's edge columns (D at np-1 and ny-np, hx at np-2 and ny-np)
+  // make a stripe general; its edge rows np-2 and nx-np (hy) are general in
+  // every stripe
+  const int np = EXT ? a.np : 0;
+  bool edge = false;  // any of the warp's columns is an edge column
+  if (EXT && np > 0) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) edge |= j0 + c == np - 2 || j0 + c == np - 1 || j0 + c == ny - np;
+    col_ok &= !edge;
+    edge = __any_sync(kAll, edge);
+  }
   const bool cint = __all_sync(kAll, col_ok);
   const bool src_here = a.src_kind != FDTD_SRC_NONE && a.src_j >= j0 - lane * 4 && a.src_j < j0 - lane * 4 + W;
   const bool col0 = j0 == 0;
@@ -207,6 +230,7 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
       g = __ldg(a.pml.gx2 + row) == 1.f && __ldg(a.pml.gx3 + row) == 1.f && __ldg(a.pml.fx1 + row) == 0.f &&
           __ldg(a.pml.fx2 + row) == 1.f && __ldg(a.pml.fx3 + row) == 1.f;
     if (src_here && row == a.src_i) g = false;
+    if (EXT && np > 0 && (row == np - 2 || row == nx - np)) g = false;
     return __ballot_sync(kAll, g);
   };
 
@@ -311,6 +335,19 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
           put(q.dz.b.y, j0 + 3);
         }
       }
+      if constexpr (EXT && !INT) {
+        if (edge && row >= np - 1 && row <= nx - np) {
+          const float lo = __ldg(a.inc_h + 2 * (LV * cw + s)), hi = __ldg(a.inc_h + 2 * (LV * cw + s) + 1);
+          auto put = [&](float& x, int j) {
+            if (j == np - 1) x = __fmaf_rn(0.5f, lo, x);
+            if (j == ny - np) x = __fmaf_rn(-0.5f, hi, x);
+          };
+          put(q.dz.a.x, j0);
+          put(q.dz.a.y, j0 + 1);
+          put(q.dz.b.x, j0 + 2);
+          put(q.dz.b.y, j0 + 3);
+        }
+      }
       const int mi = ms + I - s;
       const float* const m = mring + (mi >= MT ? mi - MT : mi) * NM * W;
       const F4 na = chain_lds(m);
@@ -319,6 +356,12 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
         q.iz = fma4(chain_lds(m + W), q.ez, q.iz);
       } else {
         q.ez = mul4(na, q.dz);
+      }
+      if constexpr (EXT) {
+        if (a.ez_rec && vout && row >= i_s && row < i_e)
+          __stcs(reinterpret_cast<float4*>(a.ez_rec + (LV * cw + s) * a.rec_slot + ((unsigned)row * (unsigned)pitch +
+                                                                                   (unsigned)j0)),
+                 to4(q.ez));
       }
       // H on row r-s-1
       const float er = __shfl_down_sync(kAll, p.ez.a.x, 1);
@@ -350,6 +393,32 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
         } else {
           nhx = fma4(0.5f, cx, p.hx);
           nhy = fma4(-0.5f, cy, p.hy);
+        }
+        if constexpr (EXT) {
+          if (np > 0) {
+            const float* er0 = a.inc_e + (size_t)(LV * cw + s) * ny;
+            if (edge && pr >= np - 1 && pr <= nx - np) {
+              const float lo = __ldg(er0 + np - 1), hi = __ldg(er0 + ny - np);
+              auto put = [&](float& x, int j) {
+                if (j == np - 2) x = __fmaf_rn(0.5f, lo, x);
+                if (j == ny - np) x = __fmaf_rn(-0.5f, hi, x);
+              };
+              put(nhx.a.x, j0);
+              put(nhx.a.y, j0 + 1);
+              put(nhx.b.x, j0 + 2);
+              put(nhx.b.y, j0 + 3);
+            }
+            if ((pr == np - 2 || pr == nx - np) && vin) {
+              const float wy = pr == np - 2 ? -0.5f : 0.5f;
+              auto put = [&](float& x, int j) {
+                if (j >= np - 1 && j <= ny - np) x = __fmaf_rn(wy, __ldg(er0 + j), x);
+              };
+              put(nhy.a.x, j0);
+              put(nhy.a.y, j0 + 1);
+              put(nhy.b.x, j0 + 2);
+              put(nhy.b.y, j0 + 3);
+            }
+          }
         }
         // row nx-1 and column ny-1 are not updated
         const int n = in ? h_cols : 0;
@@ -431,6 +500,50 @@ __global__ void __launch_bounds__(32 * NC) k_chain(const __grid_constant__ Chain
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (a.status && __any_sync(kAll, !fin) && lane == 0) raise_status(a.status, ST_NONFINITE);
+}
+
+inline ChainArgs chain_args(const fdtd2d_params& p, int pitch, const float* naz, const float* nbz, const FieldSet& in,
+                            const FieldSet& out, float* ez, int t0, int* status) {
+  ChainArgs a{};
+  a.nx = p.nx;
+  a.ny = p.ny;
+  a.pitch = pitch;
+  a.in = in;
+  a.out = out;
+  a.ez = ez;
+  a.naz = naz;
+  a.nbz = nbz;
+  a.pml = p.pml;
+  a.src_kind = p.src.kind;
+  a.src_i = p.src.i;
+  a.src_j = p.src.j;
+  a.src_table = p.src.table;
+  a.t0 = t0;
+  a.status = status;
+  return a;
+}
+
+// waves: blocks launched over those resident.  One wave ends with its slowest
+// block (SMs idle for 16% of a 2 x 4 pass at 6144^2); four short ones, the
+// general stripes first, balance themselves, at the price of more recomputed
+// rows: 8192^2 lossy with layer 580 -> 717 Gcell-updates/s, but 4096^2 521 -> 451.
+template <int LV, int NC, bool LOSSY, bool PML, bool EXT>
+int launch_t(ChainArgs a, int pml_cells, double waves, float gen_cost, cudaStream_t st) {
+  auto kern = k_chain<LV, NC, LOSSY, PML, EXT>;
+  const size_t smem = chain_smem_bytes(LV, NC, LOSSY, PML);
+  int dev = 0, nsm = 0, per_sm = 0;
+  cudaError_t e = cudaSuccess;
+  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * NC, smem);
+  if (e != cudaSuccess) {
+    fdtd_host::note_cuda_error(e);
+    return FDTD_ERR_CUDA;
+  }
+  const long blocks = chain_layout(a, LV * NC, (long)(nsm * std::max(per_sm, 1) * waves), pml_cells, gen_cost);
+  kern<<<(unsigned)blocks, 32 * NC, smem, st>>>(a);
+  return fdtd_host::check_launch();
 }
 
 }  // namespace

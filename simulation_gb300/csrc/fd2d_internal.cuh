@@ -50,6 +50,7 @@ float march_gen_cost();
 // whether large-grid passes go through the chained kernel (fd2d_chain.cuh):
 // grids that do not fit on the chip, without a caller's own march shape
 bool chain_better(int nx, int ny);
+bool chain_ext_better(int nx, int ny);  // with the plane wave or the running DFT
 // A pass that also records the state after each of its steps (the adjoint's
 // recompute): rec[s] receives dz, iz, hx, hy after step t0+s+1, s < k.
 // Point source only, with PML (plain kernels, 64-column stripes).
@@ -77,6 +78,9 @@ constexpr int kLineChunkSteps = 64;    // incident-line steps per table
 bool march_ext_supported(const fdtd2d_params& p);
 int launch_march_ext(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int k,
                      int* status, const MarchExt& ext, cudaStream_t st);
+// adds `steps` recorded ez (step t0+s+1 at ez + s*slot) to the accumulators (fd2d_dft_rec.cu)
+int launch_dft_rec(size_t ncell, int t0, int steps, int nf, const float* dft_cos, const float* dft_sin, const float* ez,
+                   size_t slot, float* r_pt, float* i_pt, cudaStream_t st);
 // Advance the incident line (ezinct, hxinct, the input-probe DFT) by nsteps
 // steps t0+1 .. t0+nsteps and record what the 2D update reads of it
 // (fd2d_simple.cu holds the per-step kernels it must equal bit for bit).

@@ -55,6 +55,14 @@ bool chain_better(int nx, int ny) {
   return (long long)nx * ny >= (1LL << 20) && (long long)nx * ny < (1LL << 31) && nx >= 64 && ny >= 128;
 }
 
+// (96 steps with plane wave and 3 frequencies, chain against the better march:
+// 128^2 875 us / 1050, 512^2 903 / 1145, 1024^2 1111 / 1495, 2048^2 2048 / 3458,
+// 4096^2 6456 / 11000)
+bool chain_ext_better(int nx, int ny) {
+  if (g_cfg.cpl || g_cfg.seg_rows) return false;
+  return (long long)nx * ny >= (1LL << 14) && (long long)nx * ny < (1LL << 31) && nx >= 64 && ny >= 128;
+}
+
 namespace {
 MarchArgs march_args(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0,
                      int* status, float* probe_ez) {

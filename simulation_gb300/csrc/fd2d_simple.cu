@@ -104,7 +104,10 @@ __global__ void k_ezinct(int ny, float* __restrict__ ezi, const float* __restric
 // k_step_d), the ezi[6] input-probe DFT of k_step_e and k_hxinct, so the
 // line equals the per-step kernels bit for bit.  Per step s it records what
 // the 2D update reads: inc_e[s][:] = ezi after the E update and source, and
-// inc_h[s] = hxi[npml-2], hxi[ny-npml] before the H update.
+// inc_h[s] = hxi[npml-2], hxi[ny-npml] before the H update.  Bound by its two
+// barriers a step, the tables' values read a step ahead (a third barrier around
+// thread 0's work on the ends, with a global read in it, made 1.1 us a step at
+// ny = 2048 of what is now 0.95).
 __global__ void k_inc_line(int ny, int npml, int t0, int nsteps, float* __restrict__ ezi, float* __restrict__ hxi,
                            float* __restrict__ bc, const float* __restrict__ tfsf_table, int nf,
                            const float* __restrict__ dft_cos, const float* __restrict__ dft_sin,
@@ -113,43 +116,60 @@ __global__ void k_inc_line(int ny, int npml, int t0, int nsteps, float* __restri
   extern __shared__ float line[];
   float* e = line;
   float* h = line + ny;
-  __shared__ float sbc[4];
+  __shared__ float sbc[2][4];  // the boundary's history before even and odd steps
   const int tid = threadIdx.x, nth = blockDim.x;
   for (int j = tid; j < ny; j += nth) {
     e[j] = ezi[j];
     h[j] = hxi[j];
   }
-  if (tid < 4) sbc[tid] = bc[tid];
-  float rin = 0.f, iin = 0.f;
+  if (tid < 4) sbc[0][tid] = bc[tid];
+  float rin = 0.f, iin = 0.f, src = 0.f, wc = 0.f, ws = 0.f;
   if (tid < nf) {
     rin = r_in[tid];
     iin = i_in[tid];
   }
+  // the tables' values of the step to come, read a step ahead
+  auto prefetch = [&](int t) {
+    if (tid == 3) src = tfsf_table[t - 1];
+    if (tid < nf) {
+      wc = dft_cos[(size_t)(t - 1) * nf + tid];
+      ws = dft_sin[(size_t)(t - 1) * nf + tid];
+    }
+  };
+  prefetch(t0 + 1);
   __syncthreads();
   for (int s = 0; s < nsteps; ++s) {
-    const int t = t0 + s + 1;
+    const float* ob = sbc[s & 1];
+    float* nb = sbc[(s + 1) & 1];
+    float* row = inc_e + (size_t)s * ny;
     if (tid == 0) {
       inc_h[2 * s] = h[npml - 2];
       inc_h[2 * s + 1] = h[ny - npml];
     }
-    for (int j = 1 + tid; j < ny; j += nth) e[j] = __fmaf_rn(0.5f, __fsub_rn(h[j - 1], h[j]), e[j]);
-    __syncthreads();
-    if (tid == 0) {
-      e[0] = sbc[0];
-      sbc[0] = sbc[1];
-      sbc[1] = e[1];
-      e[ny - 1] = sbc[3];
-      sbc[3] = sbc[2];
-      sbc[2] = e[ny - 2];
-      e[3] = tfsf_table[t - 1];
+    // E, the absorbing ends (each keeps its neighbour's last two values) and the source at 3
+    for (int j = tid; j < ny; j += nth) {
+      float v;
+      if (j == 0) {
+        v = ob[0];
+        nb[0] = ob[1];
+      } else if (j == ny - 1) {
+        v = ob[3];
+        nb[3] = ob[2];
+      } else {
+        v = __fmaf_rn(0.5f, __fsub_rn(h[j - 1], h[j]), e[j]);
+        if (j == 1) nb[1] = v;
+        if (j == ny - 2) nb[2] = v;
+        if (j == 3) v = src;
+      }
+      e[j] = v;
+      row[j] = v;
     }
+    const float c = wc, d = ws;
+    if (s + 1 < nsteps) prefetch(t0 + s + 2);
     __syncthreads();
-    float* row = inc_e + (size_t)s * ny;
-    for (int j = tid; j < ny; j += nth) row[j] = e[j];
     if (tid < nf) {
-      const size_t k = (size_t)(t - 1) * nf + tid;
-      rin = __fmaf_rn(dft_cos[k], e[6], rin);
-      iin = __fmaf_rn(-dft_sin[k], e[6], iin);
+      rin = __fmaf_rn(c, e[6], rin);
+      iin = __fmaf_rn(-d, e[6], iin);
     }
     for (int j = tid; j < ny - 1; j += nth) h[j] = __fmaf_rn(0.5f, __fsub_rn(e[j], e[j + 1]), h[j]);
     __syncthreads();
@@ -158,7 +178,7 @@ __global__ void k_inc_line(int ny, int npml, int t0, int nsteps, float* __restri
     ezi[j] = e[j];
     hxi[j] = h[j];
   }
-  if (tid < 4) bc[tid] = sbc[tid];
+  if (tid < 4) bc[tid] = sbc[nsteps & 1][tid];
   if (tid < nf) {
     r_in[tid] = rin;
     i_in[tid] = iin;
