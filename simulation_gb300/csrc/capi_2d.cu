@@ -93,8 +93,10 @@ size_t fused_workspace_bytes(const fdtd2d_params* p) { return slot_bytes(p) * ns
 // SMs, with the library's choice of steps per pass.  Its workspace: one
 // exchange set of the evolving fields (as the march's ping-pong set) and the
 // blocks' flags.
+// With plane wave or running DFT: also the incident line's tables and, with the
+// DFT, room for the ez of a launch's steps.
 bool tile_ok(const fdtd2d_params* p, int steps_per_pass, TilePlan& pl) {
-  if (ext_on(p) || steps_per_pass != 0) return false;
+  if (steps_per_pass != 0 || (p->tfsf_npml > 0 && p->ny > kLineMaxNy)) return false;
   int dev = 0, nsm = 0, coop = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -104,7 +106,17 @@ bool tile_ok(const fdtd2d_params* p, int steps_per_pass, TilePlan& pl) {
   }
   return tile_plan(p->nx, p->ny, p->nbz != nullptr, has_pml(*p), std::min(nsm, kTileMaxBlocks), pl);
 }
-size_t tile_workspace_bytes(const fdtd2d_params* p) { return slot_bytes(p) * nslots(p) + kTileFlagBytes; }
+// steps of a launch with the extras: the line's tables hold 64; with the DFT the
+// record of ez stays within 96 MB, in L2 until the DFT reads it, but is not below
+// 16 steps (a launch loads and stores the tiles: 15 us at 1024^2)
+int tile_ext_steps(const fdtd2d_params* p) {
+  if (p->nf <= 0) return kLineChunkSteps;
+  return std::min(kLineChunkSteps, std::max(16, (int)((96 << 20) / slot_bytes(p))));
+}
+size_t tile_workspace_bytes(const fdtd2d_params* p) {
+  const size_t b = slot_bytes(p) * nslots(p) + round256(kTileFlagBytes);
+  return ext_on(p) ? b + line_bytes(p) + (p->nf > 0 ? tile_ext_steps(p) * slot_bytes(p) : 0) : b;
+}
 
 // Chained passes over padded copies, for grids whose rows are no multiple of 16
 // bytes (they would otherwise go three launches a step): two ping-pong sets,
@@ -174,6 +186,37 @@ int step_padded(const fdtd2d_params* p, const fdtd2d_state* s, int t0, int nstep
     t += k;
   }
   return launch_unpad(set[cur], user, ez, s->ez, p->nx, p->ny, pitch, st);
+}
+
+// the on-chip loop with plane wave or running DFT, a launch of up to
+// tile_ext_steps steps at a time
+int step_tile_ext(const fdtd2d_params* p, const fdtd2d_state* s, int t0, int nsteps, void* workspace, unsigned* flags,
+                  const TilePlan& tile, cudaStream_t st) {
+  const FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy}, x0 = workspace_set(p, workspace, slot_bytes(p));
+  char* rest = (char*)flags + round256(kTileFlagBytes);
+  float* inc_e = (float*)rest;
+  float* inc_h = (float*)(rest + (p->tfsf_npml > 0 ? line_e_bytes(p) : 0));
+  TileExt ext;
+  ext.np = p->tfsf_npml;
+  ext.inc_e = inc_e;
+  ext.inc_h = inc_h;
+  ext.ez_rec = p->nf > 0 ? (float*)(rest + line_bytes(p)) : nullptr;
+  ext.rec_slot = slot_bytes(p) / sizeof(float);
+  const int most = tile_ext_steps(p);
+  for (int t = t0; t < t0 + nsteps;) {
+    const int n = std::min(most, t0 + nsteps - t);
+    int rc;
+    if (p->tfsf_npml > 0 && (rc = launch_inc_line(*p, *s, t, n, inc_e, inc_h, st))) return rc;
+    const bool last = t + n == t0 + nsteps;
+    if ((rc = launch_tile(*p, user, user, x0, user, last ? s->ez : nullptr, t, n, last ? s->status : nullptr,
+                          s->probe_ez, flags, tile, st, kTileExt, nullptr, &ext)))
+      return rc;
+    if (p->nf > 0 && (rc = launch_dft_rec((size_t)p->nx * p->ny, t, n, p->nf, p->dft_cos, p->dft_sin, ext.ez_rec,
+                                          ext.rec_slot, s->r_pt, s->i_pt, st)))
+      return rc;
+    t += n;
+  }
+  return FDTD_OK;
 }
 
 // one time step in the reference's order (fd2d/python/fd2d_3_4.py:268-277):
@@ -282,6 +325,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
       tile_ok(p, steps_per_pass, tile)) {
     const FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
     unsigned* flags = (unsigned*)((char*)workspace + slot_bytes(p) * nslots(p));
+    if (ext_on(p)) return step_tile_ext(p, s, t0, nsteps, workspace, flags, tile, st);
     return launch_tile(*p, user, user, workspace_set(p, workspace, slot_bytes(p)), user, s->ez, t0, nsteps, s->status, s->probe_ez,
                        flags, tile, st);
   }

@@ -51,7 +51,7 @@ bool al16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, const FieldSet& x0, const FieldSet& x1,
                 float* ez, int t0, int nsteps, int* status, float* probe_ez, unsigned* flags, const TilePlan& pl,
-                cudaStream_t st, int mode, const TileAdj* adj) {
+                cudaStream_t st, int mode, const TileAdj* adj, const TileExt* ext) {
   TileArgs a{};
   a.nx = p.nx;
   a.ny = p.ny;
@@ -75,6 +75,7 @@ int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out,
   a.probe_ez = probe_ez;
   a.flags = flags;
   if (adj) a.adj = *adj;
+  if (ext) a.ext = *ext;
   a.T = pl.T;
   a.hc = pl.hc;
   a.n_ti = pl.n_ti;
@@ -93,6 +94,10 @@ int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out,
       fdtd_host::note_cuda_error(e);
       return FDTD_ERR_CUDA;
     }
+  }
+  if (mode == kTileExt) {
+    a.vec = v && al16(a.ext.ez_rec) && a.ext.rec_slot % 4 == 0;
+    return launch_tile_ext(a, pl.V, lossy, pml, st);
   }
   if (mode != kTileFwd) {
     if (!pml || !v || !adj) return FDTD_ERR_ARG;

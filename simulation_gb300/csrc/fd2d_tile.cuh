@@ -33,7 +33,9 @@
 // direction as a step does, and the two values that cross strips are the
 // adjoint of cy downwards and that of the D update's curl upwards.  All it
 // needs of the forward run is dz' - iz in the design box and ez at the probe,
-// which a forward run in mode kTileRec leaves per step.
+// which a forward run in mode kTileRec leaves per step.  Mode kTileExt takes the
+// TF/SF box's corrections from the incident line's table and leaves ez of every
+// step for the running DFT (fd2d_dft_rec.cu).
 #pragma once
 
 #include <type_traits>
@@ -63,6 +65,7 @@ struct TileArgs {
   float* probe_ez;
   unsigned* flags;    // one per block, 32 words apart, zero at the start
   TileAdj adj;        // modes kTileRec and kTileRev
+  TileExt ext;        // mode kTileExt
   int T;              // steps between exchanges = halo rows
   int hc;             // halo columns on each side: T rounded up to whole lanes, or 0 with one tile per row
   int n_ti, n_tj;
@@ -88,6 +91,9 @@ __host__ __device__ constexpr size_t tile_smem_bytes(int V, bool lossy, bool pml
 int launch_tile_rec(const TileArgs& a, int V, bool lossy, cudaStream_t st);
 // defined in fd2d_tile_rev.cu
 int launch_tile_rev(const TileArgs& a, int V, bool lossy, cudaStream_t st);
+// defined in fd2d_tile_ext*.cu
+int launch_tile_ext(const TileArgs& a, int V, bool lossy, bool pml, cudaStream_t st);
+int launch_tile_ext_lossy(const TileArgs& a, int V, bool pml, cudaStream_t st);
 
 // what a strip of a tile has to handle in its steps
 constexpr int kTileInt = 0;    // unit coefficients
@@ -152,7 +158,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
   constexpr int W = kTileWarps, R = W * V;
   constexpr bool IHXS = tile_ihx_smem(V, PML);
   constexpr int NARR = tile_arrays(V, LOSSY, PML, MODE);
-  constexpr bool REC = MODE == kTileRec, REV = MODE == kTileRev;
+  constexpr bool REC = MODE == kTileRec, REV = MODE == kTileRev, EXT = MODE == kTileExt;
   constexpr int A_NAZ = 0, A_IHY = 1, A_NBZ = PML ? 2 : 1, A_IZ = A_NBZ + 1, A_IHX = A_NBZ + (LOSSY ? 2 : 0),
                 A_G = A_IHX + (IHXS ? 1 : 0), A_GB = A_G + 1;
   extern __shared__ float4 tsm[];
@@ -247,7 +253,17 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
   // what a strip's steps have to handle, the same in the whole warp (j0 is a multiple of 4)
   const bool last_col = j0 + 4 == ny;
   const bool masks = i0 <= 0 || i0 + V - 1 >= nx - 1 || __any_sync(kAll, j0 < ny && j0 + 4 > ny);
-  const bool unit = __all_sync(kAll, col_ok && row_ok && j0 != 0 && !last_col);
+  // TF/SF box: strips with an edge column (D at np-1 and ny-np, hx at np-2 and
+  // ny-np) or an edge row (hy at np-2 and nx-np)
+  const int np = EXT ? a.ext.np : 0;
+  bool edge_c = false;
+  if (EXT && np > 0) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) edge_c |= j0 + c == np - 2 || j0 + c == np - 1 || j0 + c == ny - np;
+    edge_c = __any_sync(kAll, edge_c);
+  }
+  const bool edge_r = np > 0 && ((np - 2 >= i0 && np - 2 < i0 + V) || (nx - np >= i0 && nx - np < i0 + V));
+  const bool unit = __all_sync(kAll, col_ok && row_ok && j0 != 0 && !last_col) && !edge_c && !edge_r;
   const int kind = src_here || probe_here ? kTilePoint : masks ? kTileEdge : unit ? kTileInt : kTileGen;
   // owned cells of the design box, in whole lanes
   [[maybe_unused]] const int bc = j0 - a.adj.jb;
@@ -436,6 +452,26 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
       fy2 = f4(cc[3 * 32 + lane]);
       fy3 = f4(cc[4 * 32 + lane]);
     }
+    [[maybe_unused]] float hxi_lo = 0.f, hxi_hi = 0.f, ezi_lo = 0.f, ezi_hi = 0.f;
+    if constexpr (EXT && !INT) {
+      if (edge_c) {
+        hxi_lo = __ldg(a.ext.inc_h + 2 * s);
+        hxi_hi = __ldg(a.ext.inc_h + 2 * s + 1);
+        ezi_lo = __ldg(a.ext.inc_e + (size_t)s * ny + np - 1);
+        ezi_hi = __ldg(a.ext.inc_e + (size_t)s * ny + ny - np);
+      }
+    }
+    // x of the lane's columns jl and jh: += lo/2, -= hi/2
+    [[maybe_unused]] auto edges = [&](F4& x, int jl, float lo, int jh, float hi) {
+      auto put = [&](float& y, int j) {
+        if (j == jl) y = __fmaf_rn(0.5f, lo, y);
+        if (j == jh) y = __fmaf_rn(-0.5f, hi, y);
+      };
+      put(x.a.x, j0);
+      put(x.a.y, j0 + 1);
+      put(x.b.x, j0 + 2);
+      put(x.b.y, j0 + 3);
+    };
     // H on strip row r, ez of rows r and r+1
     auto h_row = [&](int r, const F4& e, const F4& en) {
       const int i = i0 + r;
@@ -469,6 +505,19 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
         } else {
           nhx = fma4(0.5f, cx, hx[r]);
           nhy = fma4(-0.5f, cy, hy[r]);
+        }
+        if constexpr (EXT) {
+          if (edge_c && i >= np - 1 && i <= nx - np) edges(nhx, np - 2, ezi_lo, ny - np, ezi_hi);
+          if (edge_r && (i == np - 2 || i == nx - np)) {
+            const float wy = i == np - 2 ? -0.5f : 0.5f;
+            auto put = [&](float& y, int j) {
+              if (j >= np - 1 && j <= ny - np) y = __fmaf_rn(wy, __ldg(a.ext.inc_e + (size_t)s * ny + j), y);
+            };
+            put(nhy.a.x, j0);
+            put(nhy.a.y, j0 + 1);
+            put(nhy.b.x, j0 + 2);
+            put(nhy.b.y, j0 + 3);
+          }
         }
         if (!MASK) {  // column ny-1, the last of its lane (ny % 4 == 0), is not updated
           nhx.b.y = last_col ? hx[r].b.y : nhx.b.y;
@@ -542,6 +591,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
           put(dz[r].b.y, j0 + 3);
         }
       }
+      if constexpr (EXT && !INT) {
+        if (edge_c && i >= np - 1 && i <= nx - np) edges(dz[r], np - 1, hxi_lo, ny - np, hxi_hi);
+      }
       F4 e;
       const F4 na = f4(at(A_NAZ, r));
       if (LOSSY) {
@@ -562,6 +614,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
         rec(e.a.y, j0 + 1);
         rec(e.b.x, j0 + 2);
         rec(e.b.y, j0 + 3);
+      }
+      if constexpr (EXT) {
+        if (a.ext.ez_rec && own_c && i >= oi0 && i < oi1)
+          tile_st(a.ext.ez_rec + s * a.ext.rec_slot, (size_t)i * ny, j0, ny, vec, to4(e));
       }
       if (last && a.ez && own_c && i >= oi0 && i < oi1) {
         const float4 v = to4(e);

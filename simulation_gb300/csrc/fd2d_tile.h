@@ -17,6 +17,14 @@ constexpr size_t kTileFlagBytes = kTileMaxBlocks * 128;  // flags of the largest
 constexpr int kTileFwd = 0;  // the time loop
 constexpr int kTileRec = 1;  // and dz' - iz of the design box after each step
 constexpr int kTileRev = 2;  // steps t0, t0-1, .. undone on the adjoint fields
+constexpr int kTileExt = 3;  // the time loop with TF/SF box and record of ez
+struct TileExt {
+  int np = 0;                      // TF/SF box, 0: none
+  const float* inc_e = nullptr;    // of the run's steps, as in MarchExt
+  const float* inc_h = nullptr;
+  float* ez_rec = nullptr;         // ez of step t0+s+1 at s*rec_slot, or null
+  size_t rec_slot = 0;
+};
 struct TileAdj {
   fdtd2d_box box{};
   int jb = 0, njp = 0;   // the box's columns in whole groups of four: first column, how many
@@ -31,6 +39,7 @@ bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& b
 constexpr int tile_rev_max_V(bool lossy) { return lossy ? 4 : 5; }  // the gradients' shared memory
 int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, const FieldSet& x0, const FieldSet& x1,
                 float* ez, int t0, int nsteps, int* status, float* probe_ez, unsigned* flags, const TilePlan& pl,
-                cudaStream_t st, int mode = kTileFwd, const TileAdj* adj = nullptr);
+                cudaStream_t st, int mode = kTileFwd, const TileAdj* adj = nullptr,
+                const TileExt* ext = nullptr);
 
 }  // namespace fdtd

@@ -1,5 +1,6 @@
-"""The chained passes with plane wave and running DFT against the per-function
-kernels, bitwise: sizes around the stripes and segments, box edges on stripe
+"""Plane wave and running DFT in the chained passes and in the on-chip loop
+against the per-function kernels, bitwise: sizes around the stripes and segments, the tiles and the
+incident line's warps, box edges on stripe
 borders, with and without layer and loss, frequency counts, either extra alone,
 step counts that take every pass length, graph replay and the smallest
 workspace."""
@@ -15,7 +16,7 @@ def _sim(nx, ny, lossy, npml, tfsf, nf, ns=64):
     dt = 0.01 / 6e8
     naz = nbz = None
     if lossy:
-        naz, nbz = G.dielectric(nx, ny, 8, min(nx, ny) // 4, dt, 30.0, 0.3)
+        naz, nbz = G.dielectric(nx, ny, min(8, min(nx, ny) // 4), min(nx, ny) // 4, dt, 30.0, 0.3)
     s = G.SimTM2D(nx, ny, pml=G.pmlparam(nx, ny, npml) if npml else None, naz=naz, nbz=nbz, lossy=lossy,
                   tfsf_npml=tfsf, freq=np.linspace(1e8, 9e8, nf) if nf else None, dt=dt, ns=ns)
     i = torch.arange(nx, device="cuda", dtype=torch.float64)[:, None]
@@ -44,8 +45,22 @@ def test_sizes(cuda_lib, nx, ny, lossy, npml, tfsf, nf):
     _equal(a, b, f"{nx}x{ny}")
 
 
-def test_graph_and_march(cuda_lib):
-    mk = lambda: _sim(1024, 1400, True, 8, 8, 3)  # noqa: E731
+@pytest.mark.parametrize("nx,ny,tfsf", [(20, 17, 4), (100, 100, 8), (129, 127, 8), (250, 241, 60), (96, 385, 8),
+                                        (1001, 61, 2), (513, 516, 8), (61, 3072, 9), (40, 3076, 9), (1024, 1024, 8),
+                                        (1080, 960, 112)])
+@pytest.mark.parametrize("lossy,npml,nf", [(True, 8, 3), (False, 4, 13), (True, 0, 1), (False, 0, 0)])
+def test_on_chip(cuda_lib, nx, ny, tfsf, lossy, npml, nf):
+    npml = min(npml, (min(nx, ny) - 1) // 2 - 1)
+    a, b = _sim(nx, ny, lossy, npml, tfsf, nf, 128), _sim(nx, ny, lossy, npml, tfsf, nf, 128)
+    for n in (4, 67, 9):
+        a.step(n)
+    b.step_per_function(80)
+    _equal(a, b, f"{nx}x{ny}")
+
+
+@pytest.mark.parametrize("nx,ny", [(1024, 1400), (400, 500)])
+def test_graph_and_march(cuda_lib, nx, ny):
+    mk = lambda: _sim(nx, ny, True, 8, 8, 3)  # noqa: E731
     a, c, g = mk(), mk(), mk()
     a.step(40)
     c.step(40, steps_per_pass=4)
