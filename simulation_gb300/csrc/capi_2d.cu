@@ -118,20 +118,6 @@ size_t tile_workspace_bytes(const fdtd2d_params* p) {
   return ext_on(p) ? b + line_bytes(p) + (p->nf > 0 ? tile_ext_steps(p) * slot_bytes(p) : 0) : b;
 }
 
-// Chained passes over padded copies, for grids whose rows are no multiple of 16
-// bytes (they would otherwise go three launches a step): two ping-pong sets,
-// the materials and ez, all with rows of pad_pitch floats.
-int pad_pitch(const fdtd2d_params* p) { return (p->ny + 3) / 4 * 4; }
-size_t pad_slot_bytes(const fdtd2d_params* p) {
-  return ((size_t)p->nx * pad_pitch(p) * sizeof(float) + 255) & ~(size_t)255;
-}
-size_t pad_workspace_bytes(const fdtd2d_params* p) {
-  return pad_slot_bytes(p) * (2 * nslots(p) + (p->nbz ? 2 : 1) + 1);
-}
-bool pad_ok(const fdtd2d_params* p, int steps_per_pass) {
-  return p->ny % 4 != 0 && !ext_on(p) && steps_per_pass == 0 && chain_better(p->nx, p->ny) && p->nx <= 8 * 65535;
-}
-
 // Chained passes with the plane wave and the running DFT: the march's workspace
 // and, with the DFT on, room for the ez of kExtRecSteps steps.
 constexpr int kExtRecSteps = 16;
@@ -140,6 +126,24 @@ bool chain_ext_ok(const fdtd2d_params* p, int steps_per_pass) {
 }
 size_t chain_ext_workspace_bytes(const fdtd2d_params* p) {
   return fused_workspace_bytes(p) + (p->nf > 0 ? kExtRecSteps * slot_bytes(p) : 0);
+}
+
+// Chained passes over padded copies, for grids whose rows are no multiple of 16
+// bytes (they would otherwise go three launches a step): two ping-pong sets,
+// the materials and ez, all with rows of pad_pitch floats.
+int pad_pitch(const fdtd2d_params* p) { return (p->ny + 3) / 4 * 4; }
+size_t pad_slot_bytes(const fdtd2d_params* p) {
+  return ((size_t)p->nx * pad_pitch(p) * sizeof(float) + 255) & ~(size_t)255;
+}
+// with plane wave or running DFT also the line's tables and the ez of kExtRecSteps
+// steps
+size_t pad_workspace_bytes(const fdtd2d_params* p) {
+  return pad_slot_bytes(p) * (2 * nslots(p) + (p->nbz ? 2 : 1) + 1 + (p->nf > 0 ? kExtRecSteps : 0)) + line_bytes(p);
+}
+bool pad_ok(const fdtd2d_params* p, int steps_per_pass) {
+  if (p->ny % 4 == 0 || steps_per_pass != 0 || p->nx > 8 * 65535) return false;
+  if (!ext_on(p)) return chain_better(p->nx, p->ny);
+  return chain_ext_better(p->nx, p->ny) && (p->tfsf_npml <= 0 || p->ny <= kLineMaxNy);
 }
 
 FieldSet workspace_set(const fdtd2d_params* p, void* workspace, size_t sb) {
@@ -175,15 +179,45 @@ int step_padded(const fdtd2d_params* p, const fdtd2d_state* s, int t0, int nstep
     if ((rc = step_three_launches(t + 1, *p, *s, st))) return rc;
   const FieldSet user{s->dz, s->iz, s->hx, s->hy, s->ihx, s->ihy};
   if ((rc = launch_pad(user, set[0], p->naz, naz, p->nbz, nbz, p->nx, p->ny, pitch, st))) return rc;
+  const bool ext_steps = ext_on(p);
+  MarchExt ext{};
+  ext.tfsf_npml = p->tfsf_npml;
+  ext.nf = p->nf;
+  const size_t slot = sb / sizeof(float);
+  float* rec = ez + slot;
+  float* inc_e = rec + (p->nf > 0 ? kExtRecSteps * slot : 0);
+  float* inc_h = inc_e + line_e_bytes(p) / sizeof(float);
+  int line_t0 = t, line_n = 0, rec_n = 0;
   int cur = 0;
   while (t < t0 + nsteps) {
     const int rem = t0 + nsteps - t, k = rem >= 8 ? 8 : 4;
     const bool last = k == rem;
-    rc = launch_chain(*p, pitch, naz, nbz, set[cur], set[1 - cur], last ? ez : nullptr, t, k, last ? s->status : nullptr,
-                      march_gen_cost(), st);
+    if (!ext_steps) {
+      rc = launch_chain(*p, pitch, naz, nbz, set[cur], set[1 - cur], last ? ez : nullptr, t, k,
+                        last ? s->status : nullptr, march_gen_cost(), st);
+    } else {
+      if (p->tfsf_npml > 0) {
+        if (t + k > line_t0 + line_n) {  // rem is a multiple of 4, the tables' steps of 8
+          line_t0 = t;
+          line_n = std::min(rem, kLineChunkSteps);
+          if ((rc = launch_inc_line(*p, *s, t, line_n, inc_e, inc_h, st))) return rc;
+        }
+        ext.inc_e = inc_e + (size_t)(t - line_t0) * p->ny;
+        ext.inc_h = inc_h + (size_t)(t - line_t0) * 2;
+      }
+      rc = launch_chain_ext(*p, pitch, naz, nbz, set[cur], set[1 - cur], last ? ez : nullptr, t, k,
+                            last ? s->status : nullptr, march_gen_cost(), ext, rec + rec_n * slot, slot, st);
+    }
     if (rc) return rc;
     cur = 1 - cur;
     t += k;
+    rec_n += k;
+    if (p->nf > 0 && (last || rec_n + 8 > kExtRecSteps)) {
+      if ((rc = launch_dft_rec(p->nx, p->ny, pitch, t - rec_n, rec_n, p->nf, p->dft_cos, p->dft_sin, rec, slot, s->r_pt,
+                               s->i_pt, st)))
+        return rc;
+      rec_n = 0;
+    }
   }
   return launch_unpad(set[cur], user, ez, s->ez, p->nx, p->ny, pitch, st);
 }
@@ -211,7 +245,7 @@ int step_tile_ext(const fdtd2d_params* p, const fdtd2d_state* s, int t0, int nst
     if ((rc = launch_tile(*p, user, user, x0, user, last ? s->ez : nullptr, t, n, last ? s->status : nullptr,
                           s->probe_ez, flags, tile, st, kTileExt, nullptr, &ext)))
       return rc;
-    if (p->nf > 0 && (rc = launch_dft_rec((size_t)p->nx * p->ny, t, n, p->nf, p->dft_cos, p->dft_sin, ext.ez_rec,
+    if (p->nf > 0 && (rc = launch_dft_rec(p->nx, p->ny, p->ny, t, n, p->nf, p->dft_cos, p->dft_sin, ext.ez_rec,
                                           ext.rec_slot, s->r_pt, s->i_pt, st)))
       return rc;
     t += n;
@@ -404,7 +438,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
     const int n = rec_n;
     rec_n = 0;
     if (n == 0) return FDTD_OK;
-    return launch_dft_rec((size_t)p->nx * p->ny, t - n, n, p->nf, p->dft_cos, p->dft_sin, ez_rec, rec_slot, s->r_pt,
+    return launch_dft_rec(p->nx, p->ny, p->ny, t - n, n, p->nf, p->dft_cos, p->dft_sin, ez_rec, rec_slot, s->r_pt,
                           s->i_pt, st);
   };
   for (size_t i = 0; i < sched.size(); ++i) {
@@ -436,7 +470,7 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
       const bool chained = chain && (sched[i] == 8 || sched[i] == 4);
       if ((!chained || rec_n + sched[i] > kExtRecSteps) && (rc = flush())) return rc;
       if (chained) {
-        rc = launch_chain_ext(*p, in, out, ez, t, sched[i], status, march_gen_cost(), ext, ez_rec + rec_n * rec_slot,
+        rc = launch_chain_ext(*p, p->ny, p->naz, p->nbz, in, out, ez, t, sched[i], status, march_gen_cost(), ext, ez_rec + rec_n * rec_slot,
                               rec_slot, st);
         if (p->nf > 0) rec_n += sched[i];
       } else {

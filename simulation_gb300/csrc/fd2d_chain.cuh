@@ -144,9 +144,9 @@ int launch_chain(const fdtd2d_params& p, int pitch, const float* naz, const floa
                  const FieldSet& out, float* ez, int t0, int k, int* status, float gen_cost, cudaStream_t st);
 // the same with the plane wave and the running DFT of `ext` (fd2d_chain_ext.cu); ez_rec: room for
 // the ez of k steps, rec_slot floats each (nf > 0)
-int launch_chain_ext(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int k,
-                     int* status, float gen_cost, const MarchExt& ext, float* ez_rec, size_t rec_slot,
-                     cudaStream_t st);
+int launch_chain_ext(const fdtd2d_params& p, int pitch, const float* naz, const float* nbz, const FieldSet& in,
+                     const FieldSet& out, float* ez, int t0, int k, int* status, float gen_cost, const MarchExt& ext,
+                     float* ez_rec, size_t rec_slot, cudaStream_t st);
 
 namespace {
 

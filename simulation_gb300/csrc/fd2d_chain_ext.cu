@@ -24,11 +24,11 @@ int launch_k(const ChainArgs& a, bool lossy, bool pml, int pml_cells, float g, c
 
 }  // namespace
 
-int launch_chain_ext(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int k,
-                     int* status, float gen_cost, const MarchExt& ext, float* ez_rec, size_t rec_slot,
-                     cudaStream_t st) {
+int launch_chain_ext(const fdtd2d_params& p, int pitch, const float* naz, const float* nbz, const FieldSet& in,
+                     const FieldSet& out, float* ez, int t0, int k, int* status, float gen_cost, const MarchExt& ext,
+                     float* ez_rec, size_t rec_slot, cudaStream_t st) {
   if (k != 4 && k != 8) return FDTD_ERR_ARG;
-  ChainArgs a = chain_args(p, p.ny, p.naz, p.nbz, in, out, ez, t0, status);
+  ChainArgs a = chain_args(p, pitch, naz, nbz, in, out, ez, t0, status);
   a.np = ext.tfsf_npml;
   a.inc_e = ext.inc_e;
   a.inc_h = ext.inc_h;

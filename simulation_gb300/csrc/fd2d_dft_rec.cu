@@ -10,6 +10,7 @@ struct DftRecArgs {
   int steps, nf, f0;
   const float* ez;  // step s at ez + s*slot
   size_t slot;
+  int ny, pitch;   // columns of a row of the accumulators, and of the record (V = 1 where they differ)
   const float* cs;  // [step][nf]
   const float* sn;
   float *re, *im;   // [nf][n*V]
@@ -24,6 +25,7 @@ __global__ void __launch_bounds__(256) k_dft_rec(const DftRecArgs a) {
   const size_t n = blockIdx.x * (size_t)256 + threadIdx.x;
   if (n >= a.n) return;
   const size_t c = n * V;
+  const size_t ce = V == 1 && a.pitch != a.ny ? c / a.ny * a.pitch + c % a.ny : c;
   auto ld = [](const float* p, float (&v)[V]) {
     if constexpr (V == 4) {
       const float4 x = __ldcs(reinterpret_cast<const float4*>(p));
@@ -62,13 +64,13 @@ __global__ void __launch_bounds__(256) k_dft_rec(const DftRecArgs a) {
   for (; s + 8 <= a.steps; s += 8) {
     float e[8][V];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) ld(a.ez + (s + q) * a.slot + c, e[q]);
+    for (int q = 0; q < 8; ++q) ld(a.ez + (s + q) * a.slot + ce, e[q]);
 #pragma unroll
     for (int q = 0; q < 8; ++q) add(s + q, e[q]);
   }
   for (; s < a.steps; ++s) {
     float e[V];
-    ld(a.ez + s * a.slot + c, e);
+    ld(a.ez + s * a.slot + ce, e);
     add(s, e);
   }
 #pragma unroll
@@ -96,11 +98,12 @@ int launch_v(DftRecArgs a, cudaStream_t st) {
 
 }  // namespace
 
-int launch_dft_rec(size_t ncell, int t0, int steps, int nf, const float* dft_cos, const float* dft_sin, const float* ez,
+int launch_dft_rec(int nx, int ny, int pitch, int t0, int steps, int nf, const float* dft_cos, const float* dft_sin, const float* ez,
                    size_t slot, float* r_pt, float* i_pt, cudaStream_t st) {
   // table row t-1 = t0+s of step t0+s+1
-  DftRecArgs a{ncell, steps, nf, 0, ez, slot, dft_cos + (size_t)t0 * nf, dft_sin + (size_t)t0 * nf, r_pt, i_pt};
-  if (ncell % 4 == 0 && slot % 4 == 0 && (((uintptr_t)ez | (uintptr_t)r_pt | (uintptr_t)i_pt) & 15u) == 0) {
+  const size_t ncell = (size_t)nx * ny;
+  DftRecArgs a{ncell, steps, nf, 0, ez, slot, ny, pitch, dft_cos + (size_t)t0 * nf, dft_sin + (size_t)t0 * nf, r_pt, i_pt};
+  if (pitch == ny && ncell % 4 == 0 && slot % 4 == 0 && (((uintptr_t)ez | (uintptr_t)r_pt | (uintptr_t)i_pt) & 15u) == 0) {
     a.n = ncell / 4;
     return launch_v<4>(a, st);
   }

@@ -78,8 +78,8 @@ constexpr int kLineChunkSteps = 64;    // incident-line steps per table
 bool march_ext_supported(const fdtd2d_params& p);
 int launch_march_ext(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, float* ez, int t0, int k,
                      int* status, const MarchExt& ext, cudaStream_t st);
-// adds `steps` recorded ez (step t0+s+1 at ez + s*slot) to the accumulators (fd2d_dft_rec.cu)
-int launch_dft_rec(size_t ncell, int t0, int steps, int nf, const float* dft_cos, const float* dft_sin, const float* ez,
+// adds `steps` recorded ez (step t0+s+1 at ez + s*slot, rows of `pitch`) to the accumulators (fd2d_dft_rec.cu)
+int launch_dft_rec(int nx, int ny, int pitch, int t0, int steps, int nf, const float* dft_cos, const float* dft_sin, const float* ez,
                    size_t slot, float* r_pt, float* i_pt, cudaStream_t st);
 // Advance the incident line (ezinct, hxinct, the input-probe DFT) by nsteps
 // steps t0+1 .. t0+nsteps and record what the 2D update reads of it

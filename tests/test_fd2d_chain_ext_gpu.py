@@ -34,7 +34,7 @@ def _equal(a, b, what):
             assert torch.equal(x, y), f"{what}: {k} max {float((x - y).abs().max()):.3e}"
 
 
-@pytest.mark.parametrize("nx,ny", [(1024, 1400), (1100, 1344), (8200, 132), (300, 4096), (1403, 1012)])
+@pytest.mark.parametrize("nx,ny", [(1024, 1400), (1100, 1344), (8200, 132), (300, 4096), (1403, 1012), (1300, 1345), (1024, 1402)])
 @pytest.mark.parametrize("lossy,npml,tfsf,nf", [(True, 8, 8, 3), (True, 12, 9, 1), (False, 8, 8, 6), (True, 0, 60, 2),
                                                 (False, 8, 0, 4), (True, 8, 8, 0)])
 def test_sizes(cuda_lib, nx, ny, lossy, npml, tfsf, nf):
