@@ -279,6 +279,15 @@ int fdtd2d_tm_adjoint_forward(const fdtd2d_params* p, const fdtd2d_adjoint_param
                               void* workspace, size_t workspace_bytes, fdtd_stream_t stream);
 int fdtd2d_tm_adjoint_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz,
                               float* grad_nbz, void* workspace, size_t workspace_bytes, fdtd_stream_t stream);
+/* The same two halves for callers that run the reverse with the p, a and workspace
+ * of the forward, unchanged: the forward may leave what the reverse needs in the
+ * workspace (_reverse runs the segments again instead, and may be given another
+ * box or probe, after which _reverse_rec needs a new forward).  Same results; the
+ * reverse may be called more than once. */
+int fdtd2d_tm_adjoint_forward_rec(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* trace, double* J,
+                                  void* workspace, size_t workspace_bytes, fdtd_stream_t stream);
+int fdtd2d_tm_adjoint_reverse_rec(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz,
+                                  float* grad_nbz, void* workspace, size_t workspace_bytes, fdtd_stream_t stream);
 int fdtd2d_tm_adjoint(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* trace, double* J,
                       float* grad_naz, float* grad_nbz, void* workspace, size_t workspace_bytes,
                       fdtd_stream_t stream);

@@ -138,7 +138,11 @@ _SIGS = {
     "fdtd2d_tm_adjoint_workspace_size": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D)], C.c_size_t),
     "fdtd2d_tm_adjoint_forward": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D), F, P, P, C.c_size_t, P],
                                   C.c_int),
+    "fdtd2d_tm_adjoint_forward_rec": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D), F, P, P, C.c_size_t, P],
+                                  C.c_int),
     "fdtd2d_tm_adjoint_reverse": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D), F, F, P, C.c_size_t, P],
+                                  C.c_int),
+    "fdtd2d_tm_adjoint_reverse_rec": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D), F, F, P, C.c_size_t, P],
                                   C.c_int),
     "fdtd2d_tm_adjoint": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D), F, P, F, F, P, C.c_size_t, P], C.c_int),
     "fno_profile_features": ([C.c_int, P, P, P, P, P, P, C.c_int, C.c_double, C.c_double, F, P], C.c_int),

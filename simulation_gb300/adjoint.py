@@ -115,7 +115,7 @@ class AdjointProblem:
     def forward(self) -> float:
         """Run the time loop with checkpoints; returns J = sum_t Ez_t(probe)^2."""
         def body():
-            _lib.call("fdtd2d_tm_adjoint_forward", C.byref(self.sim._p), C.byref(self.ap), self.trace.data_ptr(),
+            _lib.call("fdtd2d_tm_adjoint_forward_rec", C.byref(self.sim._p), C.byref(self.ap), self.trace.data_ptr(),
                       self.J_dev.data_ptr(), self.ws.data_ptr(), self.ws.numel(), _lib.stream_ptr())
 
         self._run("forward", body)
@@ -128,7 +128,7 @@ class AdjointProblem:
         """dJ/dnaz on the design box (float32 [bi][bj]) by the reverse sweep
         over the checkpoints of the last ``forward``."""
         def body():
-            _lib.call("fdtd2d_tm_adjoint_reverse", C.byref(self.sim._p), C.byref(self.ap),
+            _lib.call("fdtd2d_tm_adjoint_reverse_rec", C.byref(self.sim._p), C.byref(self.ap),
                       self.grad_naz.data_ptr(), None, self.ws.data_ptr(), self.ws.numel(), _lib.stream_ptr())
 
         self._run("reverse", body)

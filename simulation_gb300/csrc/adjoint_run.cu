@@ -11,10 +11,11 @@
 //             else fused passes of up to 4 steps; each segment starts from a
 //             stored state (the one before writes it directly) and the probe's
 //             Ez is recorded every step; J is summed on the device in double;
-//   reverse   segments last first.  Where the tiles fit: the segment runs
-//             again from its checkpoint, recording what the reverse needs of
-//             it (the design box and the probe), and is undone on the chip,
-//             one launch each.  Else a segment's states are recomputed from
+//   reverse   segments last first.  Where the tiles fit a segment is undone on
+//             the chip in one launch.  What it needs of the forward run (the
+//             design box and the probe) the _rec forms leave during the forward
+//             where the box of all steps fits the record buffers; otherwise the
+//             segment first runs again from its checkpoint.  Else a segment's states are recomputed from
 //             its checkpoint by recording passes (one pass of 4 steps stores
 //             dz, iz, hx, hy after each of its steps), on a second stream,
 //             one segment ahead of the sweep (two record buffers, events
@@ -22,8 +23,8 @@
 //             two steps (one step for an odd segment's first), the adjoint
 //             fields ping-ponging between two sets.
 // At 1024^2, 1500 steps, checkpoint 64, a lossless 256^2 box: 15.4 ms on the
-// chip (forward 4.7, recording runs 5.0, reverse 5.4) against 38.5 streaming,
-// whose reverse reads two recorded states and the adjoints of every tile from
+// chip with the segments run again (forward 4.7, recording runs 5.0, reverse
+// 5.4), 10.5 with the forward's record, against 38.5 streaming, whose reverse reads two recorded states and the adjoints of every tile from
 // L2 in each launch (33 us for two steps; 7.2 here, exchanges included).
 // Results do not depend on the checkpoint interval or on the overlap: every
 // recorded state is bitwise the forward's, and each reverse step does the
@@ -225,8 +226,42 @@ bool tile_layout(const fdtd2d_params* p, const Layout& L, TilePlan& pl, int max_
          (size_t)pl.n_ti * pl.n_tj * 128 <= L.slot;
 }
 
+// What the reverse on the chip needs of the forward run: the design box's dz' - iz
+// per step, at the start of the record area, and behind `steps` of them the
+// probe's ez.
+TileAdj box_record(const fdtd2d_adjoint_params* a, const Layout& L) {
+  TileAdj adj;
+  adj.box = a->box;
+  adj.jb = a->box.j0 & ~3;
+  adj.njp = ((a->box.j0 + a->box.nj + 3) & ~3) - adj.jb;
+  adj.rec = at(L, L.rec0);
+  adj.probe_w = a->probe_weight;
+  return adj;
+}
+size_t box_floats(const TileAdj& adj) { return (size_t)adj.box.ni * adj.njp; }
+
+// both directions on the chip
+bool tile_layouts(const fdtd2d_params* p, const Layout& L, TilePlan& fwd, TilePlan& rev) {
+  return L.cp >= kTileMinSteps && tile_layout(p, L, fwd) && tile_layout(p, L, rev, tile_rev_max_V(p->nbz != nullptr));
+}
+
+// Whether the forward run can leave the box of all its steps, so that the reverse
+// runs nothing again.  The record areas hold it (whole_floats) and behind it one
+// segment's, which a reverse that does run the segments again uses.
+size_t whole_floats(const fdtd2d_adjoint_params* a, const TileAdj& adj) {
+  return ((size_t)a->nsteps * (box_floats(adj) + 1) + 63) & ~(size_t)63;
+}
+bool whole_record(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, const Layout& L) {
+  TilePlan fwd, rev;
+  if (!tile_layouts(p, L, fwd, rev)) return false;
+  const size_t room = 2 * (size_t)(L.cp - 1) * nrec(p) * (L.slot / sizeof(float));
+  const TileAdj adj = box_record(a, L);
+  return whole_floats(a, adj) + (size_t)L.cp * (box_floats(adj) + 1) <= room;
+}
+
+// record: leave the box of every step (whole_record)
 int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* trace, double* J, void* ws,
-                cudaStream_t st) {
+                bool record, cudaStream_t st) {
   const Layout L = layout(p0, a, ws);
   fdtd2d_params p = *p0;  // the probe of the objective
   p.probe_i = a->probe_i;
@@ -238,14 +273,16 @@ int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* 
   float* ez = at(L, L.ez);
   TilePlan pl;
   const bool tile = tile_layout(&p, L, pl);
+  TileAdj adj = box_record(a, L);
   for (int c = 0; c < L.ncp; ++c) {
     const int t_start = c * L.cp;
     const int len = std::min(L.cp, a->nsteps - t_start);
-    if (tile && len >= kTileMinSteps) {
+    if (tile && (record || len >= kTileMinSteps)) {
       const FieldSet out = set_of(ckpt(&p, L, c + 1));
       if ((rc = launch_tile(p, set_of(ckpt(&p, L, c)), out, set_of(xbuf(&p, L, 0)), out, nullptr, t_start, len,
-                            nullptr, trace, (unsigned*)ez, pl, st)))
+                            nullptr, trace, (unsigned*)ez, pl, st, record ? kTileRec : kTileFwd, &adj)))
         return rc;
+      adj.rec += len * box_floats(adj);
       continue;
     }
     const int kk = march_default_steps(p.nx, p.ny);
@@ -258,6 +295,10 @@ int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* 
       in = out;
       t += k;
     }
+  }
+  if (record) {
+    rc = cuda_rc(cudaMemcpyAsync(adj.rec, trace, (size_t)a->nsteps * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    if (rc) return rc;
   }
   if (J) {
     k_objective<<<1, 256, 0, st>>>(trace, a->nsteps, a->probe_weight, J);
@@ -285,33 +326,35 @@ int recompute(const fdtd2d_params* p, const Layout& L, int c, int len, int b, cu
   return FDTD_OK;
 }
 
-// The reverse sweep on the chip: segments last first, each run forward again
-// from its checkpoint to record the design box's dz' - iz and the probe's ez
-// (cp steps of at most a grid each, in the room of six recorded states a step),
-// then undone in one launch, all on the caller's stream.
+// The reverse sweep on the chip: segments last first, each undone in one launch
+// on the caller's stream.  Without the forward's record the segment is run again
+// from its checkpoint first, to record it.
 int run_reverse_tile(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* grad_naz, float* grad_nbz,
-                     const Layout& L, const TilePlan& fwd, const TilePlan& rev, cudaStream_t st) {
+                     const Layout& L, const TilePlan& fwd, const TilePlan& rev, bool recorded, cudaStream_t st) {
   fdtd2d_params p = *p0;
   p.probe_i = a->probe_i;
   p.probe_j = a->probe_j;
-  TileAdj adj;
-  adj.box = a->box;
-  adj.jb = a->box.j0 & ~3;
-  adj.njp = ((a->box.j0 + a->box.nj + 3) & ~3) - adj.jb;
-  adj.rec = at(L, L.rec0);
-  adj.probe_w = a->probe_weight;
+  TileAdj adj = box_record(a, L);
   adj.grad_naz = grad_naz;
   adj.grad_nbz = grad_nbz;
-  float* probe = adj.rec + (size_t)L.cp * adj.box.ni * adj.njp;  // [cp]
+  if (!recorded && whole_record(p0, a, L)) adj.rec += whole_floats(a, adj);
+  float* const rec = adj.rec;
+  // (one segment's record, cp steps of at most a grid each, fits in the room of six states a step)
+  float* probe = rec + (recorded ? a->nsteps : L.cp) * box_floats(adj);
   unsigned* flags = (unsigned*)at(L, L.ez);
   const FieldSet x0 = set_of(xbuf(&p, L, 0)), x1 = set_of(xbuf(&p, L, 1));
   int cur = 0;
   for (int c = L.ncp - 1; c >= 0; --c) {
     const int t_start = c * L.cp, len = std::min(L.cp, a->nsteps - t_start);
-    float* pz = probe - t_start;  // indexed by step
-    int rc = launch_tile(p, set_of(ckpt(&p, L, c)), x1, x0, x1, nullptr, t_start, len, nullptr, pz, flags, fwd, st,
-                         kTileRec, &adj);
-    if (rc) return rc;
+    float* pz = recorded ? probe : probe - t_start;  // indexed by step
+    int rc;
+    if (recorded) {
+      adj.rec = rec + (size_t)t_start * box_floats(adj);
+    } else {
+      rc = launch_tile(p, set_of(ckpt(&p, L, c)), x1, x0, x1, nullptr, t_start, len, nullptr, pz, flags, fwd, st,
+                       kTileRec, &adj);
+      if (rc) return rc;
+    }
     const FieldSet out = set_of(adjbuf(&p, L, 1 - cur));
     rc = launch_tile(p, set_of(adjbuf(&p, L, cur)), out, x0, out, nullptr, t_start + len, len, nullptr, pz, flags, rev,
                      st, kTileRev, &adj);
@@ -322,7 +365,7 @@ int run_reverse_tile(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, fl
 }
 
 int run_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz, float* grad_nbz,
-                void* ws, cudaStream_t main) {
+                void* ws, bool recorded, cudaStream_t main) {
   const Layout L = layout(p, a, ws);
   int rc;
   const size_t gb = (size_t)a->box.ni * a->box.nj * sizeof(float);
@@ -330,8 +373,8 @@ int run_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* g
   if ((rc = cuda_rc(cudaMemsetAsync(grad_naz, 0, gb, main)))) return rc;
   if (grad_nbz && (rc = cuda_rc(cudaMemsetAsync(grad_nbz, 0, gb, main)))) return rc;
   TilePlan fwd, rev;
-  if (L.cp >= kTileMinSteps && tile_layout(p, L, fwd) && tile_layout(p, L, rev, tile_rev_max_V(p->nbz != nullptr)))
-    return run_reverse_tile(p, a, grad_naz, grad_nbz, L, fwd, rev, main);
+  if (tile_layouts(p, L, fwd, rev))
+    return run_reverse_tile(p, a, grad_naz, grad_nbz, L, fwd, rev, recorded, main);
   Side* side = nullptr;
   if ((rc = side_of_device(&side))) return rc;
   cudaStream_t ss = side->stream;
@@ -393,7 +436,16 @@ int fdtd2d_tm_adjoint_forward(const fdtd2d_params* p, const fdtd2d_adjoint_param
   if (rc) return rc;
   if (!trace) return FDTD_ERR_NULL;
   if ((rc = check_ws(p, a, workspace, workspace_bytes))) return rc;
-  return run_forward(p, a, trace, J, workspace, (cudaStream_t)stream);
+  return run_forward(p, a, trace, J, workspace, false, (cudaStream_t)stream);
+}
+
+int fdtd2d_tm_adjoint_forward_rec(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* trace, double* J,
+                                  void* workspace, size_t workspace_bytes, fdtd_stream_t stream) {
+  int rc = check(p, a);
+  if (rc) return rc;
+  if (!trace) return FDTD_ERR_NULL;
+  if ((rc = check_ws(p, a, workspace, workspace_bytes))) return rc;
+  return run_forward(p, a, trace, J, workspace, whole_record(p, a, layout(p, a, workspace)), (cudaStream_t)stream);
 }
 
 int fdtd2d_tm_adjoint_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz,
@@ -403,7 +455,18 @@ int fdtd2d_tm_adjoint_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_param
   if (!grad_naz) return FDTD_ERR_NULL;
   if (grad_nbz && !p->nbz) return FDTD_ERR_ARG;
   if ((rc = check_ws(p, a, workspace, workspace_bytes))) return rc;
-  return run_reverse(p, a, grad_naz, grad_nbz, workspace, (cudaStream_t)stream);
+  return run_reverse(p, a, grad_naz, grad_nbz, workspace, false, (cudaStream_t)stream);
+}
+
+int fdtd2d_tm_adjoint_reverse_rec(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz,
+                                  float* grad_nbz, void* workspace, size_t workspace_bytes, fdtd_stream_t stream) {
+  int rc = check(p, a);
+  if (rc) return rc;
+  if (!grad_naz) return FDTD_ERR_NULL;
+  if (grad_nbz && !p->nbz) return FDTD_ERR_ARG;
+  if ((rc = check_ws(p, a, workspace, workspace_bytes))) return rc;
+  return run_reverse(p, a, grad_naz, grad_nbz, workspace, whole_record(p, a, layout(p, a, workspace)),
+                     (cudaStream_t)stream);
 }
 
 int fdtd2d_tm_adjoint(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* trace, double* J,
@@ -414,8 +477,9 @@ int fdtd2d_tm_adjoint(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, fl
   if (!trace || !grad_naz) return FDTD_ERR_NULL;
   if (grad_nbz && !p->nbz) return FDTD_ERR_ARG;
   if ((rc = check_ws(p, a, workspace, workspace_bytes))) return rc;
-  if ((rc = run_forward(p, a, trace, J, workspace, (cudaStream_t)stream))) return rc;
-  return run_reverse(p, a, grad_naz, grad_nbz, workspace, (cudaStream_t)stream);
+  const bool rec = whole_record(p, a, layout(p, a, workspace));
+  if ((rc = run_forward(p, a, trace, J, workspace, rec, (cudaStream_t)stream))) return rc;
+  return run_reverse(p, a, grad_naz, grad_nbz, workspace, rec, (cudaStream_t)stream);
 }
 
 }  // extern "C"

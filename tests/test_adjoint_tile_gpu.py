@@ -53,3 +53,38 @@ def test_against_streaming(cuda_lib, nx, ny, box, src, probe, lossy, kind):
     for x in (a, c):
         for p, q in zip(x, b):
             assert (p is None and q is None) or torch.equal(p, q)
+
+
+@pytest.mark.parametrize("box,ns,cp", [((30, 40, 40, 50), 90, 32), ((1, 1, 98, 126), 90, 8), ((1, 1, 98, 126), 400, 8),
+                                       ((60, 3, 5, 120), 91, 30)])
+def test_recorded_halves(cuda_lib, box, ns, cp):
+    """forward_rec/reverse_rec (with and without room for the whole record) equal
+    the unrecorded halves, in any order and repeated"""
+    from simulation_gb300 import _lib
+    from simulation_gb300 import fd2d as G
+    s = G.SimTM2D(100, 128, pml=G.pmlparam(100, 128, 8), source=G.PointSource(25, 64, ("gauss", 12, 4.0), "soft"),
+                  lossy=False, ns=ns)
+    s.naz.fill_(0.7)
+    ap = _lib.AdjointParams2D(ns, cp, 50, 64, 2.0, _lib.Box2D(*box))
+    n = _lib.lib().fdtd2d_tm_adjoint_workspace_size(C.byref(s._p), C.byref(ap))
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    trace = torch.zeros(ns, device="cuda")
+    J = torch.zeros(1, dtype=torch.float64, device="cuda")
+
+    def fwd(rec):
+        _lib.call("fdtd2d_tm_adjoint_forward" + rec, C.byref(s._p), C.byref(ap), trace.data_ptr(), J.data_ptr(),
+                  ws.data_ptr(), ws.numel(), _lib.stream_ptr())
+        return trace.clone(), J.clone()
+
+    def rev(rec):
+        g = torch.empty(box[2:], device="cuda")
+        _lib.call("fdtd2d_tm_adjoint_reverse" + rec, C.byref(s._p), C.byref(ap), g.data_ptr(), None, ws.data_ptr(),
+                  ws.numel(), _lib.stream_ptr())
+        return g
+
+    want = fwd("") + (rev(""),)
+    got = fwd("_rec") + (rev("_rec"), rev(""), rev("_rec"))
+    assert float(want[2].abs().max()) > 0
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    for g in got[2:]:
+        assert torch.equal(g, want[2])
