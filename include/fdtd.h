@@ -157,24 +157,29 @@ int fdtd2d_fourier(int t, const fdtd2d_params* p, fdtd2d_state* s, fdtd_stream_t
  * TF/SF on. */
 size_t fdtd2d_workspace_size(const fdtd2d_params* p, int steps_per_pass);
 /* Bytes of device workspace with which fdtd2d_step_n takes its fastest path on
- * the current device (at least fdtd2d_workspace_size): with them, grids that
- * fit on the chip run a whole call in one launch.  A smaller workspace, down to
- * fdtd2d_workspace_size, gives the same results. */
+ * the current device (at least fdtd2d_workspace_size): grids that fit on the
+ * chip run a whole call in one launch (64 steps a launch with TF/SF or the DFT),
+ * ragged rows run on padded copies, and with the DFT on 16 to 64 steps' ez are
+ * kept beside the fields.  A smaller workspace, down to fdtd2d_workspace_size,
+ * gives the same results. */
 size_t fdtd2d_fast_workspace_size(const fdtd2d_params* p, int steps_per_pass);
 
 /* fdtd2d_step_n: the program's time loop for t = t0+1 .. t0+nsteps, in the
- * reference's step order (fd2d/python/fd2d_3_4.py:268-277).  The core
- * D->source->E->H update is fused into one streaming kernel that keeps
- * `steps_per_pass` (1..4; 0 = library default: 2 below 2^21 cells, else 4) time steps in registers per
- * pass over HBM; `workspace` (fdtd2d_workspace_size bytes, 256-byte aligned)
- * holds the ping-pong copy of the evolving fields.  Results land in the
- * caller's arrays, bitwise equal to calling dfield/efield/hfield per step.
- * TF/SF and the running DFT (nf <= 8) ride in the same fused passes: the
- * incident line is advanced ahead of them in one launch per 64 steps (its
- * tables are part of the workspace), the box-edge corrections and the DFT
- * accumulation happen inside the pass, bitwise equal to the nine per-function
- * calls per step.  Grids with ny % 4 != 0, nf > 8, TF/SF with ny > 16384, a
- * probe trace together with TF/SF or the DFT, or nsteps == 1 run each step as
+ * reference's step order (fd2d/python/fd2d_3_4.py:268-277).  With
+ * steps_per_pass = 0 the library chooses: the whole loop on the chip where the
+ * grid fits (with fdtd2d_fast_workspace_size), chained passes of 8 time steps
+ * on larger grids, or passes of 2 or 4.  With 1..4 the D->source->E->H update
+ * runs in one streaming kernel that keeps that many time steps in registers per
+ * pass over HBM.  `workspace` (256-byte aligned) holds the ping-pong copy of
+ * the evolving fields.  Results land in the caller's arrays, bitwise equal to
+ * calling dfield/efield/hfield per step, whatever the choice.
+ * TF/SF and the running DFT ride in the same kernels: the incident line is
+ * advanced ahead of them in one launch per 64 steps (its tables are part of the
+ * workspace), the box-edge corrections happen inside the pass, the DFT inside
+ * it or from the record of ez, bitwise equal to the nine per-function calls per
+ * step.  What those kernels do not take (nsteps == 1; TF/SF with ny > 16384;
+ * without the larger workspace or beyond the grids that fit on the chip: ny % 4
+ * != 0, nf > 8, a probe trace together with TF/SF or the DFT) runs each step as
  * three launches instead (D + ezinct + inctdz; E + fourier + hxinct; H +
  * incthx + incthy; no workspace), with the same results.
  * Replaces the `for t in 1..ns` loops of fd2d/python/fd2d_3_2.py:139-142 and
@@ -332,6 +337,10 @@ typedef struct {
 } fdtd_gemm_desc;
 
 int fdtd_gemm_bf16(const fdtd_gemm_desc* d, int* status, fdtd_stream_t stream);
+/* the product as a gradient through the GELU of z (BF16, laid out as C16): C16 =
+ * BF16(acc * gelu'(z)), and dsum[n] += the column sums of C16.  N = 128, M % 128 ==
+ * 0, alpha = 1, no other epilogue */
+int fdtd_gemm_bf16_gelu_bwd(const fdtd_gemm_desc* d, const void* z, float* dsum, int* status, fdtd_stream_t stream);
 
 /* ------------------------------------------------ surrogate helper kernels
  * Element-wise/reduction pieces of the 1D Fourier-neural-operator surrogate

@@ -24,8 +24,9 @@
 //             fields ping-ponging between two sets.
 // At 1024^2, 1500 steps, checkpoint 64, a lossless 256^2 box: 15.4 ms on the
 // chip with the segments run again (forward 4.7, recording runs 5.0, reverse
-// 5.4), 10.5 with the forward's record, against 38.5 streaming, whose reverse reads two recorded states and the adjoints of every tile from
-// L2 in each launch (33 us for two steps; 7.2 here, exchanges included).
+// 5.4), 10.5 with the forward's record, against 38.5 streaming, whose reverse
+// reads two recorded states and the adjoints of every tile from L2 in each launch
+// (33 us for two steps; 7.2 here, exchanges included).
 // Results do not depend on the checkpoint interval or on the overlap: every
 // recorded state is bitwise the forward's, and each reverse step does the
 // same per-cell arithmetic (fdtd2d_adjoint_step's two kernels give the same

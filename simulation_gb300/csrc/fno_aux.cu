@@ -7,30 +7,12 @@
 
 #include <algorithm>
 
-#include "fdtd_common.cuh"
+#include "tc_common.cuh"
 
 namespace fdtd {
 namespace {
 
 using bf16 = __nv_bfloat16;
-
-// GELU, tanh form (Hendrycks & Gimpel 2016), the same function as the GEMM
-// epilogue: 0.5 z (1 + tanh(u)), u = sqrt(2/pi) (z + 0.044715 z^3)
-__device__ __forceinline__ float tanh_hw(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float gelu_f(float z) {
-  const float u = 0.7978845608028654f * fmaf(0.044715f * z, z * z, z);
-  return 0.5f * z * (1.0f + tanh_hw(u));
-}
-__device__ __forceinline__ float gelu_grad(float z) {
-  // d/dz = 0.5 (1 + t) + 0.5 z (1 - t^2) sqrt(2/pi) (1 + 3*0.044715 z^2)
-  const float u = 0.7978845608028654f * fmaf(0.044715f * z, z * z, z);
-  const float t = tanh_hw(u);
-  return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608028654f * fmaf(0.134145f * z, z, 1.0f);
-}
 
 // Network inputs of slab profiles, built from their layer tables (the
 // surrogate's profile_features): out[q][b][0..2] = (eps_r - 1)/eps_scale of
@@ -513,16 +495,6 @@ __global__ void k_gelu_bwd(size_t n, const bf16* __restrict__ dy16, const float*
   }
 }
 
-__device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
-    v[2 * e] = __low2float(h);
-    v[2 * e + 1] = __high2float(h);
-  }
-}
-
 // The GELU backward of rows x C values with the bias gradient: dz = dy gelu'(z)
 // in BF16, dsum[c] += sum of dz[.][c].  Thread (g, y) of a 256-thread block
 // takes channels 8g .. 8g+7 of every (gridDim*ry)-th row (16-byte accesses), so
@@ -785,7 +757,7 @@ __global__ void k_to_bf16(size_t n, const float* __restrict__ x, bf16* __restric
 __global__ void k_gelu_fwd(size_t n, const float* __restrict__ z, bf16* __restrict__ y, bf16* __restrict__ pre) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     if (pre) pre[i] = __float2bfloat16_rn(z[i]);
-    y[i] = __float2bfloat16_rn(gelu_f(z[i]));
+    y[i] = __float2bfloat16_rn(gelu(z[i]));
   }
 }
 

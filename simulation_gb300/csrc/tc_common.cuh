@@ -82,6 +82,22 @@ __device__ __forceinline__ float gelu(float z) {
   const float u = 0.7978845608028654f * fmaf(0.044715f * z, z * z, z);
   return 0.5f * z * (1.0f + tanh_hw(u));
 }
+__device__ __forceinline__ float gelu_grad(float z) {
+  // d/dz = 0.5 (1 + t) + 0.5 z (1 - t^2) sqrt(2/pi) (1 + 3*0.044715 z^2)
+  const float u = 0.7978845608028654f * fmaf(0.044715f * z, z * z, z);
+  const float t = tanh_hw(u);
+  return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608028654f * fmaf(0.134145f * z, z, 1.0f);
+}
+
+__device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
+    v[2 * e] = __low2float(h);
+    v[2 * e + 1] = __high2float(h);
+  }
+}
 
 // one of the warp's lanes, the same for every call while the warp is converged
 __device__ __forceinline__ uint32_t elect_lane() {

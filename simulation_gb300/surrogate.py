@@ -428,12 +428,18 @@ class FNO:
         dFm = torch.empty((M, Bn, 2 * C), dtype=torch.float32, device=dev)
         dF = torch.empty((Bn, C, 2 * M), dtype=BF, device=dev)
         dRbig = torch.empty((M, 2 * C, 2 * C), dtype=torch.float32, device=dev)
+        # the input gradient of a layer leaves its product as the next layer's dz, GELU backward
+        # and bias sum included, where the GEMM has that epilogue
+        chained = C == 128 and N % 128 == 0
         dz = torch.empty((Bn, N, C), dtype=BF, device=dev)
+        dz2 = torch.empty_like(dz) if chained else None
         psi_b = self.psi16.unsqueeze(0).expand(Bn, -1, -1)
         for l in reversed(range(self.L)):
             x, pre, Fm = s["x"][l], s["pre"][l], s["Fm"][l]
             p16, p32 = None if dx16 is None else dx16.data_ptr(), None if dx32 is None else dx32.data_ptr()
-            if wide:
+            if chained and l < self.L - 1:
+                pass  # dz and its sum came with layer l + 1
+            elif wide:
                 _call("fno_gelu_bwd_sum", Bn * N, C, N, None, p32, dh.data_ptr() if p32 is None else None,
                       pre.data_ptr(), dz.data_ptr(), self.g[f"L{l}.b"].data_ptr())
             else:
@@ -450,6 +456,11 @@ class FNO:
             _call("fno_fold_drbig", M, C, dRbig.data_ptr(), self.g[f"L{l}.Rr"].data_ptr(), self.g[f"L{l}.Ri"].data_ptr())
             _call("fno_modes_to_dft", Bn, C, M, dFm.data_ptr(), dF.data_ptr())
             # dx = dz W + Phi^T dF^T in one accumulator (Phi stored [2M][N]: MN-major, shared)
+            if chained and l > 0:
+                gemm(dz, self.w16[f"L{l}.W"], b_mn=True, out=dz2, second=(self.phi16, dF, True, False),
+                     gelu_bwd=(s["pre"][l - 1], self.g[f"L{l - 1}.b"]))
+                dz, dz2 = dz2, dz
+                continue
             nd = torch.empty((Bn, N, C), dtype=torch.float32, device=dev)
             gemm(dz, self.w16[f"L{l}.W"], b_mn=True, out=nd, second=(self.phi16, dF, True, False))
             dx32 = nd

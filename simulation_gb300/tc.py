@@ -24,9 +24,11 @@ def _ld_stride(t: torch.Tensor):
 def gemm(A: torch.Tensor, B: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
          out_dtype=torch.float32, bias: torch.Tensor | None = None, residual: torch.Tensor | None = None,
          alpha: float = 1.0, gelu: bool = False, accumulate: bool = False, pre: torch.Tensor | None = None,
-         status: torch.Tensor | None = None, mn_lbo: int = 0, mn_sbo: int = 0, second=None) -> torch.Tensor:
+         status: torch.Tensor | None = None, mn_lbo: int = 0, mn_sbo: int = 0, second=None,
+         gelu_bwd=None) -> torch.Tensor:
     """``second`` = (A2, B2, a2_mn, b2_mn) adds A2 @ B2' to the accumulator before
-    the epilogue (same output shape)."""
+    the epilogue (same output shape).  ``gelu_bwd`` = (z, dsum): the BF16 result is the
+    product times gelu'(z), and its column sums are added to dsum."""
     for t in (A, B):
         if t.dtype != torch.bfloat16 or not t.is_cuda:
             raise TypeError("A and B must be BF16 CUDA tensors")
@@ -77,5 +79,11 @@ def gemm(A: torch.Tensor, B: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         d.A2, d.lda2, d.stride_a2, d.a2_mn_major = A2.data_ptr(), la2, sa2, int(a2_mn)
         d.B2, d.ldb2, d.stride_b2, d.b2_mn_major = B2.data_ptr(), lb2, sb2, int(b2_mn)
     st = None if status is None else status.data_ptr()
+    if gelu_bwd is not None:
+        z, dsum = gelu_bwd
+        if z.shape != out.shape or z.stride() != out.stride() or z.dtype != torch.bfloat16:
+            raise ValueError("gelu_bwd: z must be BF16 with the output's shape and strides")
+        _lib.call("fdtd_gemm_bf16_gelu_bwd", C.byref(d), z.data_ptr(), dsum.data_ptr(), st, _lib.stream_ptr())
+        return out
     _lib.call("fdtd_gemm_bf16", C.byref(d), st, _lib.stream_ptr())
     return out

@@ -55,3 +55,23 @@ def test_lift_bwd32(cuda_lib, rows, C, cin):
     lim = 1e-6 * (d.abs().T @ x.double().abs() + 1)
     assert bool(((dP.double() - d.T @ x.double()).abs() <= lim).all())
     assert bool(((dp.double() - d.sum(0)).abs() <= 1e-6 * (d.abs().sum(0) + 1)).all())
+
+
+@pytest.mark.parametrize("B,M", [(1, 128), (3, 256), (200, 384)])
+def test_gemm_gelu_bwd(cuda_lib, B, M):
+    """the GELU-gradient epilogue against the plain product and FP64"""
+    from simulation_gb300.tc import gemm
+    g = torch.Generator().manual_seed(M)
+    A = torch.randn((B, M, 128), generator=g).cuda().bfloat16()
+    W = (torch.randn((128, 128), generator=g) / 11).cuda().bfloat16()
+    z = torch.randn((B, M, 128), generator=g).cuda().bfloat16()
+    db = torch.ones(128, device="cuda")
+    out = torch.empty((B, M, 128), dtype=torch.bfloat16, device="cuda")
+    gemm(A, W, b_mn=True, out=out, gelu_bwd=(z, db))
+    y = gemm(A, W, b_mn=True)
+    ref = y.double() * _gelu_grad(z.double())
+    torch.cuda.synchronize()
+    assert float((out.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max())
+    want = 1 + out.double().sum((0, 1))
+    scale = out.double().abs().sum((0, 1)) + 1
+    assert float(((db.double() - want).abs() / scale).max()) <= 1e-6
