@@ -47,11 +47,13 @@ METRIC = "Gcell-updates/s & %HBM peak; surrogate vs FDTD spectra/s at ≤1% L2 e
 UNIT = "Gcell-updates/s"
 WORKLOAD = ("2D TM PML lossy-cylinder benchmark program: 8192x8192, npml=32 grade 0.333, "
             "cylinder r=1000 eps_r=30 sigma=0.3, hard Gaussian Dz source t0=20 spread=6, 2000 steps, FP32")
-# DRAM bytes per cell per fused K=4 pass, from one ncu capture of the fused kernel
-# on the 4096^2 case ((dram__bytes_read.sum + dram__bytes_write.sum) / cells =
-# 1009.4 MB / 16.78 M cells, profiles/k_march_K4_CPL4_full_4096.md); traffic
-# grows in proportion to the cells, so it is scaled to the launch size
-NCU_TRAFFIC_BYTES_PER_CELL_PASS = {4: 60.2}
+# DRAM bytes per cell per fused pass, from one ncu capture each ((dram__bytes_read.sum
+# + dram__bytes_write.sum) / cells): the march's K=4 pass on 4096^2 (1009.4 MB / 16.78 M
+# cells, profiles/k_march_K4_CPL4_full_4096.md) and the chained pass of 8 steps on
+# 6144^2 (profiles/k_chain_4x2_6144.md); traffic grows in proportion to the cells, so it
+# is scaled to the launch size
+NCU_TRAFFIC_BYTES_PER_CELL_PASS = {4: 60.2, 8: 62.1}
+CHAIN_STEPS = 8  # steps per pass that the library takes for the benchmark's grid when left to choose
 
 
 def _peaks():
@@ -279,7 +281,7 @@ def run_ours(args) -> None:
 
     sim = G.benchmark_sim(NX, NY, NPML, GRADE, RGRID, EPSR, SIGMA, ns=NS, device=dev,
                           steps_per_pass=args.spp)
-    spp = args.spp
+    spp = args.spp or CHAIN_STEPS
     cells = NX * NY
     passes_per_run = -(-NS // spp)
     passes_per_run += passes_per_run % 2
@@ -307,15 +309,16 @@ def run_ours(args) -> None:
     ms = max_over_ranks(ms, world, dev)
     value = whole_job_rate(cells * NS * args.steps, world, ms)
 
-    # dominant kernel: time fused passes individually (2 passes of spp steps)
-    ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(10)]
+    # dominant kernel: time fused passes individually (10 passes of spp steps a call, of
+    # which the last also stores ez)
+    ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(5)]
     sim.reset()
     for a, b in ev:
         a.record(st)
-        sim.step(2 * spp, steps_per_pass=spp)
+        sim.step(10 * spp, steps_per_pass=args.spp)
         b.record(st)
     torch.cuda.synchronize()
-    pass_ms = statistics.median(a.elapsed_time(b) for a, b in ev) / 2
+    pass_ms = statistics.median(a.elapsed_time(b) for a, b in ev) / 10
     peak, peak_kind = _peaks()
     algo_bytes = BYTES_PER_CELL_UPDATE * cells * spp
     achieved = algo_bytes / (pass_ms / 1e3) / 1e9
@@ -359,7 +362,7 @@ def run_ours(args) -> None:
                 "hbm_frac_algorithmic": value * BYTES_PER_CELL_UPDATE / peak,
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                             "kernel": f"k_march<K={spp}> (one fused pass = {spp} time steps)",
+                             "kernel": f"{'k_march' if args.spp else 'k_chain'} (one fused pass = {spp} time steps)",
                              "algorithmic_bytes_per_launch": algo_bytes, "launch_ms": pass_ms},
                 "e2e": e2e, "cpu_baseline": cpu, "clocks": clocks,
                 "gpu_launches": passes_per_run * args.steps, "secondary_workloads": extra}
@@ -383,8 +386,9 @@ def run_secondary(args, st, world) -> dict:
 
 def _bench_tfsf_dft(st, n: int = 2048, steps: int = 400) -> dict:
     """The fd2d_3_4 program (TF/SF plane wave, lossy cylinder, PML, 3-frequency
-    full-field DFT) at n^2 through fdtd2d_step_n: fused passes of 4 steps (the
-    incident line advanced ahead in one launch per 64 steps), timed beside
+    full-field DFT) at n^2 through fdtd2d_step_n: chained passes of 8 steps (the
+    incident line advanced ahead in one launch per 64 steps, the DFT added up
+    from 16 steps' record of ez), timed beside
     the same step as three launches (one-step calls) and the nine
     per-function launches of the reference's loop."""
     import torch
@@ -414,13 +418,14 @@ def _bench_tfsf_dft(st, n: int = 2048, steps: int = 400) -> dict:
         torch.cuda.synchronize()
         out[f"{name}_Gcell_updates_per_s"] = n * n * steps / (e0.elapsed_time(e1) / 1e3) / 1e9
     nf = 3
-    # fused pass of K = 4 steps: the 60 field bytes of the lossy PML pass
-    # plus the DFT accumulators read and written once (16 bytes per frequency)
-    bpc = (60 + 16 * nf) / 4
+    # chained pass of 8 steps: the 56 field bytes of the lossy PML pass (ez is
+    # stored by the last only); the record of ez written and read (8 bytes a
+    # step); the DFT accumulators read and written once in 16 steps
+    bpc = 56 / 8 + 8 + 16 * nf / 16
     out["fused_bytes_per_cell_update"] = bpc
     out["fused_GBps_algorithmic"] = out["fused_Gcell_updates_per_s"] * bpc
     out["grid"] = [n, n]
-    out["launches_per_step"] = {"fused": 0.25 + 1 / 64, "three_launch": 3, "per_function": 9}
+    out["launches_per_step"] = {"fused": 1 / 8 + 1 / 16 + 1 / 64, "three_launch": 3, "per_function": 9}
     del sim, plain
     return out
 
@@ -591,14 +596,13 @@ def _bench_adjoint(st) -> dict:
     torch.cuda.synchronize()
     fwd, rev = ev[0].elapsed_time(ev[1]), ev[1].elapsed_time(ev[2])
     cu = pr.nx * pr.ny * pr.ns
-    # algorithmic bytes per cell and time step of this problem (lossless box: no iz, nbz):
-    # forward, passes of 2 steps: dz, hx, hy, ihx, ihy, naz in and dz, ez, hx, hy,
-    # ihx, ihy out once per pass (48 B / 2); reverse: the recompute pass the same
-    # plus the recorded dz, hx, hy of every step (12 B), and the two-step
-    # reverse kernel: both states before the steps (2 x 12 B), naz, the 5
-    # adjoints in and out once per 2 steps ((24 + 4 + 40) B / 2)
-    fwd_b = 48 / 2
-    rev_b = 48 / 2 + 12 + (24 + 4 + 40) / 2
+    # algorithmic bytes per cell and time step of this problem (lossless box: no iz, nbz),
+    # which runs on the chip: dz, hx, hy, ihx, ihy and naz in, the five out once per
+    # segment; the reverse runs the segment again and undoes it (twice that), with dz
+    # of the box written and read every step
+    box = pr.box[2] * pr.box[3] / (pr.nx * pr.ny)
+    fwd_b = 44 / pr.cp
+    rev_b = 2 * 44 / pr.cp + 8 * box
     res = {"forward_ms": fwd, "reverse_ms": rev, "forward_Gcell_updates_per_s": cu / fwd / 1e6,
            "reverse_Gcell_updates_per_s": cu / rev / 1e6, "checkpoint": pr.cp, "cuda_graphs": pr.use_graphs,
            "bytes_per_cell_update": {"forward": fwd_b, "reverse": rev_b},
@@ -842,7 +846,7 @@ def main():
     ap.add_argument("--steps", type=int, default=3)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
-    ap.add_argument("--spp", type=int, default=4, help="time steps per fused pass (1..4)")
+    ap.add_argument("--spp", type=int, default=0, help="time steps per fused pass (1..4; 0: the library's choice)")
     ap.add_argument("--grid", type=int, default=8192, help="grid edge (profiling runs use a smaller case)")
     ap.add_argument("--ns", type=int, default=2000, help="time steps per bench step")
     ap.add_argument("--no-e2e", action="store_true")
