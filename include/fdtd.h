@@ -395,10 +395,10 @@ int fno_gelu_bwd(long long n, const void* dy16, const float* dy32, const void* p
 int fno_gelu_bwd_sum(long long rows, int C, int N, const void* dy16, const float* dy32, const float* dh, const void* pre,
                      void* dz, float* dsum, fdtd_stream_t stream);
 int fno_meanpool(int B, int N, int C, const void* x, void* h, fdtd_stream_t stream);
-/* one spectral layer: z = x W^T + psi G^T + bias, x' = GELU(z).  x BF16 [B][N][K1] (K1 = 128, or 64 for packed
+/* one spectral layer: z = x W^T + psi G^T + bias, x' = GELU(z).  x BF16 [B][N][K1] (K1 = 128, or 16 for packed
  * inputs), W [C][K1], psi [N][2M], Gm [M][B][2C] (the mode products, BF16).  Either x_out [B][N][C]
  * and Fm_out [M][B][2C] (x' and its DFT, ready for the next layer's mode product) or, for the last layer,
- * h_out [B][C] (the mean of x' over positions); pre: z, optional.  C = 128, M = 32, N >= 128 a power of two,
+ * h_out [B][C] (the mean of x' over positions); pre: z, optional (K1 = 128).  C = 128, M = 32, N >= 128 a power of two,
  * B <= 65535.  The DFT uses psi, the inverse's rows: cos and sin times 2/N (1/N for mode 0) */
 int fno_layer_fwd(int B, int N, int C, int M, int K1, const void* x, const void* W, const float* bias,
                   const void* psi, const void* Gm, void* x_out, void* Fm_out, void* h_out, void* pre,

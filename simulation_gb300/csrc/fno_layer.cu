@@ -32,9 +32,10 @@
 //
 // 4096 samples of 2048 positions: 690 us a middle layer, 4.3 GB at 6.2 TB/s
 // (with MMAs, GELU and stores to shared memory cut out one by one it stays
-// above 650); 630 the first (packed inputs), 510 the last.  As separate
+// above 650); 608 the first (packed inputs; 630 from rows padded to 64), 510 the
+// last.  As separate
 // kernels (DFT, permutes, pointwise, mean pool) the network took 6.1 ms, now
-// 3.0; one sample alone 142 us instead of 171, so there is no size below
+// 2.85; one sample alone 142 us instead of 171, so there is no size below
 // which the separate form is kept for this shape.  With one group of eight
 // warps 3.5 ms, sixteen on one tile 3.4, issuing the MMAs from a converged warp
 // 3.3, Psi for Phi and alternating groups 3.0.
@@ -89,11 +90,14 @@ __device__ __forceinline__ uint32_t bf16x2(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-template <int KB1, bool LAST, bool PRE>
+// K1: input channels, 128, or 16 for packed inputs
+template <int K1, bool LAST, bool PRE>
 __global__ void __launch_bounds__(layer_threads(LAST), 1)
     k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
             const __grid_constant__ CUtensorMap tmPsi, const __grid_constant__ CUtensorMap tmG,
             const __grid_constant__ CUtensorMap tmOut, const LayerArgs a) {
+  // 64 channels (128 bytes) of 128 rows a block of x and of W, or all 16 (32 bytes)
+  constexpr int XB = K1 == 16 ? 1 : K1 / 64, X_BLOCK = K1 == 16 ? 4096 : 16384;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sm = smem_u32(base);
@@ -145,8 +149,8 @@ __global__ void __launch_bounds__(layer_threads(LAST), 1)
   if (warp == W_TMA) {
     // ------------------------------------------------ x, Psi and G
     if (lane == 0) {
-      mbar_expect_tx(bar(WFULL), KB1 * 16384);
-      for (int k = 0; k < KB1; ++k) tma_load_3d(sm + k * 16384, &tmW, 64 * k, 0, 0, bar(WFULL));
+      mbar_expect_tx(bar(WFULL), XB * X_BLOCK);
+      for (int k = 0; k < XB; ++k) tma_load_3d(sm + k * X_BLOCK, &tmW, 64 * k, 0, 0, bar(WFULL));
       int i = 0, np = 0, ng = 0;  // x tiles, Psi tiles and G loaded
       for (int b = blockIdx.x; b < a.B && ok; b += gridDim.x)
         for (int t = 0; t < tiles && ok; ++t) {
@@ -154,8 +158,8 @@ __global__ void __launch_bounds__(layer_threads(LAST), 1)
           if (i >= 2) wait(XEMPTY + p, (i >> 1) - 1);
           if (!ok) break;
           const uint32_t dst = sm + OFF_X + p * X_STAGE;
-          mbar_expect_tx(bar(XFULL + p), KB1 * 16384);
-          for (int k = 0; k < KB1; ++k) tma_load_3d(dst + k * 16384, &tmX, 64 * k, t * LT, b, bar(XFULL + p));
+          mbar_expect_tx(bar(XFULL + p), XB * X_BLOCK);
+          for (int k = 0; k < XB; ++k) tma_load_3d(dst + k * X_BLOCK, &tmX, 64 * k, t * LT, b, bar(XFULL + p));
           ++i;
           if (t == 0) {
             if (ng >= 1) wait(GEMPTY, ng - 1);
@@ -219,12 +223,16 @@ __global__ void __launch_bounds__(layer_threads(LAST), 1)
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t sx = sm + OFF_X + p * X_STAGE, sp = sm + OFF_PSI + p3 * PSI_STAGE, dacc = tmem + p * LC;
+        if constexpr (K1 == 16) {
+          mma_bf16(lead, dacc, smem_desc32(sx), smem_desc32(sm), id_w, 0u);
+        } else {
 #pragma unroll
-        for (int k = 0; k < KB1; ++k)
+          for (int k = 0; k < XB; ++k)
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_bf16(lead, dacc, smem_desc(sx + k * 16384 + kk * 32, 16, 1024),
+            for (int kk = 0; kk < 4; ++kk)
+              mma_bf16(lead, dacc, smem_desc(sx + k * 16384 + kk * 32, 16, 1024),
                      smem_desc(sm + k * 16384 + kk * 32, 16, 1024), id_w, (k > 0 || kk > 0) ? 1u : 0u);
+        }
         mma_commit(lead, bar(XEMPTY + p));
         if (t == 0) wait_warp(GFULL, s);
         wait_warp(PFULL + p3, i / 3);
@@ -391,9 +399,9 @@ __global__ void __launch_bounds__(layer_threads(LAST), 1)
   }
 }
 
-template <int KB1, bool LAST, bool PRE>
+template <int K1, bool LAST, bool PRE>
 int launch_layer(const CUtensorMap (&tm)[5], const LayerArgs& a, cudaStream_t st) {
-  auto kern = k_layer<KB1, LAST, PRE>;
+  auto kern = k_layer<K1, LAST, PRE>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LAYER_SMEM);
   if (e != cudaSuccess) {
     fdtd_host::note_cuda_error(e);
@@ -415,13 +423,15 @@ extern "C" int fno_layer_fwd(int B, int N, int C, int M, int K1, const void* x, 
   using namespace fdtd;
   if (!x || !W || !bias || !psi || !Gm) return FDTD_ERR_NULL;
   if (!x_out != !Fm_out || !x_out == !h_out) return FDTD_ERR_ARG;  // (x_out, Fm_out) or h_out
-  if (B < 1 || B > 65535 || N < LT || (N & (N - 1)) || C != LC || 2 * M != LM2 || (K1 != 64 && K1 != 128))
+  if (B < 1 || B > 65535 || N < LT || (N & (N - 1)) || C != LC || 2 * M != LM2 || (K1 != 16 && K1 != 128))
     return FDTD_ERR_SIZE;
+  if (pre && K1 != 128) return FDTD_ERR_ARG;
   for (const void* p : {x, W, psi, Gm, (const void*)x_out, (const void*)pre})
     if ((uintptr_t)p & 15u) return FDTD_ERR_ALIGN;
   CUtensorMap tm[5];
-  int rc = make_map(&tm[0], x, K1, N, B, K1, (uint64_t)N * K1, 64, LT);
-  if (!rc) rc = make_map(&tm[1], W, K1, LC, 1, K1, (uint64_t)LC * K1, 64, LC);
+  const int box = K1 == 16 ? 16 : 64;
+  int rc = make_map(&tm[0], x, K1, N, B, K1, (uint64_t)N * K1, box, LT);
+  if (!rc) rc = make_map(&tm[1], W, K1, LC, 1, K1, (uint64_t)LC * K1, box, LC);
   if (!rc) rc = make_map(&tm[2], psi, LM2, N, 1, LM2, (uint64_t)N * LM2, 64, LT);
   if (!rc) rc = make_map(&tm[3], Gm, 2 * LC, B, M, 2 * LC, (uint64_t)B * 2 * LC, 64, 1, 32);
   if (!rc && x_out) rc = make_map(&tm[4], x_out, LC, N, B, LC, (uint64_t)N * LC, 64, LT);
@@ -429,10 +439,7 @@ extern "C" int fno_layer_fwd(int B, int N, int C, int M, int K1, const void* x, 
   if (!x_out) tm[4] = tm[0];  // not used by the last layer
   const LayerArgs a{B, N, bias, (__nv_bfloat16*)Fm_out, (__nv_bfloat16*)h_out, (__nv_bfloat16*)pre, status};
   cudaStream_t st = (cudaStream_t)stream;
-  if (pre) {
-    if (K1 == 64) return h_out ? launch_layer<1, true, true>(tm, a, st) : launch_layer<1, false, true>(tm, a, st);
-    return h_out ? launch_layer<2, true, true>(tm, a, st) : launch_layer<2, false, true>(tm, a, st);
-  }
-  if (K1 == 64) return h_out ? launch_layer<1, true, false>(tm, a, st) : launch_layer<1, false, false>(tm, a, st);
-  return h_out ? launch_layer<2, true, false>(tm, a, st) : launch_layer<2, false, false>(tm, a, st);
+  if (K1 == 16) return h_out ? launch_layer<16, true, false>(tm, a, st) : launch_layer<16, false, false>(tm, a, st);
+  if (pre) return h_out ? launch_layer<128, true, true>(tm, a, st) : launch_layer<128, false, true>(tm, a, st);
+  return h_out ? launch_layer<128, true, false>(tm, a, st) : launch_layer<128, false, false>(tm, a, st);
 }

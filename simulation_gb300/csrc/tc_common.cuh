@@ -65,6 +65,17 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return d;
 }
 
+// the same for rows of 32 bytes (16 BF16 along K, 32B swizzle): 8 rows are 256 bytes
+__device__ __forceinline__ uint64_t smem_desc32(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(256 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)6 << 61;
+  return d;
+}
+
 // instruction descriptor, kind::f16: BF16 A and B, FP32 accumulator, M x N
 __host__ __device__ constexpr uint32_t instr_desc(int m, int n, int a_mn, int b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
@@ -161,7 +172,7 @@ inline int get_encode(PFN_cuTensorMapEncodeTiled_v12000* out) {
   return FDTD_OK;
 }
 
-// 3D tensor map over a BF16 operand: dims {inner, outer, batch}, 128-byte swizzle
+// 3D tensor map over a BF16 operand: dims {inner, outer, batch}, 128-byte swizzle, or 32-byte for a box of 16
 inline int make_map(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t outer, uint64_t batch,
                     uint64_t ld_elems, uint64_t stride_elems, uint32_t box_inner, uint32_t box_outer,
                     uint32_t box_batch = 1) {
@@ -173,7 +184,8 @@ inline int make_map(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t 
   cuuint32_t box[3] = {box_inner, box_outer, box_batch};
   cuuint32_t es[3] = {1, 1, 1};
   const CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            box_inner == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? FDTD_OK : FDTD_ERR_ARG;
 }

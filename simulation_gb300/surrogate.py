@@ -251,6 +251,7 @@ class FNO:
         _call("fno_small_matmul", 1, C, KPW, C, self.p["L0.W"].data_ptr(), Pw.data_ptr(), w0.data_ptr())
         self.w0f16 = torch.empty((C, KPW), dtype=BF, device=self.dev)
         _call("fno_to_bf16", w0.numel(), w0.data_ptr(), self.w0f16.data_ptr())
+        self.w0k16 = self.w0f16[:, :KIN].contiguous()  # the fused layer's, without the padding
         rr = torch.empty((M, C, KIN), dtype=torch.float32, device=self.dev)
         ri = torch.empty((M, C, KIN), dtype=torch.float32, device=self.dev)
         _call("fno_small_matmul", M, C, KIN, C, self.p["L0.Rr"].data_ptr(), Pp.data_ptr(), rr.data_ptr())
@@ -258,8 +259,9 @@ class FNO:
         self.rbig0f = torch.empty((M, 2 * C, 2 * KIN), dtype=BF, device=self.dev)
         _call("fno_build_rbig_rect", M, C, KIN, rr.data_ptr(), ri.data_ptr(), self.rbig0f.data_ptr())
 
-    def _first_modes_folded(self, inp: torch.Tensor):
-        """The packed inputs [B][N][KPW] and their mode coefficients [M][B][2 KIN]."""
+    def _first_modes_folded(self, inp: torch.Tensor, padded: bool):
+        """The packed inputs [B][N][KIN] ([B][N][KPW] with ``padded``) and their mode
+        coefficients [M][B][2 KIN]."""
         Bn, N, C, M, KIN = inp.shape[0], self.N, self.C, self.M, self.KIN
         dev = self.dev
         # the 64-wide operand lives per (stream, batch size): its zero padding is
@@ -267,12 +269,12 @@ class FNO:
         key = (torch.cuda.current_stream(dev).cuda_stream, Bn)
         if not hasattr(self, "_packed"):
             self._packed = {}
-        inp16 = self._packed.get(key)
+        inp16 = self._packed.get(key) if padded else torch.empty((Bn, N, KIN), dtype=BF, device=dev)
         if inp16 is None:
             inp16 = torch.zeros((Bn, N, self.KPW), dtype=BF, device=dev)
             self._packed[key] = inp16
         inpT = torch.empty((N, Bn * KIN), dtype=BF, device=dev)  # position-major copy
-        _call("fno_pack_inputs", Bn, N, self.cin, self.KPW, 0, inp.data_ptr(), inp16.data_ptr(), inpT.data_ptr())
+        _call("fno_pack_inputs", Bn, N, self.cin, inp16.shape[2], 0, inp.data_ptr(), inp16.data_ptr(), inpT.data_ptr())
         # the DFT of every sample's 16 channels in one product: F[(b, c)][j] = sum_n inpT[n][(b, c)] Phi[j][n]
         F = torch.empty((Bn, KIN, 2 * M), dtype=torch.float32, device=dev)
         gemm(inpT, self.phi16, a_mn=True, out=F.view(Bn * KIN, 2 * M))
@@ -283,7 +285,7 @@ class FNO:
     def _first_layer_folded(self, inp: torch.Tensor) -> torch.Tensor:
         """x1 of the first spectral layer straight from the packed inputs."""
         Bn, N, C, M, dev = inp.shape[0], self.N, self.C, self.M, self.dev
-        inp16, Fm = self._first_modes_folded(inp)
+        inp16, Fm = self._first_modes_folded(inp, True)
         Gm = torch.empty((M, Bn, 2 * C), dtype=torch.float32, device=dev)
         gemm(Fm, self.rbig0f, out=Gm)
         G = torch.empty((Bn, C, 2 * M), dtype=BF, device=dev)
@@ -303,7 +305,7 @@ class FNO:
         Bn, N, C, M, dev = inp.shape[0], self.N, self.C, self.M, self.dev
         folded = saved is None and self.fold and self.cin + 1 <= self.KIN
         if folded:
-            x, Fm = self._first_modes_folded(inp)
+            x, Fm = self._first_modes_folded(inp, False)
         else:
             x = torch.empty((Bn, N, C), dtype=BF, device=dev)
             _call("fno_lift_fwd", Bn * N, C, self.cin, inp.data_ptr(), self.p["P"].data_ptr(),
@@ -316,7 +318,7 @@ class FNO:
         for l in range(self.L):
             first, last = folded and l == 0, l == self.L - 1
             gemm(Fm, self.rbig0f if first else self.rbig[l], out=Gm)
-            w = self.w0f16 if first else self.w16[f"L{l}.W"]
+            w = self.w0k16 if first else self.w16[f"L{l}.W"]
             pre = None
             if saved is not None:
                 pre = torch.empty((Bn, N, C), dtype=BF, device=dev)

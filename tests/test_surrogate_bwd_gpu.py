@@ -1,4 +1,4 @@
-"""The fused backward kernels of the surrogate against plain FP32/FP64 torch:
+"""The input packing and the fused backward kernels of the surrogate against plain FP32/FP64 torch:
 GELU backward with the bias sum from each of its three sources, and the lift's
 backward from FP32 gradients, at row counts and widths off the blocks' shape."""
 import numpy as np
@@ -75,3 +75,21 @@ def test_gemm_gelu_bwd(cuda_lib, B, M):
     want = 1 + out.double().sum((0, 1))
     scale = out.double().abs().sum((0, 1)) + 1
     assert float(((db.double() - want).abs() / scale).max()) <= 1e-6
+
+
+@pytest.mark.parametrize("B,N,cin,ldo,pad", [(1, 1, 1, 16, 1), (3, 33, 6, 64, 0), (8, 32, 15, 64, 1), (41, 100, 6, 24, 1)])
+def test_pack_inputs(cuda_lib, B, N, cin, ldo, pad):
+    """rows (inputs, 1, zeros) in both layouts, exact; columns past 16 kept unless padded"""
+    from simulation_gb300 import surrogate as S
+    g = torch.Generator().manual_seed(N)
+    x = torch.randn((B, N, cin), generator=g).cuda()
+    out = torch.full((B, N, ldo), 5.0, dtype=torch.bfloat16, device="cuda")
+    out_t = torch.full((N, B, 16), 5.0, dtype=torch.bfloat16, device="cuda")
+    S._call("fno_pack_inputs", B, N, cin, ldo, pad, x.data_ptr(), out.data_ptr(), out_t.data_ptr())
+    want = torch.zeros((B, N, ldo), dtype=torch.bfloat16, device="cuda")
+    want[..., :cin] = x.bfloat16()
+    want[..., cin] = 1.0
+    if not pad:
+        want[..., 16:] = 5.0
+    assert torch.equal(out, want)
+    assert torch.equal(out_t, want[..., :16].transpose(0, 1))

@@ -35,6 +35,6 @@ def test_layer_refuses(cuda_lib):
     p = torch.zeros(64, device="cuda").data_ptr()
     args = lambda **k: [{**dict(B=1, N=128, C=128, M=32, K1=128), **k}[q] for q in ("B", "N", "C", "M", "K1")]  # noqa: E731
     f = lambda a, xo=p, fm=p, h=None: _lib.lib().fno_layer_fwd(*a, p, p, p, p, p, xo, fm, h, None, None, None)  # noqa: E731
-    for bad in (dict(N=100), dict(N=384), dict(N=64), dict(C=64), dict(M=16), dict(K1=96), dict(B=0), dict(B=65536)):
+    for bad in (dict(N=100), dict(N=384), dict(N=64), dict(C=64), dict(M=16), dict(K1=96), dict(K1=64), dict(B=0), dict(B=65536)):
         assert f(args(**bad)) == -2
     assert f(args(), p, None) != 0 and f(args(), p, p, p) != 0 and f(args(), p + 4) != 0
