@@ -49,6 +49,54 @@ __global__ void k_profile_features(int n, const int* __restrict__ run_idx, const
   }
 }
 
+// The same, a block per profile: the quotients once per layer (in double, of which
+// the chip does little: forming them per bin took 355 us for 4096 profiles of 2048
+// bins), the cells' values through shared memory, contiguous stores: 34 us.  A cell
+// always belongs to the same thread, so that later layers replace earlier ones.
+constexpr int kFeatMaxBins = 2800;  // 2 x (2 nbins + 1) floats of shared memory beside the 4 KB of layers
+__global__ void __launch_bounds__(256)
+    k_profile_features_block(const int* __restrict__ run_idx, const int* __restrict__ layer_off,
+                             const int* __restrict__ layer_start, const int* __restrict__ layer_end,
+                             const double* __restrict__ epsr, const double* __restrict__ sigma, int nbins,
+                             double eps_scale, double sig_scale, float* __restrict__ out) {
+  extern __shared__ float feat[];  // [2][2 nbins + 1]: cells -1 .. 2 nbins - 1
+  __shared__ int ls[256], le[256];
+  __shared__ float ve[256], vg[256];
+  const int cells = 2 * nbins + 1, tid = threadIdx.x;
+  const int r = run_idx ? run_idx[blockIdx.x] : blockIdx.x;
+  const int l0 = layer_off[r], l1 = layer_off[r + 1];
+  float* fe = feat;
+  float* fg = feat + cells;
+  for (int x = tid; x < cells; x += 256) fe[x] = fg[x] = 0.f;
+  for (int base = l0; base < l1; base += 256) {
+    const int m = min(256, l1 - base);
+    __syncthreads();
+    if (tid < m) {
+      ls[tid] = max(layer_start[base + tid], -1) + 1;
+      le[tid] = min(layer_end[base + tid], 2 * nbins) + 1;
+      ve[tid] = (float)((epsr[base + tid] - 1.0) / eps_scale);
+      vg[tid] = (float)(sigma[base + tid] / sig_scale);
+    }
+    __syncthreads();
+    for (int l = 0; l < m; ++l) {
+      const int lo = ls[l], hi = le[l];
+      const float e = ve[l], g = vg[l];
+      for (int x = lo + ((tid - lo) & 255); x < hi; x += 256) {
+        fe[x] = e;
+        fg[x] = g;
+      }
+    }
+  }
+  __syncthreads();
+  float2* o = reinterpret_cast<float2*>(out + (size_t)blockIdx.x * nbins * 6);
+  for (int x = tid; x < 3 * nbins; x += 256) {  // pairs (0, 1), (2, 3), (4, 5) of a bin
+    const int b = x / 3, k = x - 3 * b;
+    const float* c = fe + 2 * b;
+    const float* d = fg + 2 * b;
+    o[x] = k == 0 ? make_float2(c[0], c[1]) : k == 1 ? make_float2(c[2], d[0]) : make_float2(d[1], d[2]);
+  }
+}
+
 inline dim3 grid1(size_t n, int t = 256) {
   size_t b = (n + t - 1) / t;
   if (b > 152 * 64) b = 152 * 64;
@@ -837,6 +885,11 @@ int fno_profile_features(int n, const int* run_idx, const int* layer_off, const 
   if (!layer_off || !layer_start || !layer_end || !epsr || !sigma || !out) return FDTD_ERR_NULL;
   if (n < 1 || nbins < 1 || !(eps_scale > 0) || !(sig_scale > 0)) return FDTD_ERR_SIZE;
   if ((uintptr_t)out & 7) return FDTD_ERR_ALIGN;
+  if (nbins <= fdtd::kFeatMaxBins) {
+    fdtd::k_profile_features_block<<<(unsigned)n, 256, 2 * (2 * nbins + 1) * sizeof(float), (cudaStream_t)stream>>>(
+        run_idx, layer_off, layer_start, layer_end, epsr, sigma, nbins, eps_scale, sig_scale, out);
+    return fdtd_host::check_launch();
+  }
   FNO_LAUNCH(fdtd::k_profile_features, fdtd::grid1((size_t)n * nbins), 256, n, run_idx, layer_off, layer_start,
              layer_end, epsr, sigma, nbins, eps_scale, sig_scale, out);
 }

@@ -93,3 +93,30 @@ def test_pack_inputs(cuda_lib, B, N, cin, ldo, pad):
         want[..., 16:] = 5.0
     assert torch.equal(out, want)
     assert torch.equal(out_t, want[..., :16].transpose(0, 1))
+
+
+@pytest.mark.parametrize("nbins", [1, 100, 2048, 2800, 2801, 3000])
+def test_profile_features(cuda_lib, nbins):
+    """overlapping, empty, clipped and many layers: the last that holds a cell counts"""
+    from simulation_gb300 import surrogate as S
+    rng = np.random.default_rng(nbins)
+    counts = np.array([0, 1, 5, 300, 2])
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    st = rng.integers(0, 2 * nbins + 20, off[-1]).astype(np.int32)
+    en = (st + rng.integers(-3, nbins + 3, off[-1])).astype(np.int32)
+    ep, sg = rng.uniform(1, 9, off[-1]), rng.uniform(0, 0.05, off[-1])
+    idx = np.array([3, 0, 4, 2, 1, 3], dtype=np.int32)
+    want = np.zeros((idx.size, nbins, 6), dtype=np.float32)
+    for q, r in enumerate(idx):
+        e, s = np.zeros(2 * nbins + 1), np.zeros(2 * nbins + 1)  # cells -1 .. 2 nbins - 1
+        for l in range(off[r], off[r + 1]):
+            lo, hi = min(st[l], 2 * nbins) + 1, max(min(en[l], 2 * nbins) + 1, 0)  # no negative slice ends
+            e[lo:hi] = (ep[l] - 1.0) / S.EPS_SCALE
+            s[lo:hi] = sg[l] / S.SIG_SCALE
+        for j in range(3):
+            want[q, :, j], want[q, :, 3 + j] = e[j:j + 2 * nbins:2], s[j:j + 2 * nbins:2]
+    dev = [torch.as_tensor(a).cuda() for a in (idx, off, st, en, ep, sg)]
+    out = torch.empty((idx.size, nbins, 6), device="cuda")
+    S._call("fno_profile_features", idx.size, *(t.data_ptr() for t in dev), nbins, S.EPS_SCALE, S.SIG_SCALE,
+            out.data_ptr())
+    assert torch.equal(out.cpu(), torch.from_numpy(want))
