@@ -443,7 +443,12 @@ __global__ void __launch_bounds__(halo_max_threads(FORM, CPT)) k_fd1d_halo(const
   else if (lo_kind) time_loop(std::integral_constant<int, 1>{});
   else if (hi_kind) time_loop(std::integral_constant<int, 2>{});
   else time_loop(std::integral_constant<int, 0>{});
-  if (C > 1) cgx::this_cluster().sync();  // no block leaves while a neighbour may read its buffers
+  // Results go where the fields came from, and a warp's halo lanes hold cells that
+  // its neighbour stores.  A call of no more steps than H has no exchange, so this
+  // barrier alone orders every warp's loads before any warp's stores; between blocks
+  // it also keeps a block from leaving while a neighbour may read its buffers.
+  if (C > 1) cgx::this_cluster().sync();
+  else __syncthreads();
 
   // ---- results
   if (owned) {

@@ -43,3 +43,29 @@ def test_split_calls_and_initial_fields(cuda_lib, nx):
     torch.cuda.synchronize()
     for k in ("ex", "hy", "dx", "ix", "sx", "bc", "r_pt", "i_pt", "r_pr", "i_pr"):
         assert torch.equal(getattr(a, k), getattr(b, k)), f"nx={nx} {k}"
+
+
+@pytest.mark.parametrize("nx,form,nf", [(513, "cb", 0), (700, "cacb", 0), (1184, "dform", 0), (800, "debye", 0),
+                                        (66, "cb", 3), (300, "debye", 3), (688, "dform", 3), (130, "cb", 8)])
+def test_many_calls_shorter_than_the_exchange_period(cuda_lib, nx, form, nf):
+    """A call of 1 to 16 steps on a line that one block of several warps holds ends before
+    the warps' first exchange: its stores must still come after every warp's loads.  Several
+    hundred calls in a row, so that a warp that starts from later values shows."""
+    from simulation_gb300 import fd1d as G
+    kw = dict(src_kind="soft", src_k=nx // 3, wave=("gauss", 30, 8.0), **_coeffs(nx, form))
+    if nf:
+        kw.update(freq=np.linspace(5e7, 9e8, nf), full_dft=True, probes=(1, nx // 2, nx - 2))
+    a, b = G.Sim1D(nx, form, **kw), G.Sim1D(nx, form, **kw)
+    init = torch.sin(torch.arange(nx, dtype=torch.float32, device="cuda") * 0.1)
+    for s in (a, b):
+        s.ex.copy_(init)
+        s.hy.copy_(init.flip(0))
+    total = 0
+    for n in (1, 2, 3, 5, 8, 13, 16) * 40:
+        a.step(n)
+        total += n
+    b.step_per_function(total)
+    torch.cuda.synchronize()
+    for k in ("ex", "hy", "dx", "ix", "sx", "bc", "r_pt", "i_pt", "r_pr", "i_pr"):
+        x, y = getattr(a, k), getattr(b, k)
+        assert x is None or torch.equal(x, y), f"nx={nx} {form} nf={nf}: {k}"
