@@ -280,6 +280,12 @@ typedef struct {
 } fdtd2d_adjoint_params;
 
 size_t fdtd2d_tm_adjoint_workspace_size(const fdtd2d_params* p, const fdtd2d_adjoint_params* a);
+/* Byte offset in the workspace of two device status words (int), the forward's and
+ * the reverse's, each cleared as its half starts; 0 for arguments that the calls
+ * refuse.  On grids that run on the chip the kernels' blocks wait on one another, for
+ * a bounded time: a wait that runs out sets FDTD_STATUS_TIMEOUT there, and trace and J,
+ * or the gradients (of this reverse, and of any from such a forward), are NaN. */
+size_t fdtd2d_tm_adjoint_status_offset(const fdtd2d_params* p, const fdtd2d_adjoint_params* a);
 int fdtd2d_tm_adjoint_forward(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* trace, double* J,
                               void* workspace, size_t workspace_bytes, fdtd_stream_t stream);
 int fdtd2d_tm_adjoint_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz,

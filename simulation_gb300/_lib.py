@@ -136,6 +136,7 @@ _SIGS = {
     "fdtd2d_adjoint_step": ([C.c_int, C.POINTER(Params2D), C.POINTER(Fields2D), C.POINTER(Fields2D), F, C.c_int,
                              C.c_int, C.c_float, Box2D, F, F, P], C.c_int),
     "fdtd2d_tm_adjoint_workspace_size": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D)], C.c_size_t),
+    "fdtd2d_tm_adjoint_status_offset": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D)], C.c_size_t),
     "fdtd2d_tm_adjoint_forward": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D), F, P, P, C.c_size_t, P],
                                   C.c_int),
     "fdtd2d_tm_adjoint_forward_rec": ([C.POINTER(Params2D), C.POINTER(AdjointParams2D), F, P, P, C.c_size_t, P],

@@ -73,6 +73,9 @@ class AdjointProblem:
         if n == 0:
             raise ValueError("fdtd2d_tm_adjoint_workspace_size rejected the problem")
         self.ws = torch.empty(n, dtype=torch.uint8, device=self.device)
+        off = _lib.lib().fdtd2d_tm_adjoint_status_offset(C.byref(self.sim._p), C.byref(self.ap))
+        self.status = self.ws[off:off + 8].view(torch.int32)  # of the last forward and of the last reverse
+        self.status.zero_()
         self.J = None
         # the loops are static for a problem (pointers, steps, segment order):
         # from the second call on, each sweep replays a CUDA graph of itself
@@ -121,7 +124,17 @@ class AdjointProblem:
         self._run("forward", body)
         self.sim.t = self.ns
         self.J = float(self.J_dev.item())
+        if self.J != self.J:
+            self.check()
         return self.J
+
+    def check(self) -> None:
+        """Raise FdtdError if a wait between the kernels' blocks ran out in the last
+        forward or reverse, whose results are then NaN (host sync).  ``forward``
+        checks itself."""
+        v = int(self.status[0].item()) | int(self.status[1].item())
+        if v:
+            raise _lib.FdtdError(_lib.lib().fdtd_status_to_error(v), f"adjoint status word {v:#x}")
 
     # ------------------------------------------------------------ reverse
     def gradient_naz(self) -> torch.Tensor:

@@ -27,6 +27,9 @@
 // 5.4), 10.5 with the forward's record, against 38.5 streaming, whose reverse
 // reads two recorded states and the adjoints of every tile from L2 in each launch
 // (33 us for two steps; 7.2 here, exchanges included).
+// The on-chip launches' waits between blocks are bounded.  One that runs out sets
+// FDTD_STATUS_TIMEOUT in its half's status word in the workspace, and the half's
+// results are then NaN (k_poison): the call has long returned FDTD_OK.
 // Results do not depend on the checkpoint interval or on the overlap: every
 // recorded state is bitwise the forward's, and each reverse step does the
 // same per-cell arithmetic (fdtd2d_adjoint_step's two kernels give the same
@@ -62,7 +65,7 @@ struct Layout {
   size_t slot;
   char* base;
   // slot indices
-  size_t ckpt0, x0, ez, rec0, adj0, jbuf, end;
+  size_t ckpt0, x0, ez, rec0, adj0, status, end;
 };
 
 Layout layout(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, void* ws) {
@@ -83,8 +86,8 @@ Layout layout(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, void* ws) 
   s += 2 * (size_t)(L.cp > 1 ? L.cp - 1 : 0) * R;  // two record buffers
   L.adj0 = s;
   s += 2 * (size_t)F;  // adjoint ping-pong
-  L.jbuf = s;
-  s += 1;  // J accumulator and spare
+  L.status = s;
+  s += 1;  // two words: the forward's and the reverse's
   L.end = s;
   return L;
 }
@@ -156,6 +159,29 @@ __global__ void k_objective(const float* trace, int n, float w, double* J) {
     __syncthreads();
   }
   if (threadIdx.x == 0) *J = 0.5 * (double)w * part[0];
+}
+
+// The half's status word, cleared as it starts.
+int* status_word(const Layout& L, bool reverse) { return (int*)at(L, L.status) + (reverse ? 1 : 0); }
+int clear_status(const Layout& L, bool reverse, cudaStream_t st) {
+  return cuda_rc(cudaMemsetAsync(status_word(L, reverse), 0, sizeof(int), st));
+}
+
+// NaN in x[n] and y[n] (either may be null) if one of the first `words` status words
+// reports a wait that ran out
+__global__ void k_poison(const int* status, int words, float* x, float* y, size_t n) {
+  int bad = 0;
+  for (int k = 0; k < words; ++k) bad |= status[k] & ST_TIMEOUT;
+  if (!bad) return;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    if (x) x[i] = __int_as_float(0x7fffffff);
+    if (y) y[i] = __int_as_float(0x7fffffff);
+  }
+}
+// the forward's results look at its own word, the reverse's at both
+int poison(const Layout& L, bool reverse, float* x, float* y, size_t n, cudaStream_t st) {
+  k_poison<<<(unsigned)std::min((n + 255) / 256, (size_t)64), 256, 0, st>>>(status_word(L, false), reverse ? 2 : 1, x, y, n);
+  return fdtd_host::check_launch();
 }
 
 // the reverse sweep's second stream and its events, made once per device
@@ -271,6 +297,7 @@ int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* 
   int rc = zero_fields(&p, ckpt(&p, L, 0), st);
   if (rc) return rc;
   if ((rc = cuda_rc(cudaMemsetAsync(trace, 0, (size_t)a->nsteps * sizeof(float), st)))) return rc;
+  if ((rc = clear_status(L, false, st))) return rc;
   float* ez = at(L, L.ez);
   TilePlan pl;
   const bool tile = tile_layout(&p, L, pl);
@@ -281,7 +308,8 @@ int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* 
     if (tile && (record || len >= kTileMinSteps)) {
       const FieldSet out = set_of(ckpt(&p, L, c + 1));
       if ((rc = launch_tile(p, set_of(ckpt(&p, L, c)), out, set_of(xbuf(&p, L, 0)), out, nullptr, t_start, len,
-                            nullptr, trace, (unsigned*)ez, pl, st, record ? kTileRec : kTileFwd, &adj)))
+                            status_word(L, false), trace, (unsigned*)ez, pl, st, record ? kTileRec : kTileFwd, &adj,
+                            nullptr, false)))
         return rc;
       adj.rec += len * box_floats(adj);
       continue;
@@ -297,6 +325,7 @@ int run_forward(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, float* 
       t += k;
     }
   }
+  if (tile && (rc = poison(L, false, trace, nullptr, a->nsteps, st))) return rc;  // J, too, is then NaN
   if (record) {
     rc = cuda_rc(cudaMemcpyAsync(adj.rec, trace, (size_t)a->nsteps * sizeof(float), cudaMemcpyDeviceToDevice, st));
     if (rc) return rc;
@@ -343,6 +372,7 @@ int run_reverse_tile(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, fl
   // (one segment's record, cp steps of at most a grid each, fits in the room of six states a step)
   float* probe = rec + (recorded ? a->nsteps : L.cp) * box_floats(adj);
   unsigned* flags = (unsigned*)at(L, L.ez);
+  int* const status = status_word(L, true);
   const FieldSet x0 = set_of(xbuf(&p, L, 0)), x1 = set_of(xbuf(&p, L, 1));
   int cur = 0;
   for (int c = L.ncp - 1; c >= 0; --c) {
@@ -352,17 +382,17 @@ int run_reverse_tile(const fdtd2d_params* p0, const fdtd2d_adjoint_params* a, fl
     if (recorded) {
       adj.rec = rec + (size_t)t_start * box_floats(adj);
     } else {
-      rc = launch_tile(p, set_of(ckpt(&p, L, c)), x1, x0, x1, nullptr, t_start, len, nullptr, pz, flags, fwd, st,
-                       kTileRec, &adj);
+      rc = launch_tile(p, set_of(ckpt(&p, L, c)), x1, x0, x1, nullptr, t_start, len, status, pz, flags, fwd, st,
+                       kTileRec, &adj, nullptr, false);
       if (rc) return rc;
     }
     const FieldSet out = set_of(adjbuf(&p, L, 1 - cur));
-    rc = launch_tile(p, set_of(adjbuf(&p, L, cur)), out, x0, out, nullptr, t_start + len, len, nullptr, pz, flags, rev,
-                     st, kTileRev, &adj);
+    rc = launch_tile(p, set_of(adjbuf(&p, L, cur)), out, x0, out, nullptr, t_start + len, len, status, pz, flags, rev,
+                     st, kTileRev, &adj, nullptr, false);
     if (rc) return rc;
     cur = 1 - cur;
   }
-  return FDTD_OK;
+  return poison(L, true, grad_naz, grad_nbz, (size_t)a->box.ni * a->box.nj, st);
 }
 
 int run_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* grad_naz, float* grad_nbz,
@@ -373,6 +403,7 @@ int run_reverse(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* g
   if ((rc = zero_fields(p, adjbuf(p, L, 0), main))) return rc;
   if ((rc = cuda_rc(cudaMemsetAsync(grad_naz, 0, gb, main)))) return rc;
   if (grad_nbz && (rc = cuda_rc(cudaMemsetAsync(grad_nbz, 0, gb, main)))) return rc;
+  if ((rc = clear_status(L, true, main))) return rc;
   TilePlan fwd, rev;
   if (tile_layouts(p, L, fwd, rev))
     return run_reverse_tile(p, a, grad_naz, grad_nbz, L, fwd, rev, recorded, main);
@@ -429,6 +460,12 @@ size_t fdtd2d_tm_adjoint_workspace_size(const fdtd2d_params* p, const fdtd2d_adj
   if (check(p, a) != FDTD_OK) return 0;
   const Layout L = layout(p, a, nullptr);
   return L.slot * L.end;
+}
+
+size_t fdtd2d_tm_adjoint_status_offset(const fdtd2d_params* p, const fdtd2d_adjoint_params* a) {
+  if (check(p, a) != FDTD_OK) return 0;
+  const Layout L = layout(p, a, nullptr);
+  return L.slot * L.status;
 }
 
 int fdtd2d_tm_adjoint_forward(const fdtd2d_params* p, const fdtd2d_adjoint_params* a, float* trace, double* J,

@@ -242,8 +242,10 @@ int step_tile_ext(const fdtd2d_params* p, const fdtd2d_state* s, int t0, int nst
     int rc;
     if (p->tfsf_npml > 0 && (rc = launch_inc_line(*p, *s, t, n, inc_e, inc_h, st))) return rc;
     const bool last = t + n == t0 + nsteps;
-    if ((rc = launch_tile(*p, user, user, x0, user, last ? s->ez : nullptr, t, n, last ? s->status : nullptr,
-                          s->probe_ez, flags, tile, st, kTileExt, nullptr, &ext)))
+    // (the Inf/NaN test of the last launch sees what an earlier one's would have; a wait
+    // that runs out is reported by the launch it happens in)
+    if ((rc = launch_tile(*p, user, user, x0, user, last ? s->ez : nullptr, t, n, s->status, s->probe_ez, flags, tile,
+                          st, kTileExt, nullptr, &ext, last)))
       return rc;
     if (p->nf > 0 && (rc = launch_dft_rec(p->nx, p->ny, p->ny, t, n, p->nf, p->dft_cos, p->dft_sin, ext.ez_rec,
                                           ext.rec_slot, s->r_pt, s->i_pt, st)))

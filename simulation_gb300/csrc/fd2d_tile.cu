@@ -51,7 +51,7 @@ bool al16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, const FieldSet& x0, const FieldSet& x1,
                 float* ez, int t0, int nsteps, int* status, float* probe_ez, unsigned* flags, const TilePlan& pl,
-                cudaStream_t st, int mode, const TileAdj* adj, const TileExt* ext) {
+                cudaStream_t st, int mode, const TileAdj* adj, const TileExt* ext, bool check_finite) {
   TileArgs a{};
   a.nx = p.nx;
   a.ny = p.ny;
@@ -70,6 +70,7 @@ int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out,
   a.t0 = t0;
   a.nsteps = nsteps;
   a.status = status;
+  a.check_finite = status && check_finite;
   a.probe_i = p.probe_i;
   a.probe_j = p.probe_j;
   a.probe_ez = probe_ez;

@@ -61,6 +61,7 @@ struct TileArgs {
   const float* src_table;
   int t0, nsteps;
   int* status;
+  int check_finite;   // test the stored fields for Inf/NaN
   int probe_i, probe_j;
   float* probe_ez;
   unsigned* flags;    // one per block, 32 words apart, zero at the start
@@ -749,7 +750,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
       const size_t row = (size_t)i * ny;
       auto st = [&](float* p, const float4& v) {
         tile_st(p, row, j0, ny, vec, v);
-        if (a.status) {
+        if (a.check_finite) {
           const bool f = (j0 + 3 < ny) ? tile_finite(v)
                                        : (j0 >= ny || isfinite(v.x)) && (j0 + 1 >= ny || isfinite(v.y)) &&
                                              (j0 + 2 >= ny || isfinite(v.z));
@@ -778,7 +779,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
       if (LOSSY) put(a.adj.grad_nbz, at(A_GB, r));
     }
   }
-  if (a.status && !fin) raise_status(a.status, ST_NONFINITE);
+  if (!fin) raise_status(a.status, ST_NONFINITE);
 }
 
 template <int V, bool LOSSY, bool PML, int MODE>

@@ -34,12 +34,14 @@ struct TileAdj {
   float* grad_nbz = nullptr;
 };
 
-// defined in fd2d_tile.cu.  max_V: the largest strip to consider
+// defined in fd2d_tile.cu.  max_V: the largest strip to consider.  Every launch that
+// can wait gets a status word (FDTD_STATUS_TIMEOUT where a wait ran out, after which the
+// fields are wrong); check_finite: it also tests the fields it stores
 bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& best, int max_V = 5);
 constexpr int tile_rev_max_V(bool lossy) { return lossy ? 4 : 5; }  // the gradients' shared memory
 int launch_tile(const fdtd2d_params& p, const FieldSet& in, const FieldSet& out, const FieldSet& x0, const FieldSet& x1,
                 float* ez, int t0, int nsteps, int* status, float* probe_ez, unsigned* flags, const TilePlan& pl,
                 cudaStream_t st, int mode = kTileFwd, const TileAdj* adj = nullptr,
-                const TileExt* ext = nullptr);
+                const TileExt* ext = nullptr, bool check_finite = true);
 
 }  // namespace fdtd

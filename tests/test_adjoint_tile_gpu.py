@@ -88,3 +88,24 @@ def test_recorded_halves(cuda_lib, box, ns, cp):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     for g in got[2:]:
         assert torch.equal(g, want[2])
+
+
+def test_a_wait_that_ran_out_is_reported(cuda_lib):
+    """An expired wait of the forward leaves FDTD_STATUS_TIMEOUT in its word: every
+    gradient taken from that forward is then NaN and check() raises; the next forward
+    starts clean."""
+    from simulation_gb300 import _lib
+    from simulation_gb300.adjoint import AdjointProblem
+    pr = AdjointProblem(nx=128, ny=128, npml=8, box=(16, 16), src_offset=20, probe_offset=20, ns=240, checkpoint=16)
+    pr.set_eps(torch.full((16, 16), 2.0))
+    J = pr.forward()
+    want = pr.gradient_naz().clone()
+    assert bool(torch.isfinite(want).all()) and float(want.abs().max()) > 0
+    pr.check()
+    pr.status[0] = 2
+    assert bool(torch.isnan(pr.gradient_naz()).all())
+    with pytest.raises(_lib.FdtdError):
+        pr.check()
+    assert pr.forward() == J
+    assert torch.equal(pr.gradient_naz(), want)
+    pr.check()
