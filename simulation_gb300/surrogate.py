@@ -213,9 +213,20 @@ class FNO:
         self.m = {k: torch.zeros_like(v) for k, v in self.p.items()}
         self.v = {k: torch.zeros_like(v) for k, v in self.p.items()}
         self.step = 0
+        self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)  # of every product and fused layer
         self._refresh_bf16()
 
     # ------------------------------------------------------------ helpers
+    def _gemm(self, *args, **kw):
+        return gemm(*args, status=self.status, **kw)
+
+    def check(self) -> None:
+        """Raise FdtdError if a bounded wait ran out in a tensor-core kernel of this
+        network since ``status`` was last zero, whose results are then wrong (host sync)."""
+        v = int(self.status.item())
+        if v:
+            raise _lib.FdtdError(_lib.lib().fdtd_status_to_error(v), f"FNO status word {v:#x}")
+
     def _refresh_bf16(self):
         self.w16 = {}
         for k in ["H1", "H2"] + [f"L{l}.W" for l in range(self.L)]:
@@ -277,7 +288,7 @@ class FNO:
         _call("fno_pack_inputs", Bn, N, self.cin, inp16.shape[2], 0, inp.data_ptr(), inp16.data_ptr(), inpT.data_ptr())
         # the DFT of every sample's 16 channels in one product: F[(b, c)][j] = sum_n inpT[n][(b, c)] Phi[j][n]
         F = torch.empty((Bn, KIN, 2 * M), dtype=torch.float32, device=dev)
-        gemm(inpT, self.phi16, a_mn=True, out=F.view(Bn * KIN, 2 * M))
+        self._gemm(inpT, self.phi16, a_mn=True, out=F.view(Bn * KIN, 2 * M))
         Fm = torch.empty((M, Bn, 2 * KIN), dtype=BF, device=dev)
         _call("fno_dft_to_modes", Bn, KIN, M, F.data_ptr(), Fm.data_ptr())
         return inp16, Fm
@@ -287,11 +298,11 @@ class FNO:
         Bn, N, C, M, dev = inp.shape[0], self.N, self.C, self.M, self.dev
         inp16, Fm = self._first_modes_folded(inp, True)
         Gm = torch.empty((M, Bn, 2 * C), dtype=torch.float32, device=dev)
-        gemm(Fm, self.rbig0f, out=Gm)
+        self._gemm(Fm, self.rbig0f, out=Gm)
         G = torch.empty((Bn, C, 2 * M), dtype=BF, device=dev)
         _call("fno_modes_to_dft", Bn, C, M, Gm.data_ptr(), G.data_ptr())
         x = torch.empty((Bn, N, C), dtype=BF, device=dev)
-        gemm(inp16, self.w0f16, out=x, bias=self.p["L0.b"], gelu=True, second=(self.psi16, G, False, False))
+        self._gemm(inp16, self.w0f16, out=x, bias=self.p["L0.b"], gelu=True, second=(self.psi16, G, False, False))
         return x
 
     # ------------------------------------------------------------ fused layers
@@ -310,14 +321,14 @@ class FNO:
             x = torch.empty((Bn, N, C), dtype=BF, device=dev)
             _call("fno_lift_fwd", Bn * N, C, self.cin, inp.data_ptr(), self.p["P"].data_ptr(),
                   self.p["pb"].data_ptr(), x.data_ptr())
-            F = gemm(x, self.phi16.unsqueeze(0).expand(Bn, -1, -1), a_mn=True)
+            F = self._gemm(x, self.phi16.unsqueeze(0).expand(Bn, -1, -1), a_mn=True)
             Fm = torch.empty((M, Bn, 2 * C), dtype=BF, device=dev)
             _call("fno_dft_to_modes", Bn, C, M, F.data_ptr(), Fm.data_ptr())
         Gm = torch.empty((M, Bn, 2 * C), dtype=BF, device=dev)
         h = torch.empty((Bn, C), dtype=BF, device=dev)
         for l in range(self.L):
             first, last = folded and l == 0, l == self.L - 1
-            gemm(Fm, self.rbig0f if first else self.rbig[l], out=Gm)
+            self._gemm(Fm, self.rbig0f if first else self.rbig[l], out=Gm)
             w = self.w0k16 if first else self.w16[f"L{l}.W"]
             pre = None
             if saved is not None:
@@ -331,7 +342,7 @@ class FNO:
             _call("fno_layer_fwd", Bn, N, C, M, w.shape[1], x.data_ptr(), w.data_ptr(), self.p[f"L{l}.b"].data_ptr(),
                   self.psi16.data_ptr(), Gm.data_ptr(), None if last else xn.data_ptr(),
                   None if last else fn.data_ptr(), h.data_ptr() if last else None,
-                  None if pre is None else pre.data_ptr(), None)
+                  None if pre is None else pre.data_ptr(), self.status.data_ptr())
             x, Fm = xn, fn
         return h
 
@@ -367,17 +378,17 @@ class FNO:
         G = torch.empty((Bn, C, 2 * M), dtype=BF, device=dev)
         for l in range(1 if folded else 0, self.L):
             # truncated DFT: F_b[C][2M] = x_b^T Phi^T   (A = x_b stored [N][C]: MN-major)
-            gemm(x, phi_b, a_mn=True, out=F)
+            self._gemm(x, phi_b, a_mn=True, out=F)
             _call("fno_dft_to_modes", Bn, C, M, F.data_ptr(), Fm.data_ptr())
             # mode mixing: Gm_k[B][2C] = Fm_k Rbig_k^T
-            gemm(Fm, self.rbig[l], out=Gm)
+            self._gemm(Fm, self.rbig[l], out=Gm)
             _call("fno_modes_to_dft", Bn, C, M, Gm.data_ptr(), G.data_ptr())
             # pointwise + inverse DFT in one accumulator, then bias and GELU:
             # x'_b = GELU(x_b W^T + Psi G_b^T + b); pre-activation kept for backward
             xn = torch.empty((Bn, N, C), dtype=BF, device=dev)
             pre = torch.empty((Bn, N, C), dtype=BF, device=dev) if keep else None
-            gemm(x, self.w16[f"L{l}.W"], out=xn, bias=self.p[f"L{l}.b"], gelu=True, pre=pre,
-                 second=(self.psi16, G, False, False))
+            self._gemm(x, self.w16[f"L{l}.W"], out=xn, bias=self.p[f"L{l}.b"], gelu=True, pre=pre,
+                       second=(self.psi16, G, False, False))
             if keep:
                 saved["x"].append(x)
                 saved["pre"].append(pre)
@@ -392,9 +403,9 @@ class FNO:
         Bn, dev = h.shape[0], self.dev
         a1 = torch.empty((Bn, self.H), dtype=BF, device=dev)
         z1 = torch.empty((Bn, self.H), dtype=BF, device=dev)
-        gemm(h, self.w16["H1"], out=a1, bias=self.p["hb1"], gelu=True, pre=z1)
+        self._gemm(h, self.w16["H1"], out=a1, bias=self.p["hb1"], gelu=True, pre=z1)
         o = torch.empty((Bn, self.D), dtype=torch.float32, device=dev)
-        gemm(a1, self.w16["H2"], out=o, bias=self.p["hb2"])
+        self._gemm(a1, self.w16["H2"], out=o, bias=self.p["hb2"])
         if saved is not None:
             saved.update(h=h, a1=a1, z1=z1)
             self._saved = saved
@@ -411,14 +422,14 @@ class FNO:
         dO16 = torch.empty((Bn, D), dtype=BF, device=dev)
         _call("fno_to_bf16", dO.numel(), dO.data_ptr(), dO16.data_ptr())
         # head
-        gemm(dO16, s["a1"], a_mn=True, b_mn=True, out=self.g["H2"])            # dH2 = dO^T a1
+        self._gemm(dO16, s["a1"], a_mn=True, b_mn=True, out=self.g["H2"])       # dH2 = dO^T a1
         _call("fno_colsum", Bn, D, None, dO.data_ptr(), self.g["hb2"].data_ptr())
-        da1 = gemm(dO16, self.w16["H2"], b_mn=True)                             # da1 = dO H2  [B][H]
+        da1 = self._gemm(dO16, self.w16["H2"], b_mn=True)                       # da1 = dO H2  [B][H]
         dz1 = torch.empty((Bn, H), dtype=BF, device=dev)
         _call("fno_gelu_bwd", Bn * H, None, da1.data_ptr(), s["z1"].data_ptr(), dz1.data_ptr())
-        gemm(dz1, s["h"], a_mn=True, b_mn=True, out=self.g["H1"])               # dH1 = dz1^T h
+        self._gemm(dz1, s["h"], a_mn=True, b_mn=True, out=self.g["H1"])         # dH1 = dz1^T h
         _call("fno_colsum", Bn, H, dz1.data_ptr(), None, self.g["hb1"].data_ptr())
-        dh = gemm(dz1, self.w16["H1"], b_mn=True)                               # dh = dz1 H1  [B][C]
+        dh = self._gemm(dz1, self.w16["H1"], b_mn=True)                         # dh = dz1 H1  [B][C]
         wide = C % 8 == 0 and C <= 2048  # the fused kernels' channel groups
         dx16 = dx32 = None
         if not wide:
@@ -448,23 +459,23 @@ class FNO:
                 _call("fno_gelu_bwd", dz.numel(), p16 if p32 is None else None, p32, pre.data_ptr(), dz.data_ptr())
                 _call("fno_colsum", Bn * N, C, dz.data_ptr(), None, self.g[f"L{l}.b"].data_ptr())
             # dW = sum_b dz_b^T x_b  (per-sample products, then summed)
-            gemm(dz, x, a_mn=True, b_mn=True, out=parts)
+            self._gemm(dz, x, a_mn=True, b_mn=True, out=parts)
             _call("fno_sum_parts", Bn, C * C, parts.data_ptr(), self.g[f"L{l}.W"].data_ptr())
             # spectral branch: dG_b = dz_b^T Psi ; dFm_k = dGm_k Rbig_k ; dRbig_k = dGm_k^T Fm_k
-            gemm(dz, psi_b, a_mn=True, b_mn=True, out=dG)
+            self._gemm(dz, psi_b, a_mn=True, b_mn=True, out=dG)
             _call("fno_dft_to_modes", Bn, C, M, dG.data_ptr(), dGm.data_ptr())
-            gemm(dGm, self.rbig[l], b_mn=True, out=dFm)
-            gemm(dGm, Fm, a_mn=True, b_mn=True, out=dRbig)
+            self._gemm(dGm, self.rbig[l], b_mn=True, out=dFm)
+            self._gemm(dGm, Fm, a_mn=True, b_mn=True, out=dRbig)
             _call("fno_fold_drbig", M, C, dRbig.data_ptr(), self.g[f"L{l}.Rr"].data_ptr(), self.g[f"L{l}.Ri"].data_ptr())
             _call("fno_modes_to_dft", Bn, C, M, dFm.data_ptr(), dF.data_ptr())
             # dx = dz W + Phi^T dF^T in one accumulator (Phi stored [2M][N]: MN-major, shared)
             if chained and l > 0:
-                gemm(dz, self.w16[f"L{l}.W"], b_mn=True, out=dz2, second=(self.phi16, dF, True, False),
-                     gelu_bwd=(s["pre"][l - 1], self.g[f"L{l - 1}.b"]))
+                self._gemm(dz, self.w16[f"L{l}.W"], b_mn=True, out=dz2, second=(self.phi16, dF, True, False),
+                           gelu_bwd=(s["pre"][l - 1], self.g[f"L{l - 1}.b"]))
                 dz, dz2 = dz2, dz
                 continue
             nd = torch.empty((Bn, N, C), dtype=torch.float32, device=dev)
-            gemm(dz, self.w16[f"L{l}.W"], b_mn=True, out=nd, second=(self.phi16, dF, True, False))
+            self._gemm(dz, self.w16[f"L{l}.W"], b_mn=True, out=nd, second=(self.phi16, dF, True, False))
             dx32 = nd
         if wide:
             _call("fno_lift_bwd32", Bn * N, C, self.cin, s["inp"].data_ptr(), dx32.data_ptr(), self.g["P"].data_ptr(),
@@ -602,6 +613,7 @@ def train(model: FNO, inp: np.ndarray, tgt: np.ndarray, samples: int = 200_000, 
         model.adam_step(lr_final + (lr - lr_final) * a)
         if it % log_every == 0 or it == steps - 1:
             hist.append((it, float(loss.item())))
+            model.check()
     return hist
 
 
@@ -684,6 +696,7 @@ class JudgedSurrogate:
             bad = err > self.tol
             pred.index_copy_(0, ci, torch.where(bad[:, None], ref, pred.index_select(0, ci)))
             e = err.cpu().numpy()
+            self.model.check()
             info.update(check_err_median=float(np.median(e)), check_err_p90=float(np.quantile(e, 0.9)),
                         fell_back=int((e > self.tol).sum()))
         return pred, info
@@ -786,6 +799,7 @@ def main(argv=None) -> None:
     out["baseline_zero"] = summary(rel_l2_spectrum(np.zeros_like(Yte), Yte))
     out["baseline_frame_only"] = summary(rel_l2_spectrum(cmul(P, ones).cpu().numpy(), Yte))
     out["network"] = summary(rel_l2_spectrum(m.spectrum(Xd).cpu().numpy(), Yte))
+    m.check()
     for name, gate in (("judged", None), ("judged_gated", (1.0, 6.0))):
         judge = JudgedSurrogate(m, check_frac=0.01, tol=0.01, gate=gate, seed=1)
         judge(test, Xd)  # warm-up (plans, buffers)
