@@ -13,6 +13,7 @@ graph (``run_graph``).
 """
 from __future__ import annotations
 
+import sys
 from collections import namedtuple
 
 import numpy as np
@@ -23,6 +24,7 @@ from ._lib import call, ptr
 from .sources import dft_tables, to_device, wave_values
 
 EPS0 = 8.854e-12  # fd2d/python/fd2d_3_4.py:180
+WS_EXTRA_SMALL = 256 << 20  # workspace beyond the smallest that is taken without a look at the free memory
 
 pmlayer = namedtuple("pmlayer", ("fx1", "fx2", "fx3", "fy1", "fy2", "fy3", "gx2", "gx3", "gy2", "gy3"))
 
@@ -85,6 +87,15 @@ def dielectric(nx: int, ny: int, npml: int, rgrid: float, dt: float, epsr: float
     return naz, nbz
 
 
+def free_bytes(device: torch.device) -> int:
+    """Device memory that new tensors can still take, the allocator's unused share
+    included (unlimited on the host and while a CUDA graph is being captured)."""
+    if device.type != "cuda" or torch.cuda.is_current_stream_capturing():
+        return sys.maxsize
+    return (torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device)
+            - torch.cuda.memory_allocated(device))
+
+
 class PointSource:
     """Hard (``dz[i,j] = v``) or soft (``+=``) point source with a float64 waveform."""
 
@@ -139,6 +150,7 @@ class SimTM2D:
         self._ns = 0
         self._tables(ns)
         self._workspace = None
+        self._ws_declined = sys.maxsize  # a workspace size that the device had no room for
         self._graphs = {}
 
     # ------------------------------------------------------------ setup
@@ -188,11 +200,32 @@ class SimTM2D:
             self._tables(max(t_last, 2 * self._ns))
 
     def workspace(self):
+        """The time loop's device workspace (None: it needs none): what its fastest
+        path takes, or, where the device lacks the room for that, the smaller size
+        with which the results are the same."""
+        have = 0 if self._workspace is None else self._workspace.numel()
         n = _lib.lib().fdtd2d_fast_workspace_size(self._p, self.steps_per_pass)
-        if n and (self._workspace is None or self._workspace.numel() < n):
-            self._workspace = torch.empty(n, dtype=torch.uint8, device=self.device)
-            self._graphs = {}
+        if n > have and n >= self._ws_declined:
+            n = self._plain_workspace_size()
+        if n > have:
+            plain = self._plain_workspace_size()
+            # the fast path's extra is whole grids' worth on large ragged or DFT grids:
+            # it leaves half of the free memory to the caller
+            if n - plain > WS_EXTRA_SMALL and 2 * (n - plain) > free_bytes(self.device):
+                self._ws_declined, n = n, plain
+            if n > have:
+                try:
+                    self._workspace = torch.empty(n, dtype=torch.uint8, device=self.device)
+                except torch.cuda.OutOfMemoryError:
+                    if n == plain:
+                        raise
+                    self._ws_declined = n
+                    return self.workspace()
+                self._graphs = {}
         return self._workspace
+
+    def _plain_workspace_size(self) -> int:
+        return _lib.lib().fdtd2d_workspace_size(self._p, self.steps_per_pass)
 
     # ------------------------------------------------------------ time loop
     def step(self, n: int = 1, steps_per_pass: int | None = None) -> None:
