@@ -189,7 +189,8 @@ int fdtd2d_step_n(const fdtd2d_params* p, fdtd2d_state* s, int t0, int nsteps, i
 
 /* Tuning knob of the fused kernel (used by the bench/autotuner): columns per
  * lane (2 or 4; 0 = automatic) and rows per warp segment (0 = automatic, one
- * wave of warps).
+ * wave of warps).  With a shape set, calls that leave the steps per pass to the
+ * library march in it, on grids of every size.
  * No reference counterpart. */
 int fdtd2d_set_march_config(int cols_per_lane, int warps_per_block, int seg_rows);
 /* Tuning knob of the fused kernel's work layout: the time of a general row

@@ -90,13 +90,13 @@ size_t line_bytes(const fdtd2d_params* p) {
 size_t fused_workspace_bytes(const fdtd2d_params* p) { return slot_bytes(p) * nslots(p) + line_bytes(p); }
 
 // The on-chip loop (fd2d_tile.cuh): point-source programs whose tiles fit the
-// SMs, with the library's choice of steps per pass.  Its workspace: one
+// SMs, with the library's choice of steps per pass and of the march's shape.  Its workspace: one
 // exchange set of the evolving fields (as the march's ping-pong set) and the
 // blocks' flags.
 // With plane wave or running DFT: also the incident line's tables and, with the
 // DFT, room for the ez of a launch's steps.
 bool tile_ok(const fdtd2d_params* p, int steps_per_pass, TilePlan& pl) {
-  if (steps_per_pass != 0 || (p->tfsf_npml > 0 && p->ny > kLineMaxNy)) return false;
+  if (steps_per_pass != 0 || march_shape_set() || (p->tfsf_npml > 0 && p->ny > kLineMaxNy)) return false;
   int dev = 0, nsm = 0, coop = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||

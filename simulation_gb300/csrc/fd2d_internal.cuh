@@ -47,6 +47,8 @@ int march_max_steps_per_pass();
 int march_default_steps(int nx, int ny);
 // the caller's balance knob (fdtd2d_set_march_balance; 0: default)
 float march_gen_cost();
+// whether the caller has set a march shape of its own (fdtd2d_set_march_config): calls then march
+bool march_shape_set();
 // whether large-grid passes go through the chained kernel (fd2d_chain.cuh):
 // grids that do not fit on the chip, without a caller's own march shape
 bool chain_better(int nx, int ny);

@@ -49,8 +49,10 @@ int march_default_steps(int nx, int ny) { return (long long)nx * ny < (1LL << 21
 
 float march_gen_cost() { return g_cfg.gen_cost; }
 
+bool march_shape_set() { return g_cfg.cpl || g_cfg.seg_rows; }
+
 bool chain_better(int nx, int ny) {
-  if (g_cfg.cpl || g_cfg.seg_rows) return false;
+  if (march_shape_set()) return false;
   // (32-bit element offsets)
   return (long long)nx * ny >= (1LL << 20) && (long long)nx * ny < (1LL << 31) && nx >= 64 && ny >= 128;
 }
@@ -59,7 +61,7 @@ bool chain_better(int nx, int ny) {
 // 128^2 875 us / 1050, 512^2 903 / 1145, 1024^2 1111 / 1495, 2048^2 2048 / 3458,
 // 4096^2 6456 / 11000)
 bool chain_ext_better(int nx, int ny) {
-  if (g_cfg.cpl || g_cfg.seg_rows) return false;
+  if (march_shape_set()) return false;
   return (long long)nx * ny >= (1LL << 14) && (long long)nx * ny < (1LL << 31) && nx >= 64 && ny >= 128;
 }
 

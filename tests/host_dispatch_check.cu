@@ -134,6 +134,7 @@ int launch_adjoint_fused2(P, int t, const fdtd2d_fields&, const fdtd2d_fields&, 
 int march_max_steps_per_pass() { return 4; }
 int march_default_steps(int, int) { return 2; }
 float march_gen_cost() { return 0.f; }
+bool march_shape_set() { return fake::march_set; }
 bool chain_better(int nx, int ny) { return !fake::march_set && (long long)nx * ny > (1 << 20); }
 bool chain_ext_better(int nx, int ny) { return chain_better(nx, ny); }
 bool march_ext_supported(P p) { return p.nf <= kMarchMaxNf; }
@@ -211,6 +212,28 @@ void check_ext_status() {
     }
 }
 
+// a march shape that the caller has set is used where the library would otherwise
+// take the loop on the chip, as it is on larger grids
+void check_march_shape() {
+  for (bool ext : {false, true}) {
+    fdtd2d_params p = params(100, 96);
+    if (ext) {
+      p.nf = 2;
+      p.dft_cos = p.dft_sin = F;
+      p.dft_table_len = 1000;
+    }
+    fdtd2d_state s = state();
+    const size_t n = fdtd2d_fast_workspace_size(&p, 0);
+    for (bool set : {false, true}) {
+      reset();
+      fake::march_set = set;
+      expect(fdtd2d_step_n(&p, &s, 0, 24, 0, WS, n, nullptr) == FDTD_OK, "step_n");
+      expect((count(ext ? "tile_ext" : "tile") > 0) == !set, "on the chip unless a march shape is set");
+      expect((count(ext ? "march_ext" : "march") > 0) == set, "marching where a march shape is set");
+    }
+    fake::march_set = false;
+  }
+}
 #else
 // the adjoint's launches report into words of the workspace that the call clears first
 void check_adjoint_status() {
@@ -266,6 +289,7 @@ int main() {
   check_adjoint_status();
 #else
   check_ext_status();
+  check_march_shape();
 #endif
   if (g_fail) return 1;
   std::printf("ok\n");

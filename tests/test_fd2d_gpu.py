@@ -275,3 +275,20 @@ def test_full_size_linearity(cuda_lib):
         assert torch.equal(x2[big], y[big]), k
         assert float((x2 - y).abs().max()) <= 1e-35, k
     assert float(a.ez.abs().max()) > 0.0
+
+
+def test_march_shape_with_the_librarys_steps(cuda_lib):
+    """A march shape set by the caller holds for the library's own choice of steps per
+    pass too, on a grid that would otherwise run on the chip; still bitwise."""
+    from simulation_gb300 import _lib
+    try:
+        for cpl, seg in ((4, 7), (2, 33)):
+            _lib.call("fdtd2d_set_march_config", cpl, 4, seg)
+            a, b = _mk(200, 136, 8, True, True), _mk(200, 136, 8, True, True)
+            a.step(23)
+            b.step_per_function(23)
+            torch.cuda.synchronize()
+            for k in ("dz", "ez", "iz", "hx", "hy", "ihx", "ihy"):
+                assert torch.equal(getattr(a, k), getattr(b, k)), f"cpl={cpl} seg={seg} {k}"
+    finally:
+        _lib.call("fdtd2d_set_march_config", 0, 4, 0)
