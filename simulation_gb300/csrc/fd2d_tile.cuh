@@ -748,8 +748,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
     const int i = i0 + r;
     if (i >= oi0 && i < oi1 && own_c) {
       const size_t row = (size_t)i * ny;
-      auto st = [&](float* p, const float4& v) {
-        tile_st(p, row, j0, ny, vec, v);
+      auto test = [&](const float4& v) {
         if (a.check_finite) {
           const bool f = (j0 + 3 < ny) ? tile_finite(v)
                                        : (j0 >= ny || isfinite(v.x)) && (j0 + 1 >= ny || isfinite(v.y)) &&
@@ -757,6 +756,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
           fin &= f;
         }
       };
+      auto st = [&](float* p, const float4& v) {
+        tile_st(p, row, j0, ny, vec, v);
+        test(v);
+      };
+      // ez = naz*dz; with loss an Inf or NaN of ez is in iz too
+      if (!LOSSY) test(to4(mul4(f4(at(A_NAZ, r)), dz[r])));
       st(a.out.dz, to4(dz[r]));
       st(a.out.hx, to4(hx[r]));
       st(a.out.hy, to4(hy[r]));

@@ -90,3 +90,22 @@ def test_subnormal_fields(cuda_lib, lossy, npml):
     a.step(24)
     b.step_per_function(24)
     _equal(a, b, "subnormal")
+
+
+@pytest.mark.parametrize("nx,ny", [(100, 100), (250, 241), (700, 512)])
+@pytest.mark.parametrize("lossy,npml", [(False, 0), (False, 8), (True, 8)])
+@pytest.mark.parametrize("ext", [False, True])
+def test_nonfinite_ez_of_the_last_cell(cuda_lib, nx, ny, lossy, npml, ext):
+    """No H update reads ez of cell (nx-1, ny-1): an Inf or NaN there is in ez alone"""
+    from simulation_gb300 import _lib
+    from simulation_gb300 import fd2d as G
+    for bad in (float("inf"), float("nan")):
+        s = G.SimTM2D(nx, ny, pml=G.pmlparam(nx, ny, npml) if npml else None, lossy=lossy,
+                      source=G.PointSource(nx // 2, ny // 2, ("gauss", 20, 6.0)), tfsf_npml=8 if ext else 0)
+        s.step(12)
+        s.check()
+        s.naz[nx - 1, ny - 1] = bad
+        s.step(12)
+        assert not bool(torch.isfinite(s.ez[nx - 1, ny - 1]))
+        with pytest.raises(_lib.FdtdError):
+            s.check()
