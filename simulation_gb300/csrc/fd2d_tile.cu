@@ -1,41 +1,9 @@
-// Launch and layout choice of the on-chip 2D time loop (fd2d_tile.cuh).
+// Launch of the on-chip 2D time loop (fd2d_tile.cuh).
 #include "fd2d_tile.cuh"
 
 #include <type_traits>
 
 namespace fdtd {
-
-// The layout with the shortest modelled step among those whose tiles fit the
-// SMs, one block each; false when none does (the caller marches).  The model,
-// in us, fitted to measured layouts with an absorbing layer (the general
-// steps, on which all tiles wait): a step takes 0.35 + 0.27 V (V = 1: 0.58,
-// 2: 0.75, 5: 1.7), loss adds 0.1 V; an exchange 2.1 + 0.52 V (fence, flag and
-// read latencies, and the halo's traffic), once in T steps.  100^2 runs 1.2 a
-// step with V = 1, T = 4 (6.2 marching), 1024^2 3.3 with V = 5, T = 4 (10.5).
-bool tile_plan(int nx, int ny, bool lossy, bool pml, int max_blocks, TilePlan& best, int max_V) {
-  double best_cost = 1e30;
-  for (int V = 1; V <= max_V; ++V)
-    for (int T = 2; T <= 8; ++T) {
-      TilePlan pl;
-      pl.V = V;
-      pl.T = T;
-      pl.hc = ny <= kTileCols ? 0 : (T + 3) / 4 * 4;  // whole lanes
-      pl.own_r = kTileWarps * V - 2 * T;
-      pl.own_c = kTileCols - 2 * pl.hc;
-      if (pl.own_r < T) continue;
-      pl.n_ti = (nx + pl.own_r - 1) / pl.own_r;
-      pl.n_tj = (ny + pl.own_c - 1) / pl.own_c;
-      const long blocks = (long)pl.n_ti * pl.n_tj;
-      if (blocks > max_blocks) continue;
-      const double step = 0.35 + V * ((pml ? 0.27 : 0.2) + (lossy ? 0.1 : 0.0));
-      const double cost = step + (blocks > 1 ? (2.1 + 0.52 * V) / T : 0.0);
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = pl;
-      }
-    }
-  return best_cost < 1e30;
-}
 
 namespace {
 

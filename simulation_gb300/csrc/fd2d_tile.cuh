@@ -46,9 +46,6 @@
 
 namespace fdtd {
 
-constexpr int kTileWarps = 16;
-constexpr int kTileCols = 128;
-
 struct TileArgs {
   int nx, ny;
   FieldSet in, out;   // read at the start; written at the end

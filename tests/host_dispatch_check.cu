@@ -118,11 +118,6 @@ int launch_tile(P, FS, FS, FS, FS, float*, int t0, int n, int* status, float*, u
   static const char* const kName[] = {"tile", "tile_rec", "tile_rev", "tile_ext"};
   return log(kName[mode], status, finite && status, t0, n);
 }
-bool tile_plan(int nx, int ny, bool, bool, int, TilePlan& pl, int) {  // four tiles on grids of up to 2^20 cells
-  pl.V = pl.n_ti = pl.n_tj = 2;
-  pl.T = 4;
-  return (long long)nx * ny <= (1 << 20);
-}
 int launch_adjoint_fused(P, int t, const fdtd2d_fields&, const fdtd2d_fields&, const fdtd2d_fields&, int, int, float,
                          const fdtd2d_box&, float*, float*, St) {
   return log("adjoint_fused", nullptr, false, t, 1);
@@ -234,6 +229,29 @@ void check_march_shape() {
     fake::march_set = false;
   }
 }
+// no layout for grids far beyond the chip, up to the largest extents that are taken
+void check_plan_extents() {
+  for (int n : {2000, 1 << 20, 2147483647 - 100, 2147483647})
+    for (bool lossy : {false, true})
+      for (bool pml : {false, true}) {
+        TilePlan pl;
+        expect(!tile_plan(n, n == 2000 ? n : 4000, lossy, pml, 152, pl), "no layout");
+        expect(!tile_plan(n == 2000 ? n : 4000, n, lossy, pml, 152, pl), "no layout");
+        if (n > 2000) expect(!tile_plan(n, 3, lossy, pml, 152, pl) && !tile_plan(3, n, lossy, pml, 152, pl), "no layout");
+      }
+  for (int nx : {3, 100, 1024, 1080})
+    for (int ny : {3, 100, 960, 1024}) {
+      TilePlan pl;
+      expect(tile_plan(nx, ny, true, true, 152, pl), "a layout");
+      expect((long long)pl.n_ti * pl.own_r >= nx && (long long)pl.n_tj * pl.own_c >= ny && pl.n_ti * pl.n_tj <= 152,
+             "the layout covers the grid");
+    }
+  fdtd2d_params p = params(2147483647 - 10, 3);
+  fdtd2d_state s = state();
+  reset();
+  expect(fdtd2d_step_n(&p, &s, 0, 8, 0, WS, ~(size_t)0, nullptr) == FDTD_OK && count("step3") == 8,
+         "a grid of 2^31 rows steps in three launches");
+}
 #else
 // the adjoint's launches report into words of the workspace that the call clears first
 void check_adjoint_status() {
@@ -290,6 +308,7 @@ int main() {
 #else
   check_ext_status();
   check_march_shape();
+  check_plan_extents();
 #endif
   if (g_fail) return 1;
   std::printf("ok\n");
