@@ -30,6 +30,34 @@ def test_fused_layers_equal_separate(cuda_lib, monkeypatch, N, layers, B, fold):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("N,layers,B", [(128, 1, 1), (128, 3, 5), (256, 2, 153), (2048, 2, 3)])
+def test_gradients_equal_separate(cuda_lib, monkeypatch, N, layers, B):
+    """The gradients from either forward.  The weights' come from products: the same bits.
+    The lift's and the biases' are added up by atomics in any order: of at most k = 1216
+    partial sums p, so two runs differ by 2 k 2^-24 sum|p| = 1.5e-4 sum|p| at most; 1e-3 of
+    the largest entry leaves room for sums that cancel to a seventh."""
+    from simulation_gb300 import surrogate as S
+    m = S.FNO(seed=3, nbins=N, layers=layers)
+    g = torch.Generator().manual_seed(N * B)
+    m.p["H2"].copy_(((torch.rand(m.p["H2"].shape, generator=g) * 2 - 1) / 16).cuda())
+    m._refresh_bf16()
+    x = (torch.rand((B, N, 6), generator=g) * 2 - 1).cuda()
+    t = torch.randn((B, 128), generator=g).cuda()
+    got = []
+    fused = S.FNO._fused
+    for pick in (lambda self, n: False, fused):
+        monkeypatch.setattr(S.FNO, "_fused", pick)
+        m.loss_and_grad(x, t)
+        got.append({k: v.clone() for k, v in m.g.items()})
+    for k, a in got[0].items():
+        b = got[1][k]
+        assert float(a.abs().max()) > 0, k
+        if k.startswith("H") or k.split(".")[-1] in ("W", "Rr", "Ri"):
+            assert torch.equal(a, b), k
+        else:
+            assert float((a - b).abs().max()) <= 1e-3 * float(a.abs().max()), k
+
+
 def test_layer_refuses(cuda_lib):
     from simulation_gb300 import _lib
     p = torch.zeros(64, device="cuda").data_ptr()
