@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(layer_threads(LAST), 1)
       if (!ok) {  // a wait ran out: let the copies in flight land before the CTA ends
         mbar_wait(bar(WFULL), 0, a.status);
         for (int j = i > 2 ? i - 2 : 0; j < i; ++j)
-          mbar_wait(bar(XFULL + j & 1), (uint32_t)((j >> 1) & 1), a.status);
+          mbar_wait(bar(XFULL + (j & 1)), (uint32_t)((j >> 1) & 1), a.status);
         for (int j = np > 3 ? np - 3 : 0; j < np; ++j)
           mbar_wait(bar(PFULL + j % 3), (uint32_t)((j / 3) & 1), a.status);
         if (ng >= 1) mbar_wait(bar(GFULL), (uint32_t)((ng - 1) & 1), a.status);
