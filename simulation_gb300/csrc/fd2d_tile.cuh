@@ -757,8 +757,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1) k_tile(const TileArgs a) {
         tile_st(p, row, j0, ny, vec, v);
         test(v);
       };
-      // ez = naz*dz; with loss an Inf or NaN of ez is in iz too
-      if (!LOSSY) test(to4(mul4(f4(at(A_NAZ, r)), dz[r])));
+      // ez = naz*dz; with loss an Inf or NaN of ez is in iz too.  (The adjoint's modes are
+      // not tested; with this line in them 1500 steps at 1024^2 took 10.35 ms against 10.30)
+      if (!LOSSY && !REC && !REV) test(to4(mul4(f4(at(A_NAZ, r)), dz[r])));
       st(a.out.dz, to4(dz[r]));
       st(a.out.hx, to4(hx[r]));
       st(a.out.hy, to4(hy[r]));
