@@ -49,9 +49,8 @@ WORKLOAD = ("2D TM PML lossy-cylinder benchmark program: 8192x8192, npml=32 grad
             "cylinder r=1000 eps_r=30 sigma=0.3, hard Gaussian Dz source t0=20 spread=6, 2000 steps, FP32")
 # DRAM bytes per cell per fused pass, from one ncu capture each ((dram__bytes_read.sum
 # + dram__bytes_write.sum) / cells): the march's K=4 pass on 4096^2 (1009.4 MB / 16.78 M
-# cells, profiles/k_march_K4_CPL4_full_4096.md) and the chained pass of 8 steps on
-# 6144^2 (profiles/k_chain_4x2_6144.md); traffic grows in proportion to the cells, so it
-# is scaled to the launch size
+# cells) and the chained pass of 8 steps on 6144^2; traffic grows in proportion to the
+# cells, so it is scaled to the launch size
 NCU_TRAFFIC_BYTES_PER_CELL_PASS = {4: 60.2, 8: 62.1}
 CHAIN_STEPS = 8  # steps per pass that the library takes for the benchmark's grid when left to choose
 
@@ -598,11 +597,11 @@ def _bench_adjoint(st) -> dict:
     cu = pr.nx * pr.ny * pr.ns
     # algorithmic bytes per cell and time step of this problem (lossless box: no iz, nbz),
     # which runs on the chip: dz, hx, hy, ihx, ihy and naz in, the five out once per
-    # segment; the reverse runs the segment again and undoes it (twice that), with dz
-    # of the box written and read every step
+    # segment, and the same of the adjoint fields in the reverse; the forward writes dz
+    # of the box every step and the reverse reads it (the record of all steps fits the
+    # workspace, so no segment runs again)
     box = pr.box[2] * pr.box[3] / (pr.nx * pr.ny)
-    fwd_b = 44 / pr.cp
-    rev_b = 2 * 44 / pr.cp + 8 * box
+    fwd_b = rev_b = 44 / pr.cp + 4 * box
     res = {"forward_ms": fwd, "reverse_ms": rev, "forward_Gcell_updates_per_s": cu / fwd / 1e6,
            "reverse_Gcell_updates_per_s": cu / rev / 1e6, "checkpoint": pr.cp, "cuda_graphs": pr.use_graphs,
            "bytes_per_cell_update": {"forward": fwd_b, "reverse": rev_b},

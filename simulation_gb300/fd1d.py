@@ -139,8 +139,8 @@ class Sim1D:
     MAX_FUSED_NX = 65536  # FDTD1D_MAX_FUSED_NX
 
     def step(self, n: int = 1) -> None:
-        """Advance n steps: one fused launch (one thread-block cluster) when the
-        line fits on-chip, else one launch per reference function per step."""
+        """Advance n steps: one fused launch (a warp, a block or a thread-block
+        cluster, by the line's length) when the line fits on-chip, else one launch per reference function per step."""
         if n <= 0:
             return
         if self.nx > self.MAX_FUSED_NX:
